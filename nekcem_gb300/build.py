@@ -24,6 +24,7 @@ SOURCES = {
     "nekgpu_host.cpp": ["-Xcompiler", "-ffp-contract=off"],  # same rounding on x86 and Arm
     "nekgpu_plain.cu": ["--fmad=false"],
     "nekgpu_fused.cu": [],
+    "nekgpu_fp64.cu": [],
     "nekgpu_mixed.cu": [],
     "nekgpu_util.cu": [],
     "nekgpu_noalloc.cu": [],

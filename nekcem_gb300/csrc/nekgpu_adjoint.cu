@@ -1,4 +1,4 @@
-// Discrete adjoint of the FP64 fused stage (nekgpu_fused.cu, T = double) with
+// Discrete adjoint of the FP64 fused stage (nekgpu_fp64.cu) with
 // respect to the state and to the permittivity eps at every node.
 //
 // Forward stage i (src/cem_maxwell.F:484-508, src/cem_common.F:18-75):
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(ACfg<NX>::NT) k_adjoint_stage(const AdjointDev
     if (vi == 0) add(3, vj + NX * vk);
     if (vk == 0) add(4, vi + NX * vj);
     if (vk == NX - 1) add(5, vi + NX * vj);
-    const double cH = a.b_next * a.coef[g], cE = a.b_next * a.coef[P + g];
+    const double cH = a.bdt_next * a.hbm1[g], cE = a.bdt_next * a.ebm1[g];
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
       a.ub_out[c * P + g] = out[c];
@@ -250,20 +250,12 @@ __global__ void __launch_bounds__(ACfg<NX>::NT) k_adjoint_stage(const AdjointDev
   }
 }
 
-__global__ void k_adjoint_seed(double* w, const double* ub, const double* coef, long P, double b) {
+__global__ void k_adjoint_seed(double* w, const double* ub, const double* hbm1, const double* ebm1,
+                               long P, double bdt) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= 6 * P) return;
   const long g = i % P;
-  w[i] = b * coef[(i < 3 * P ? 0 : P) + g] * ub[i];
-}
-
-// dt hbm1 | dt ebm1: the same product the fused FP64 form's coefficient
-// scaling forms from its unnormalised base
-__global__ void k_adjoint_coef64(double* coef, const double* hbm1, const double* ebm1, long P,
-                                 double dt) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= 2 * P) return;
-  coef[i] = dt * (i < P ? hbm1[i] : ebm1[i - P]);
+  w[i] = bdt * (i < 3 * P ? hbm1[g] : ebm1[g]) * ub[i];
 }
 
 template <int NX>
@@ -305,17 +297,10 @@ int adjoint_stage(Context* c, const AdjointDev& a) {
   }
 }
 
-int adjoint_seed(Context* c, double* w, const double* ub, const double* coef, double b) {
+int adjoint_seed(Context* c, double* w, const double* ub, double bdt) {
   const long n = 6 * c->npts;
-  k_adjoint_seed<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(w, ub, coef, c->npts, b);
-  c->last_launches += 1;
-  return check_cuda(cudaGetLastError());
-}
-
-int adjoint_coef64(Context* c, double* coef, double dt) {
-  const long n = c->npts;
-  k_adjoint_coef64<<<(unsigned)((2 * n + 255) / 256), 256, 0, c->stream>>>(coef, c->d_hbm1,
-                                                                           c->d_ebm1, n, dt);
+  k_adjoint_seed<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(w, ub, c->d_hbm1, c->d_ebm1,
+                                                                     c->npts, bdt);
   c->last_launches += 1;
   return check_cuda(cudaGetLastError());
 }

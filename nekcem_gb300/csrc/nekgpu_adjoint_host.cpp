@@ -85,13 +85,7 @@ int build_adjoint_data(Context* c) {
       check_cuda(cudaMemcpy(nbr.data(), c->d_nbr, nbr.size() * sizeof(int), cudaMemcpyDeviceToHost)))
     return NEKGPU_ERR_CUDA;
   const double C0 = c->fargs.C0;
-  if (c->form == NEKGPU_MIXED) {
-    fc = c->host_fcoef64;  // the device holds float pairs
-  } else if (c->d_fcoef) {
-    fc.resize(4 * (size_t)nxzfl);
-    if (check_cuda(cudaMemcpy(fc.data(), c->d_fcoef, fc.size() * 8, cudaMemcpyDeviceToHost)))
-      return NEKGPU_ERR_CUDA;
-  }
+  fc = c->host_fcoef64;  // the device's copies are pairs, or scaled
   auto coef = [&](long j, int q) {
     const double def[4] = {-0.5, 0.5 * C0, 0.5, 0.5 * C0};
     return fc.empty() ? def[q] : fc[4 * j + q];
@@ -253,12 +247,12 @@ struct HostSlots {
 
 // forward stages in the context's form
 int fwd_stage(Context* c, int r, double t, double dt) {
-  return c->form == NEKGPU_MIXED ? mixed_stage(c, r, t, dt) : fused_stage(c, r, t, dt);
+  return c->form == NEKGPU_MIXED ? mixed_stage(c, r, t, dt) : fp64_stage(c, r, t, dt);
 }
 int fwd_stage_buffers(Context* c, int r, double t, double dt, const double* u_in, double* u_out,
                       double* k_in, double* k_out) {
   return c->form == NEKGPU_MIXED ? mixed_stage_buffers(c, r, t, dt, u_in, u_out, k_in, k_out)
-                                 : fused_stage_buffers(c, r, t, dt, u_in, u_out, k_in, k_out);
+                                 : fp64_stage_buffers(c, r, t, dt, u_in, u_out, k_in, k_out);
 }
 
 }  // namespace
@@ -300,7 +294,6 @@ struct Sweep {
   double* ub[2];
   double* wb[2];
   double* deps;
-  const double* coef64 = nullptr;  // dt hbm1 | dt ebm1 in FP64
   int cu = 0;
   AdjointDev a{};
   double J = 0.0;
@@ -330,7 +323,7 @@ struct Sweep {
       return NEKGPU_ERR_CUDA;
     cu = 0;
     seeded = true;
-    return adjoint_seed(c, wb[0], ub[0], coef64, c->rk_b[4]);
+    return adjoint_seed(c, wb[0], ub[0], c->rk_b[4] * dt);
   }
 
   // the five reverse stages of step j from its stage states (U[0..4]) and
@@ -345,7 +338,7 @@ struct Sweep {
       a.k_cur = K[r];
       a.k_prev = K[r - 1];
       a.a = c->rk_a[r - 1];
-      a.b_next = c->rk_b[r == 1 ? 4 : r - 2];
+      a.bdt_next = c->rk_b[r == 1 ? 4 : r - 2] * dt;
       int st = adjoint_stage(c, a);
       if (st) return st;
       cu ^= 1;
@@ -356,7 +349,8 @@ struct Sweep {
   void init_args() {
     a.nelt = c->nelt;
     a.npts = c->npts;
-    a.coef = coef64;
+    a.hbm1 = c->d_hbm1;
+    a.ebm1 = c->d_ebm1;
     a.bm1 = c->d_bm1;
     a.deps = deps;
     a.nbr = c->d_nbr;
@@ -465,17 +459,16 @@ extern "C" int nekgpu_adjoint_gradient(nekgpu_ctx* c, int nsteps, double t0, dou
   // sqrt scheme: ceil(n/S) checkpoints + sets x 2 x (5S+1) segment states +
   // 4 adjoint states; binomial scheme: 4 adjoint + 10 stage + 1 scratch
   // states + device snapshots (+ the pinned host snapshots allowed by
-  // nekgpu_adjoint_host_snapshots).  Both also hold dJ/deps (npts doubles)
-  // and, for the mixed form, the FP64 inverse-mass scale (2 npts doubles).
+  // nekgpu_adjoint_host_snapshots).  Both also hold dJ/deps (npts doubles).
   // stride > 0: segments of `stride` steps; 0: sqrt(steps) segments if they
   // fit, else the binomial schedule with the snapshots that fit; < 0: the
   // binomial schedule with -stride device snapshots.
   // fused FP64 with mixed recomputation: the mixed stage arguments of the
-  // context (coefficient pairs and their FP64 base, 32 B per face node of
-  // face coefficient pairs) -- about 32 + 4.5 * 6/nx bytes per node
+  // context (coefficient pairs, and 32 B per face node of face coefficient
+  // pairs)
   const bool hybrid = !mixed && c->adj_mixed_recompute;
-  const double hybrid_b = hybrid ? (32.0 + 32.0 * 6.0 / c->nx) * npts : 0.0;
-  const double avail = (double)adjoint_budget(c) - (double)npts * 8 - (mixed ? 16.0 * npts : 0.0) - hybrid_b;
+  const double hybrid_b = hybrid ? (16.0 + 32.0 * 6.0 / c->nx) * npts : 0.0;
+  const double avail = (double)adjoint_budget(c) - (double)npts * 8 - hybrid_b;
   const int S = stride > 0 ? stride : (int)std::ceil(std::sqrt((double)nsteps));
   const int nseg = (nsteps + S - 1) / S;
   auto sqrt_states = [&](int sets) { return (double)nseg + 4.0 + sets * 2.0 * (5.0 * S + 1.0); };
@@ -511,15 +504,7 @@ extern "C" int nekgpu_adjoint_gradient(nekgpu_ctx* c, int nsteps, double t0, dou
   w.wb[1] = mem.get(ns);
   w.deps = mem.get(npts);
   if (!w.ub[0] || !w.ub[1] || !w.wb[0] || !w.wb[1] || !w.deps) return NEKGPU_ERR_NOMEM;
-  if (mixed) {  // the context's coefficients are float pairs: an FP64 copy for the reverse
-    double* cf = mem.get(2 * npts);
-    if (!cf) return NEKGPU_ERR_NOMEM;
-    if ((st = scale_coef_pairs(c, dt)) || (st = adjoint_coef64(c, cf, dt))) return st;
-    w.coef64 = cf;
-  } else {
-    if ((st = scale_coef(c, dt))) return st;
-    w.coef64 = c->d_coef;
-  }
+  if ((st = mixed ? scale_coef_pairs(c, dt) : scale_coef(c, dt))) return st;
   w.init_args();
   float f_ms = 0, a_ms = 0;
 

@@ -1,0 +1,725 @@
+// Fused FP64 stage on affine axis-aligned hexahedra (NEKGPU_FUSED64): weighted
+// curl (src/nek5_grad.F:2-19, src/cem_maxwell.F:1428-1497), upwind face flux
+// with the in-kernel partner read that replaces gs_op_fields
+// (src/cem_maxwell.F:922-1002, 1368-1426), lift (src/cem_maxwell.F:725-735),
+// PML, dispersive currents, incident fields, graphene sheets, volume source,
+// inverse mass (src/cem_maxwell.F:1878-1886) and the low-storage RK update
+// (src/cem_common.F:18-75), one kernel per stage.
+//
+// What bounds it: GB300 issues two FP64 lanes per clock and SM.  With the
+// contractions in FP64 (96 of its ~165 operations per node at N=7) a stage of
+// the 16^3-element N=7 box took 690 us; it takes 223 us (56 G DOF-stage
+// updates/s, FP64 pipe 61 % busy) with
+//  * the contractions in 64-bit integer arithmetic (nekgpu_fixed.cuh) on
+//    another pipe, one thread per GLL line, D as constant-bank operands;
+//  * the residual normalised by w3*rx as in the mixed form, so that the curl
+//    takes one FP64 multiply-add per derivative at most (none for the r-lines),
+//    the lift factor is part of the face coefficients, and w3 is folded into
+//    the inverse-mass coefficient;
+//  * only the four field components tangential to a face in its flux.
+// About 40 FP64 operations per node are left (finish 18, curl 8, flux 12): 20
+// of the 33 clocks per node and SM.
+//
+// Phases per element: state to shared memory (8-byte asynchronous copies into
+// an odd row length), flux per face node, two phases of line tasks into the
+// residual, then node by node the finish.  The split form gives an element's
+// k-slabs to several blocks, for meshes with fewer elements than SMs: every
+// block stages the whole element (the t-lines need it) and works out the
+// nodes of its slab, so the blocks share nothing.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "nekgpu_fixed.cuh"
+#include "nekgpu_internal.h"
+
+namespace nekgpu {
+
+namespace {
+
+__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
+__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
+__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
+constexpr int cmax(int a, int b) { return a > b ? a : b; }
+constexpr int round32(int a) { return (a + 31) / 32 * 32; }
+
+template <int NX>
+__device__ __forceinline__ int face_vol(int f, int a, int b) {
+  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
+  const int ax = slot_axis(f);
+  return ax == 0 ? fixed + NX * a + NX * NX * b
+                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
+}
+
+// x with its sign flipped where neg (no FP64 instruction)
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+template <int NX>
+struct DCfg {
+  static constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
+  // node (i,j,k) of the element arrays at i + RS*j + SZ*k, an odd row length:
+  // lines in every direction are read with at most two threads of a half warp
+  // on a bank
+  static constexpr int RS = NX | 1, SZ = RS * NX, N3P = NX * SZ;
+  static constexpr int NT = NX == 9 ? 384 : (NX == 8 ? 256 : round32(cmax(3 * N2, (N3 + 1) / 2)));
+  static constexpr int FPT = (NF + NT - 1) / NT;
+  // state, residual, flux [face][line slot][N2], D rows (split form)
+  static constexpr size_t off_R = 6 * (size_t)N3P * 8, off_F = 2 * off_R;
+  static constexpr size_t off_D = (off_F + 24 * (size_t)N2 * 8 + 15) / 16 * 16;
+  static constexpr size_t smem(bool split) { return off_D + (split ? N2 * 16 : 0); }
+};
+
+// The line types of the two contraction phases: the first starts each of the
+// six residual components, the second completes it, so a phase has six
+// component-lines per line and one barrier ends it.  Residual index 0..2 =
+// H1..H3 (-curl E), 3..5 = E1..E3 (curl H); field 0..2 = H, 3..5 = E:
+//   E1 = ds Hz - dt Hy   E2 = dt Hx - dr Hz   E3 = dr Hy - ds Hx
+//   H1 = dt Ey - ds Ez   H2 = dr Ez - dt Ex   H3 = ds Ex - dr Ey
+// slot: the type's place among the four flux components of a face normal to
+// its direction.
+struct LineType {
+  int dir, comp, res, neg, slot;
+};
+__constant__ const LineType kLine[2][6] = {
+    {{0, 1, 5, 0, 0}, {0, 2, 4, 1, 1}, {0, 4, 2, 1, 2}, {0, 5, 1, 0, 3}, {1, 2, 3, 0, 1}, {1, 5, 0, 1, 3}},
+    {{1, 0, 5, 1, 0}, {1, 3, 2, 0, 2}, {2, 0, 4, 0, 0}, {2, 1, 3, 1, 1}, {2, 3, 1, 1, 2}, {2, 4, 0, 0, 3}}};
+
+template <int NX>
+__device__ __forceinline__ int pnode(int v) {  // stored index of node v = i + NX*j + NX^2*k
+  return (v % NX) + DCfg<NX>::RS * ((v / NX) % NX) + DCfg<NX>::SZ * (v / (NX * NX));
+}
+
+// Field component of the k-th partner value of face f: all six with the
+// extension terms, else H and E along the two axes tangential to f.
+template <bool EXT>
+__device__ __forceinline__ int partner_comp(int f, int k) {
+  if (EXT) return k;
+  const int ax = slot_axis(f);
+  const int tang = (k & 1) ? (ax == 2 ? 1 : 2) : (ax == 0 ? 1 : 0);
+  return (k < 2 ? 0 : 3) + tang;
+}
+
+// The part of an element a block works out: its nodes with k in [k0, k1).
+struct Slab {
+  int k0, k1;
+};
+
+// Face task t of the slab: slot f and in-face node (a, b)
+template <int NX, bool SPLIT>
+__device__ __forceinline__ int face_tasks(Slab s) {
+  if (!SPLIT) return 6 * NX * NX;
+  return 4 * NX * (s.k1 - s.k0) + (s.k0 == 0 ? NX * NX : 0) + (s.k1 == NX ? NX * NX : 0);
+}
+template <int NX, bool SPLIT>
+__device__ __forceinline__ void face_task(Slab s, int t, int& f, int& a, int& b) {
+  constexpr int N2 = NX * NX;
+  if (!SPLIT) {
+    f = t / N2;
+    a = t % NX;
+    b = (t - f * N2) / NX;
+    return;
+  }
+  const int per = NX * (s.k1 - s.k0);
+  if (t < 4 * per) {  // the side faces: rows b = k of the slab
+    f = t / per;
+    const int ab = t - f * per;
+    a = ab % NX;
+    b = s.k0 + ab / NX;
+    return;
+  }
+  t -= 4 * per;
+  f = s.k0 == 0 && t < N2 ? 4 : 5;
+  if (f == 5 && s.k0 == 0) t -= N2;
+  a = t % NX;
+  b = t / NX;
+}
+
+// One output x of a line task into the residual: the r-lines (OP 0) start
+// their components, whose derivative has coefficient one; the s-lines of
+// phase 0 (OP 1) start theirs times rho; phase 1 (OP 2) completes all six.  F
+// is the lifted flux at a line's end.
+template <int OP>
+__device__ __forceinline__ void line_put(double* Rp, double x, bool neg, double rho, bool end, double F) {
+  double v;
+  if (OP == 0) {
+    v = flip(x, neg);
+    if (end) v += F;
+  } else if (OP == 1) {
+    v = fma(flip(rho, neg), x, end ? F : 0.0);
+  } else {
+    v = fma(flip(rho, neg), x, *Rp);
+    if (end) v += F;
+  }
+  *Rp = v;
+}
+
+// Line type `type` of phase PH along line lam: outputs [i0, i1) (all of them
+// unless SPLIT, which takes D's rows from shared memory instead of the
+// constant bank).
+template <int NX, int PH, int OP, bool SPLIT>
+__device__ __forceinline__ void line_task(int type, int lam, int i0, int i1, const double* s_u,
+                                          double* s_R, const double* s_F, const int4* s_D,
+                                          double rho_s, double rho_t, const Fp64Dev& a) {
+  using C = DCfg<NX>;
+  constexpr int N2 = C::N2;
+  const LineType& lt = kLine[PH][type];
+  const int dir = lt.dir;
+  const bool neg = lt.neg != 0;
+  const int la = lam % NX, lb = lam / NX;
+  const int base = dir == 0 ? C::RS * la + C::SZ * lb : (dir == 1 ? la + C::SZ * lb : la + C::RS * lb);
+  const int step = dir == 0 ? 1 : (dir == 1 ? C::RS : C::SZ);
+  const double rho = dir == 2 ? rho_t : rho_s;
+  const double* pu = s_u + lt.comp * C::N3P + base;
+  double* R = s_R + lt.res * C::N3P + base;
+  // faces 3|1 (r), 0|2 (s), 4|5 (t)
+  const double* Fm = s_F + ((dir == 0 ? 3 : (dir == 1 ? 0 : 4)) * 4 + lt.slot) * N2 + lam;
+  const double* Fp = s_F + ((dir == 0 ? 1 : (dir == 1 ? 2 : 5)) * 4 + lt.slot) * N2 + lam;
+  FixedLine<NX> f;
+  {
+    double u[NX];
+#pragma unroll
+    for (int l = 0; l < NX; ++l) u[l] = pu[step * l];
+    fixed_line<NX>(u, f);
+  }
+  auto put = [&](int i, double x) {
+    const bool end = i == 0 || i == NX - 1;
+    line_put<OP>(R + step * i, x, neg, rho, end, end ? (i == 0 ? *Fm : *Fp) : 0.0);
+  };
+  if (a.fd.ok && !f.special) {
+    if (!SPLIT) {
+#pragma unroll
+      for (int i = 0; i < NX; ++i)
+        put(i, fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
+              hi = a.fd.hi[i + NX * l];
+              lo = a.fd.lo[i + NX * l];
+              hi8 = a.fd.hi8[i + NX * l];
+            }));
+    } else {
+#pragma unroll 1
+      for (int i = i0; i < i1; ++i)
+        put(i, fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
+              const int4 d = s_D[i + NX * l];
+              hi = d.x;
+              lo = d.y;
+              hi8 = d.z;
+            }));
+    }
+  } else {  // a line out of the integer form's range: in FP64
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i) {
+      double x = a.D[i] * pu[0];
+#pragma unroll 1
+      for (int l = 1; l < NX; ++l) x = fma(a.D[i + NX * l], pu[step * l], x);
+      put(i, x);
+    }
+  }
+}
+
+// Phase PH of the contractions over the slab: tasks (line type, line), in the
+// split form (type, group of og outputs, line).
+template <int NX, int PH, bool SPLIT>
+__device__ __forceinline__ void line_phase(const double* s_u, double* s_R, const double* s_F,
+                                           const int4* s_D, double rho_s, double rho_t, Slab sl,
+                                           int og, const Fp64Dev& a) {
+  using C = DCfg<NX>;
+  constexpr int N2 = C::N2, NT = C::NT;
+  const int tid = threadIdx.x;
+  if constexpr (!SPLIT) {
+    constexpr int NA = PH == 0 ? 4 : 6;  // types of the phase's first operation
+#pragma unroll 1
+    for (int task = tid; task < NA * N2; task += NT) {
+      const int type = task / N2;
+      line_task<NX, PH, PH == 0 ? 0 : 2, false>(type, task - type * N2, 0, NX, s_u, s_R, s_F, s_D,
+                                                rho_s, rho_t, a);
+    }
+    if (PH == 0) {
+      // the other two types, starting with the threads the first four left idle
+      constexpr int off = (NA * N2) % NT;
+#pragma unroll 1
+      for (int task = tid >= off ? tid - off : tid + NT - off; task < 2 * N2; task += NT) {
+        const int type = task / N2;
+        line_task<NX, 0, 1, false>(NA + type, task - type * N2, 0, NX, s_u, s_R, s_F, s_D, rho_s,
+                                   rho_t, a);
+      }
+    }
+  } else {
+    // r and s types run along the slab's lines, t types along all lines
+    const int nl = NX * (sl.k1 - sl.k0), nrs = nl * ((NX + og - 1) / og);
+    const int nt = N2 * ((sl.k1 - sl.k0 + og - 1) / og);
+    const int nrt = PH == 0 ? 6 : 2;
+    const int ntask = nrt * nrs + (6 - nrt) * nt;
+#pragma unroll 1
+    for (int task = tid; task < ntask; task += NT) {
+      if (PH == 0 || task < 2 * nrs) {
+        const int type = task / nrs, q = task - type * nrs, grp = q / nl;
+        const int lam = q - grp * nl + NX * sl.k0, i0 = grp * og, i1 = min(NX, i0 + og);
+        if (PH == 0 && type < 4)
+          line_task<NX, 0, 0, true>(type, lam, i0, i1, s_u, s_R, s_F, s_D, rho_s, rho_t, a);
+        else
+          line_task<NX, PH, PH == 0 ? 1 : 2, true>(type, lam, i0, i1, s_u, s_R, s_F, s_D, rho_s, rho_t, a);
+      } else {
+        const int q0 = task - 2 * nrs, type = q0 / nt, q = q0 - type * nt, grp = q / N2;
+        const int i0 = sl.k0 + grp * og, i1 = min(sl.k1, i0 + og);
+        line_task<NX, 1, 2, true>(2 + type, q - grp * N2, i0, i1, s_u, s_R, s_F, s_D, rho_s, rho_t, a);
+      }
+    }
+  }
+}
+
+// PML (pml_step, src/cem_maxwell_pml.F:508-590) at one node of a PML element:
+// the auxiliary residuals from res/bm1 = R * (w3 rx / bm1), their RK update
+// (src/cem_maxwell.F:1942-1955), and the PML terms added to R.
+template <int N3>
+__device__ __forceinline__ void pml_node(const Fp64Dev& a, int l, int v, const double* u,
+                                         bool first_stage, double* R) {
+  const long nn = a.pml.n, q = (long)l * N3 + v;
+  const double* pd = a.pml.data;
+  const double sxp = pd[q], syp = pd[nn + q], szp = pd[2 * nn + q];
+  const double sigx = pd[3 * nn + q], sigy = pd[4 * nn + q], sigz = pd[5 * nn + q];
+  const double mu = pd[6 * nn + q], fac = pd[9 * nn + q], inv = pd[10 * nn + q];
+  double* aux = a.pml.aux;
+  double* kx = a.pml.k;
+  const double bn[3] = {aux[q], aux[nn + q], aux[2 * nn + q]};
+  const double dn[3] = {aux[3 * nn + q], aux[4 * nn + q], aux[5 * nn + q]};
+  double rp[6], t[6];
+  rp[0] = R[0] * fac - syp * bn[0];
+  rp[1] = R[1] * fac - szp * bn[1];
+  rp[2] = R[2] * fac - sxp * bn[2];
+  rp[3] = R[3] * fac - syp * dn[0];
+  rp[4] = R[4] * fac - szp * dn[1];
+  rp[5] = R[5] * fac - sxp * dn[2];
+  t[0] = -syp * bn[0] + sxp * bn[0] - szp * mu * u[0];
+  t[1] = -szp * bn[1] + syp * bn[1] - sxp * mu * u[1];
+  t[2] = -sxp * bn[2] + szp * bn[2] - syp * mu * u[2];
+  t[3] = -syp * dn[0] + sxp * dn[0] - sigz * u[3];
+  t[4] = -szp * dn[1] + syp * dn[1] - sigx * u[4];
+  t[5] = -sxp * dn[2] + szp * dn[2] - sigy * u[5];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    R[c] += t[c] * inv;  // res += t bm1
+    const double kv = first_stage ? a.dt * rp[c] : fma(a.a, kx[c * nn + q], a.dt * rp[c]);
+    kx[c * nn + q] = kv;
+    aux[c * nn + q] = fma(a.b, kv, c < 3 ? bn[c] : dn[c - 3]);
+  }
+}
+
+// Dispersive currents inside usersrc (cem_maxwell_drude / cem_maxwell_lorentz,
+// src/cem_maxwell.F:3095-3212): resE -= J1 bm1, the currents' RK update.
+template <int N3>
+__device__ __forceinline__ void disp_node(const Fp64Dev& a, int l, int v, const double* u,
+                                          bool first_stage, double* R) {
+  const DispDev& d = a.disp;
+  const long nn = d.n, q = (long)l * N3 + v;
+  const int kind = (int)d.data[q];
+  if (kind == 0) return;
+  const double pa = d.data[nn + q], pb = d.data[2 * nn + q], pc = d.data[3 * nn + q];
+  const double inv = d.data[5 * nn + q];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double j1 = d.aux[c * nn + q], ev = u[3 + c];
+    R[3 + c] -= j1 * inv;
+    double r1 = -pa * j1 + pb * ev;
+    if (kind == 2) {
+      const double j2 = d.aux[(3 + c) * nn + q];
+      r1 = -pa * j1 - pb * j2 + pc * ev;
+      const double k2 = first_stage ? a.dt * j1 : fma(a.a, d.k[(3 + c) * nn + q], a.dt * j1);
+      d.k[(3 + c) * nn + q] = k2;
+      d.aux[(3 + c) * nn + q] = fma(a.b, k2, j2);
+    }
+    const double k1 = first_stage ? a.dt * r1 : fma(a.a, d.k[c * nn + q], a.dt * r1);
+    d.k[c * nn + q] = k1;
+    d.aux[c * nn + q] = fma(a.b, k1, j1);
+  }
+}
+
+// Incident field (userinc) and graphene sheet (userfsrc) terms of face node t
+// of element e in its jumps JH, JE.
+template <int NX>
+__device__ __noinline__ void face_extras(const Fp64Dev& a, int e, int t, int f, int pe,
+                                         const double* h, const double* ev, const double* hp,
+                                         const double* ep, bool first_stage, double* JH, double* JE) {
+  constexpr int NF = DCfg<NX>::NF;
+  double hm[3], em[3], hq[3], eq[3];
+  for (int c = 0; c < 3; ++c) {
+    hm[c] = h[c];
+    em[c] = ev[c];
+    hq[c] = hp[c];
+    eq[c] = ep[c];
+  }
+  const int io = a.inc_elem ? a.inc_elem[e] : -1;
+  if (io >= 0) {
+    // the incident field on the own side of a listed face node, or on the
+    // partner's side when the partner's slot is listed
+    const double* iv = a.inc_val + (long)io * 12 * NF + t;
+    for (int c = 0; c < 3; ++c) {
+      hm[c] += iv[c * NF];
+      em[c] += iv[(3 + c) * NF];
+      hq[c] += iv[(6 + c) * NF];
+      eq[c] += iv[(9 + c) * NF];
+    }
+  }
+  for (int c = 0; c < 3; ++c) {
+    JH[c] = pe >= 0 ? hq[c] - hm[c] : 0.0;
+    JE[c] = pe >= 0 ? eq[c] - em[c] : -2.0 * em[c];
+  }
+  if (!a.gr.elem) return;
+  // the sheet's currents on both sides of the face node enter as
+  // n x [H] - J, i.e. [H] + n x J
+  const int gr = a.gr.elem[e];
+  const int go = gr >= 0 ? a.gr.own[(long)gr * NF + t] : -1;
+  const int gp = gr >= 0 ? a.gr.part[(long)gr * NF + t] : -1;
+  if (go < 0 && gp < 0) return;
+  double nv[3], nm[3], J[3] = {0.0, 0.0, 0.0};
+  for (int c = 0; c < 3; ++c) {
+    nv[c] = c == slot_axis(f) ? (double)slot_side(f) : 0.0;
+    nm[c] = -nv[c];
+  }
+  if (go >= 0) graphene_slot(a.gr, go, nv, hm, em, true, first_stage, a.a, a.b, a.dt, J);
+  if (gp >= 0 && pe >= 0) graphene_slot(a.gr, gp, nm, hq, eq, false, first_stage, a.a, a.b, a.dt, J);
+  if (pe >= 0) {  // a PEC face keeps its mirror flux
+    JH[0] += nv[1] * J[2] - nv[2] * J[1];
+    JH[1] += nv[2] * J[0] - nv[0] * J[2];
+    JH[2] += nv[0] * J[1] - nv[1] * J[0];
+  }
+}
+
+template <int NX, bool EXT>
+constexpr int fp64_min_blocks() {
+  return NX == 9 || EXT ? 2 : (NX == 8 ? 3 : 4);
+}
+
+template <int NX, bool EXT, bool SPLIT>
+__global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
+    k_fp64_stage(const __grid_constant__ Fp64Dev a, int nsplit, int og) {
+  using C = DCfg<NX>;
+  constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF;
+  constexpr int NPC = EXT ? 6 : 4;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* s_u = reinterpret_cast<double*>(smem);
+  double* s_R = reinterpret_cast<double*>(smem + C::off_R);
+  double* s_F = reinterpret_cast<double*>(smem + C::off_F);
+  int4* s_D = reinterpret_cast<int4*>(smem + C::off_D);
+  const int tid = threadIdx.x;
+  const long P = a.npts;
+  const bool first_stage = (a.a == 0.0);  // rk4a(1) = 0: k restarts
+  if (SPLIT)
+    for (int t = tid; t < N2; t += NT) s_D[t] = make_int4(a.fd.hi[t], a.fd.lo[t], a.fd.hi8[t], 0);
+  // a programmatic dependent of the previous stage: nothing it wrote is read
+  // before it has completed; the next stage may launch from the last task on
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const int ntask = SPLIT ? a.nelt * nsplit : a.nelt;
+  for (int w = blockIdx.x; w < ntask; w += gridDim.x) {
+    if (w + (int)gridDim.x >= ntask) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int e = SPLIT ? w / nsplit : w;
+    Slab sl{0, NX};
+    if (SPLIT) {
+      const int q = w - e * nsplit;
+      sl = Slab{q * NX / nsplit, (q + 1) * NX / nsplit};
+    }
+    const int* nbr = a.nbr + 6 * (long)e;
+    const double* eg = a.egn + 14 * (long)e;
+    // ---- own state to shared memory, partner face values to registers --------
+    for (int v = tid; v < N3; v += NT) {
+      const int pv = pnode<NX>(v);
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+        cp_async8(s_u + c * C::N3P + pv, a.u_in + c * P + (long)e * N3 + v);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    // what the finish reads, and the next element's state, on their way to L2
+    if (!SPLIT) {
+      const int en = w + (int)gridDim.x < ntask ? w + gridDim.x : e;
+#pragma unroll 1
+      for (int t = tid; t < 14 * ((N3 + 15) / 16); t += NT) {
+        const int q = t / ((N3 + 15) / 16), o = 16 * (t - q * ((N3 + 15) / 16));
+        const double* p = q < 6 ? a.u_in + q * P + (long)en * N3
+                                : (q < 12 ? a.k + (q - 6) * P : a.coef + (q - 12) * P) + (long)e * N3;
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p + o));
+      }
+    }
+    const int nft = face_tasks<NX, SPLIT>(sl);
+    double nbv[C::FPT][NPC];
+#pragma unroll
+    for (int q = 0; q < C::FPT; ++q) {
+      const int t = tid + q * NT;
+      if (t < nft) {
+        int f, fa, fb;
+        face_task<NX, SPLIT>(sl, t, f, fa, fb);
+        const int pe = nbr[f];
+        if (pe >= 0) {
+          const long pv = (long)pe * N3 + face_vol<NX>(slot_opp(f), fa, fb);
+#pragma unroll
+          for (int k = 0; k < NPC; ++k) nbv[q][k] = __ldg(a.u_in + partner_comp<EXT>(f, k) * P + pv);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    // ---- upwind flux per face node, lifted, into s_F ---------------------------
+#pragma unroll
+    for (int q = 0; q < C::FPT; ++q) {
+      const int t = tid + q * NT;
+      if (t >= nft) continue;
+      int f, fa, fb;
+      face_task<NX, SPLIT>(sl, t, f, fa, fb);
+      const int j = f * N2 + fa + NX * fb;
+      const int pv = pnode<NX>(face_vol<NX>(f, fa, fb));
+      const int pe = nbr[f];
+      const int ax = slot_axis(f);
+      // the tangential axes ta < tb; jumps partner - own (PEC mirror: [H] = 0,
+      // [E] = -2 E)
+      const int ta = ax == 0 ? 1 : 0, tb = ax == 2 ? 1 : 2;
+      double JHa, JHb, JEa, JEb;
+      if (EXT) {
+        double h[3], ev[3], JH[3], JE[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          h[c] = s_u[c * C::N3P + pv];
+          ev[c] = s_u[(3 + c) * C::N3P + pv];
+          JH[c] = pe >= 0 ? nbv[q][c] - h[c] : 0.0;
+          JE[c] = pe >= 0 ? nbv[q][EXT ? 3 + c : 0] - ev[c] : -2.0 * ev[c];
+        }
+        if (a.inc_elem || a.gr.elem) {
+          double hp[3], ep[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            hp[c] = pe >= 0 ? nbv[q][c] : 0.0;
+            ep[c] = pe >= 0 ? nbv[q][EXT ? 3 + c : 0] : 0.0;
+          }
+          face_extras<NX>(a, e, j, f, pe, h, ev, hp, ep, first_stage, JH, JE);
+        }
+        JHa = ax == 0 ? JH[1] : JH[0];
+        JHb = ax == 2 ? JH[1] : JH[2];
+        JEa = ax == 0 ? JE[1] : JE[0];
+        JEb = ax == 2 ? JE[1] : JE[2];
+      } else {
+        const double ea = s_u[(3 + ta) * C::N3P + pv], eb = s_u[(3 + tb) * C::N3P + pv];
+        if (pe >= 0) {
+          JHa = nbv[q][0] - s_u[ta * C::N3P + pv];
+          JHb = nbv[q][1] - s_u[tb * C::N3P + pv];
+          JEa = nbv[q][2] - ea;
+          JEb = nbv[q][3] - eb;
+        } else {
+          JHa = JHb = 0.0;
+          JEa = -2.0 * ea;
+          JEb = -2.0 * eb;
+        }
+      }
+      // In the line slot order of the face's direction (residuals 5,4,2,1 |
+      // 5,3,2,0 | 4,3,1,0), with s = side for faces normal to r and t, -side
+      // for s:  F0 = s Z JHa + CZ JEb,  F1 = -s Z JHb + CZ JEa,
+      //         F2 = s Y JEa + CY JHb,  F3 = -s Y JEb + CY JHa,
+      // the coefficients times the lift factor (uniform media: Y = -1/2,
+      // Z = 1/2, CY = CZ = C0/2).
+      const bool neg = (slot_side(f) < 0) != (ax == 1);
+      double2 cy, cz;
+      if (a.fcoef) {
+        const double2* fc = reinterpret_cast<const double2*>(a.fcoef + 4 * ((long)e * NF + j));
+        cy = fc[0];
+        cz = fc[1];
+      } else {
+        cz = make_double2(eg[2 + f], eg[8 + f]);
+        cy = make_double2(flip(cz.x, true), cz.y);
+      }
+      double* Fo = s_F + f * 4 * N2 + fa + NX * fb;
+      Fo[0] = fma(cz.x, flip(JHa, neg), cz.y * JEb);
+      Fo[N2] = fma(cz.x, flip(JHb, !neg), cz.y * JEa);
+      Fo[2 * N2] = fma(cy.x, flip(JEa, neg), cy.y * JHb);
+      Fo[3 * N2] = fma(cy.x, flip(JEb, !neg), cy.y * JHa);
+    }
+    __syncthreads();
+    const double rho_s = eg[0], rho_t = eg[1];
+    line_phase<NX, 0, SPLIT>(s_u, s_R, s_F, s_D, rho_s, rho_t, sl, og, a);
+    __syncthreads();
+    line_phase<NX, 1, SPLIT>(s_u, s_R, s_F, s_D, rho_s, rho_t, sl, og, a);
+    __syncthreads();
+    // ---- PML, currents, source, inverse mass, RK update, node by node ----------
+    const int so = a.src_elem ? a.src_elem[e] : -1;
+    const int pml_l = (EXT && a.pml.slot) ? a.pml.slot[e] : -1;
+    const int disp_l = (EXT && a.disp.slot) ? a.disp.slot[e] : -1;
+#pragma unroll 1
+    for (int v = tid + sl.k0 * N2; v < sl.k1 * N2; v += NT) {
+      const int pv = pnode<NX>(v);
+      const long g = (long)e * N3 + v;
+      double R[6], u[6], kk[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) kk[c] = first_stage ? 0.0 : a.k[c * P + g];
+      const double ch = a.coef[g], ce = a.coef[P + g];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        R[c] = s_R[c * C::N3P + pv];
+        u[c] = s_u[c * C::N3P + pv];
+      }
+      if (EXT && pml_l >= 0) pml_node<N3>(a, pml_l, v, u, first_stage, R);
+      if (EXT && disp_l >= 0) disp_node<N3>(a, disp_l, v, u, first_stage, R);
+      if (so >= 0) R[5] = fma(a.src_w[(long)so * N3 + v], a.src_ft, R[5]);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        const double r = R[c] * (c < 3 ? ch : ce);
+        const double kn = first_stage ? r : fma(a.a, kk[c], r);
+        a.k_out[c * P + g] = kn;
+        a.u_out[c * P + g] = fma(a.b, kn, u[c]);
+      }
+    }
+    if (w + (int)gridDim.x < ntask) __syncthreads();  // the element's shared data is consumed
+  }
+}
+
+template <int NX, bool EXT, bool SPLIT>
+int launch(Context* c, const Fp64Dev& a, bool pdl, int nsplit, int og) {
+  using C = DCfg<NX>;
+  constexpr size_t smem = C::smem(SPLIT);
+  auto kern = k_fp64_stage<NX, EXT, SPLIT>;
+  static int grid = 0;
+  if (!grid) {
+    if (check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
+      return NEKGPU_ERR_CUDA;
+    int per_sm = 0;
+    if (check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem)))
+      return NEKGPU_ERR_CUDA;
+    if (per_sm < 1) return NEKGPU_ERR_UNSUPPORTED;
+    grid = per_sm * num_sms(c);
+  }
+  const int n = a.nelt * nsplit, g = n < grid ? n : grid;
+  c->fused_grid = g;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g);
+  cfg.blockDim = dim3(C::NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  if (check_cuda(cudaLaunchKernelEx(&cfg, kern, a, nsplit, og))) return NEKGPU_ERR_CUDA;
+  c->last_launches += 1;
+  return check_cuda(cudaGetLastError());
+}
+
+// Fewer elements than half the SMs: each is split over as many blocks as give
+// one block per SM (27 elements, N=8: 10.0 us per stage in five slabs, 11.3
+// in three or four, 13.0 in eight, 17.8 unsplit; 64 elements, N=7: 10.8 us in
+// two, 12.7 in four, 13.4 unsplit).  With more elements the slabs only repeat
+// the staging and the t-lines' conversions (100 elements, N=7: 13.4 us
+// unsplit, 14.6 in two).
+template <int NX, bool EXT>
+int dispatch_split(Context* c, const Fp64Dev& a, bool pdl) {
+  // outputs per task of a split line: three at NX = 9 (10.0 against 10.6 us
+  // with five), halves otherwise (64 elements, N=7: 10.8 us, 12.1 with three,
+  // 11.4 with two)
+  constexpr int og = NX == 9 ? 3 : (NX + 1) / 2;
+  const int ns = std::min(num_sms(c) / a.nelt, NX);
+  return ns >= 2 ? launch<NX, EXT, true>(c, a, pdl, ns, og) : launch<NX, EXT, false>(c, a, pdl, 1, NX);
+}
+
+template <bool EXT>
+int dispatch(Context* c, const Fp64Dev& a, bool pdl) {
+  switch (c->nx) {
+    case 3: return dispatch_split<3, EXT>(c, a, pdl);
+    case 4: return dispatch_split<4, EXT>(c, a, pdl);
+    case 5: return dispatch_split<5, EXT>(c, a, pdl);
+    case 6: return dispatch_split<6, EXT>(c, a, pdl);
+    case 7: return dispatch_split<7, EXT>(c, a, pdl);
+    case 8: return dispatch_split<8, EXT>(c, a, pdl);
+    case 9: return dispatch_split<9, EXT>(c, a, pdl);
+    default: return NEKGPU_ERR_UNSUPPORTED;
+  }
+}
+
+int fp64_launch(Context* c, Fp64Dev& a, int rkstep, double time, double dt, bool pdl) {
+  a.a = c->rk_a[rkstep - 1];
+  a.b = c->rk_b[rkstep - 1];
+  a.dt = dt;
+  a.src_elem = c->fargs.src_elem;
+  a.src_w = reinterpret_cast<const double*>(c->fargs.src_w);
+  if (c->src.enabled) a.src_ft = source_ft(c->src, time + dt * c->rk_c[rkstep - 1]);
+  const bool ext = a.pml.slot || a.disp.slot || a.inc_elem || a.gr.elem;
+  return ext ? dispatch<true>(c, a, pdl) : dispatch<false>(c, a, pdl);
+}
+
+}  // namespace
+
+// The fixed-point table of D (nekgpu_fixed.cuh): the largest scale 2^kd with
+// |D| 2^kd < 2^59 whose cross sums stay below 2^63 for any line.
+void fixed_table(const double* D, int n, FixedD& t) {
+  t = FixedD{};
+  double dmax = 0.0;
+  bool fine = n <= kMaxFixed;
+  for (int k = 0; k < n * n; ++k) {
+    fine = fine && std::isfinite(D[k]);
+    dmax = std::fmax(dmax, std::fabs(D[k]));
+  }
+  if (!fine || !(dmax > 0.0)) return;
+  int ex = 0;
+  std::frexp(dmax, &ex);  // dmax < 2^ex
+  for (int kd = 59 - ex; kd >= 57 - ex; --kd) {
+    if (kd > 150 || kd < -60) return;
+    bool fits = true;
+    for (int i = 0; i < n && fits; ++i) {
+      double cross = 0.0;
+      for (int l = 0; l < n; ++l) {
+        const int k = i + n * l;
+        const double d = std::ldexp(D[k], kd);
+        const long long m = std::llrint(std::fabs(d));
+        if (m >= (1LL << 59)) fits = false;
+        const int s = d < 0 ? -1 : 1;
+        t.hi[k] = s * (int)(m >> 31);
+        t.lo[k] = s * (int)(m & 0x7FFFFFFF);
+        t.hi8[k] = 8 * t.hi[k];
+        cross += (double)(1 << 28) * (double)(m & 0x7FFFFFFF) + 2147483648.0 * (double)(m >> 31);
+      }
+      fits = fits && cross < 9.2e18;
+    }
+    if (fits) {
+      t.ok = 1;
+      t.bias = 1022 + kd;
+      return;
+    }
+  }
+}
+
+int fp64_stage_buffers(Context* c, int rkstep, double time, double dt, const double* u_in,
+                       double* u_out, const double* k_in, double* k_out) {
+  const int st = scale_coef(c, dt);
+  if (st) return st;
+  Fp64Dev a = c->dargs;
+  a.u_in = u_in;
+  a.u_out = u_out;
+  a.k = k_in;
+  a.k_out = k_out;
+  return fp64_launch(c, a, rkstep, time, dt, false);
+}
+
+int fp64_stage(Context* c, int rkstep, double time, double dt) {
+  int st = scale_coef(c, dt);
+  if (st) return st;
+  Fp64Dev a = c->dargs;
+  a.u_in = c->d_u[c->cur];
+  a.u_out = c->d_u[c->cur ^ 1];
+  a.disp = c->fargs.disp;
+  a.inc_elem = c->fargs.inc_elem;
+  a.inc_val = c->fargs.inc_val;
+  a.gr = c->fargs.gr;
+  if (a.inc_elem && (st = incident_upload(c, time + dt * c->rk_c[rkstep - 1]))) return st;
+  if (a.gr.elem) {
+    a.gr.f_in = c->d_gr_f[c->gr_cur];
+    a.gr.f_out = c->d_gr_f[c->gr_cur ^ 1];
+  }
+  if ((st = fp64_launch(c, a, rkstep, time, dt, true))) return st;
+  if (a.gr.elem) c->gr_cur ^= 1;
+  c->cur ^= 1;
+  return NEKGPU_OK;
+}
+
+}  // namespace nekgpu

@@ -954,13 +954,14 @@ int upload_fused(Context* c, const Compact& cp) {
   c->host_w3 = cp.w3;
   c->host_rx.resize(c->nelt);
   for (int e = 0; e < c->nelt; ++e) c->host_rx[e] = cp.egeom[9 * (size_t)e];
-  // unscaled inverse-mass coefficients: hbm1|ebm1, or for the mixed form the
-  // normalised hbm1*w3*rx | ebm1*w3*rx (the residual is res/(bm1*2/hx))
+  // unscaled inverse-mass coefficients: hbm1|ebm1, or for the mixed and fused
+  // FP64 forms the normalised hbm1*w3*rx | ebm1*w3*rx (their residual is
+  // res/(w3*rx))
   {
     std::vector<double> base(2 * c->npts);
     for (long g = 0; g < c->npts; ++g) {
       double f = 1.0;
-      if (c->form == NEKGPU_MIXED) f = cp.w3[g % n3] * cp.egeom[9 * (g / n3)];
+      if (c->form != NEKGPU_MIXED_NAIVE) f = cp.w3[g % n3] * cp.egeom[9 * (g / n3)];
       base[g] = cp.hbm1[g] * f;
       base[c->npts + g] = cp.ebm1[g] * f;
     }
@@ -969,10 +970,18 @@ int upload_fused(Context* c, const Compact& cp) {
   c->uniform = cp.uniform;
   c->d_fcoef = nullptr;
   if (!cp.uniform) {
-    if (c->form == NEKGPU_FUSED64) {
+    if (c->form == NEKGPU_FUSED64) {  // times the lift factor of the slot
+      std::vector<double> f(cp.fcoef);
+      const size_t n2 = (size_t)c->nx * c->nx;
+      for (size_t j = 0; j < f.size() / 4; ++j) {
+        const double* g = &cp.egeom[9 * (j / (6 * n2))];
+        const double lf = g[3 + (j / n2) % 6] / (cp.w[0] * g[0]);
+        for (int q = 0; q < 4; ++q) f[4 * j + q] *= lf;
+      }
       double* d;
-      if ((st = A.put(&d, cp.fcoef))) return st;
+      if ((st = A.put(&d, f))) return st;
       c->d_fcoef = d;
+      c->host_fcoef64 = cp.fcoef;
     } else {
       std::vector<float> f(cp.fcoef.begin(), cp.fcoef.end());
       if (c->form == NEKGPU_MIXED) {
@@ -1053,6 +1062,43 @@ int upload_fused(Context* c, const Compact& cp) {
     return upload_pml_fused(c, A, cp, m.pml);
   }
   if ((st = A.put(&c->d_egeom, cp.egeom))) return st;
+  if (c->form == NEKGPU_FUSED64) {
+    // per element: sy/rx, tz/rx, and with the lift factor l = A_f/(w_end*rx)
+    // l/2 per slot, then l C0/2 (the flux coefficients of uniform media)
+    std::vector<double> egn(14 * (size_t)c->nelt);
+    for (int e = 0; e < c->nelt; ++e) {
+      const double* g = &cp.egeom[9 * (size_t)e];
+      double* o = &egn[14 * (size_t)e];
+      o[0] = g[1] / g[0];
+      o[1] = g[2] / g[0];
+      for (int f = 0; f < 6; ++f) {
+        o[2 + f] = 0.5 * (g[3 + f] / (cp.w[0] * g[0]));
+        o[8 + f] = o[2 + f] * cp.C0;
+      }
+    }
+    double* d_egn;
+    if ((st = A.put(&d_egn, egn))) return st;
+    Fp64Dev& d = c->dargs;
+    d = Fp64Dev{};
+    d.nelt = c->nelt;
+    d.npts = c->npts;
+    d.k = c->d_k;
+    d.k_out = c->d_k;
+    d.coef = c->d_coef;
+    d.nbr = c->d_nbr;
+    d.egn = d_egn;
+    d.fcoef = (const double*)c->d_fcoef;
+    for (int i = 0; i < c->nx * c->nx; ++i) d.D[i] = cp.D[i];
+    fixed_table(d.D, c->nx, d.fd);
+    FusedDev& f = c->fargs;  // what the adjoint and the set_* calls read
+    f = FusedDev{};
+    f.nelt = c->nelt;
+    f.npts = c->npts;
+    f.C0 = cp.C0;
+    for (int i = 0; i < c->nx * c->nx; ++i) f.D[i] = cp.D[i];
+    for (int i = 0; i < c->nx; ++i) f.w[i] = cp.w[i];
+    return upload_pml_fused(c, A, cp, d.pml);
+  }
   std::vector<float> gf(cp.egeom.begin(), cp.egeom.end());
   if ((st = A.put(&c->d_egeomf, gf))) return st;
   FusedDev& a = c->fargs;
@@ -1076,8 +1122,7 @@ int upload_fused(Context* c, const Compact& cp) {
     a.w[i] = cp.w[i];
     a.wf[i] = (float)cp.w[i];
   }
-  if (cp.pml.on() && c->form != NEKGPU_FUSED64) return NEKGPU_ERR_UNSUPPORTED;
-  return upload_pml_fused(c, A, cp, a.pml);
+  return cp.pml.on() ? NEKGPU_ERR_UNSUPPORTED : NEKGPU_OK;
 }
 
 // Curvilinear mesh for the fused FP64 and the mixed forms: the reference's
@@ -1486,6 +1531,7 @@ int do_stage(Context* c, int rkstep, double time, double dt) {
     return c->form == NEKGPU_MIXED ? mixed_curved_stage(c, rkstep, time, dt) : curved_stage(c, rkstep, time, dt);
   if (c->form == NEKGPU_PLAIN) return plain_stage(c, rkstep, time, dt);
   if (c->form == NEKGPU_MIXED) return mixed_stage(c, rkstep, time, dt);
+  if (c->form == NEKGPU_FUSED64) return fp64_stage(c, rkstep, time, dt);
   return fused_stage(c, rkstep, time, dt);
 }
 
@@ -1532,10 +1578,8 @@ int mixed_companion(Context* c, double dt, std::vector<void*>& owned, MixedDev& 
   split_D(D, n, tab);
   int st = mixed_upload_D(n, tab.data(), tab.size());
   if (st) return st;
-  std::vector<double> eg(9 * (size_t)nelt), hb(npts), eb(npts);
-  if (check_cuda(cudaMemcpy(eg.data(), c->d_egeom, eg.size() * 8, cudaMemcpyDeviceToHost)) ||
-      check_cuda(cudaMemcpy(hb.data(), c->d_hbm1, npts * 8, cudaMemcpyDeviceToHost)) ||
-      check_cuda(cudaMemcpy(eb.data(), c->d_ebm1, npts * 8, cudaMemcpyDeviceToHost)))
+  std::vector<double> eg(9 * (size_t)nelt);
+  if (check_cuda(cudaMemcpy(eg.data(), c->d_egeom, eg.size() * 8, cudaMemcpyDeviceToHost)))
     return NEKGPU_ERR_CUDA;
   m = MixedDev{};
   m.nelt = c->nelt;
@@ -1565,26 +1609,16 @@ int mixed_companion(Context* c, double dt, std::vector<void*>& owned, MixedDev& 
       return d ? NEKGPU_ERR_CUDA : NEKGPU_ERR_NOMEM;
     m.egm = d;
   }
-  // normalised inverse mass hbm1*w3*rx | ebm1*w3*rx, scaled by dt into pairs
+  // the context's normalised inverse mass hbm1*w3*rx | ebm1*w3*rx, scaled by dt into pairs
   {
-    std::vector<double> base(2 * (size_t)npts);
-    for (long g = 0; g < npts; ++g) {
-      const double f = c->host_w3[g % n3] * eg[9 * (g / n3)];
-      base[g] = hb[g] * f;
-      base[npts + g] = eb[g] * f;
-    }
-    double* db = (double*)dev(base.size() * 8);
-    float2* cf = (float2*)dev(base.size() * sizeof(float2));
-    if (!db || !cf) return NEKGPU_ERR_NOMEM;
-    if (check_cuda(cudaMemcpy(db, base.data(), base.size() * 8, cudaMemcpyHostToDevice))) return NEKGPU_ERR_CUDA;
-    if ((st = mixed_scale_pairs(c, cf, db, 2 * npts, dt))) return st;
+    float2* cf = (float2*)dev(2 * (size_t)npts * sizeof(float2));
+    if (!cf) return NEKGPU_ERR_NOMEM;
+    if ((st = mixed_scale_pairs(c, cf, c->d_cbase, 2 * npts, dt))) return st;
     m.coef = cf;
   }
   // face coefficients as pairs (hi float4, lo float4 per face node)
   if (c->d_fcoef) {
-    std::vector<double> fc(4 * (size_t)nxzfl);
-    if (check_cuda(cudaMemcpy(fc.data(), c->d_fcoef, fc.size() * 8, cudaMemcpyDeviceToHost)))
-      return NEKGPU_ERR_CUDA;
+    const std::vector<double>& fc = c->host_fcoef64;
     std::vector<float> f(8 * (size_t)nxzfl);
     for (long j = 0; j < nxzfl; ++j)
       for (int q = 0; q < 4; ++q) {
@@ -1597,7 +1631,7 @@ int mixed_companion(Context* c, double dt, std::vector<void*>& owned, MixedDev& 
       return d ? NEKGPU_ERR_CUDA : NEKGPU_ERR_NOMEM;
     m.fcoef = d;
   }
-  // volume source: the FP64 weights normalised by w3*rx, as pairs
+  // volume source: the context's normalised FP64 weights, as pairs
   if (c->src.enabled && c->fargs.src_elem) {
     std::vector<int> off(nelt);
     if (check_cuda(cudaMemcpy(off.data(), c->fargs.src_elem, nelt * sizeof(int), cudaMemcpyDeviceToHost)))
@@ -1608,14 +1642,9 @@ int mixed_companion(Context* c, double dt, std::vector<void*>& owned, MixedDev& 
     if (cnt && check_cuda(cudaMemcpy(wd.data(), c->fargs.src_w, wd.size() * 8, cudaMemcpyDeviceToHost)))
       return NEKGPU_ERR_CUDA;
     std::vector<float> wf(2 * wd.size());
-    for (long e = 0; e < nelt; ++e) {
-      if (off[e] < 0) continue;
-      for (long v = 0; v < n3; ++v) {
-        const size_t i = (size_t)off[e] * n3 + v;
-        const double x = wd[i] / (c->host_w3[v] * eg[9 * (size_t)e]);
-        wf[2 * i] = (float)x;
-        wf[2 * i + 1] = (float)(x - (double)wf[2 * i]);
-      }
+    for (size_t i = 0; i < wd.size(); ++i) {
+      wf[2 * i] = (float)wd[i];
+      wf[2 * i + 1] = (float)(wd[i] - (double)wf[2 * i]);
     }
     float* d = (float*)dev(std::max<size_t>(wf.size(), 2) * sizeof(float));
     if (!d) return NEKGPU_ERR_NOMEM;
@@ -2454,20 +2483,18 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
     }
     int* d_off;
     if ((st = A.put(&d_off, off))) return st;
+    if (c->form != NEKGPU_MIXED_NAIVE && !c->curved) {
+      // normalised like the residual: weight / (w3 * rx)
+      for (int e = 0; e < c->nelt; ++e)
+        if (off[e] >= 0)
+          for (long v = 0; v < n3; ++v) wd[off[e] * n3 + v] /= c->host_w3[v] * c->host_rx[e];
+    }
     if (c->form == NEKGPU_MIXED && !c->curved) {
-      // normalised like the residual: weight / (bm1 * 2/hx) = weight / (w3 * rx),
-      // as a (hi, lo) float pair (~2^-48 of the weight)
+      // as (hi, lo) float pairs (~2^-48 of the weight)
       std::vector<float> wf(2 * wd.size());
-      for (int e = 0, s0 = 0; e < c->nelt; ++e) {
-        if (off[e] < 0) continue;
-        for (long v = 0; v < n3; ++v) {
-          const size_t i = (size_t)s0 * n3 + v;
-          const double w = wd[i] / (c->host_w3[v] * c->host_rx[e]);
-          const float hi = (float)w;
-          wf[2 * i] = hi;
-          wf[2 * i + 1] = (float)(w - (double)hi);
-        }
-        ++s0;
+      for (size_t i = 0; i < wd.size(); ++i) {
+        wf[2 * i] = (float)wd[i];
+        wf[2 * i + 1] = (float)(wd[i] - (double)wf[2 * i]);
       }
       float* d;
       if ((st = A.put(&d, wf))) return st;

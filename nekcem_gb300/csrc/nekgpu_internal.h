@@ -208,6 +208,42 @@ __device__ inline void graphene_slot(const GrapheneDev& G, long g, const double 
 }
 #endif
 
+// D in fixed point for the integer contractions of the FP64 kernels
+// (nekgpu_fixed.cuh): entry i + nx*l holds D(i,l) 2^kd = hi 2^31 + lo, hi8 =
+// 8 hi; bias = 1022 + kd.  ok = 0: D does not fit, contract in FP64.
+constexpr int kMaxFixed = 9;
+struct FixedD {
+  int ok, bias;
+  int hi[kMaxFixed * kMaxFixed], lo[kMaxFixed * kMaxFixed], hi8[kMaxFixed * kMaxFixed];
+};
+
+// Fused FP64 stage (nekgpu_fp64.cu): arguments as in FusedDev, with the
+// residual normalised as in the mixed form (res / (w3 rx)).
+struct Fp64Dev {
+  int nelt;
+  long npts;
+  const double* u_in;
+  double* u_out;
+  const double* k;      // RK register read
+  double* k_out;        // RK register written (== k unless stage data is being kept)
+  const double* coef;   // 2*npts: dt*hbm1*w3*rx then dt*ebm1*w3*rx
+  const int* nbr;       // 6*nelt
+  const double* egn;    // 14*nelt: sy/rx, tz/rx, and with the lift factor l = area/(w_end*rx)
+                        // of the slot l/2 per slot and l C0/2 per slot
+  const double* fcoef;  // 4 per face node, l times (Y02, C02Y, Z02, C02Z); null when uniform
+  const int* src_elem;  // nelt: offset (in elements) into src_w or -1; null if no source
+  const double* src_w;  // source weights / (w3*rx), nx^3 per source element
+  double src_ft;
+  double a, b, dt;
+  PmlDev pml;
+  DispDev disp;
+  const int* inc_elem;
+  const double* inc_val;
+  GrapheneDev gr;
+  FixedD fd;
+  double D[kMaxFixed * kMaxFixed];  // D(i,j) at [i + nx*j]
+};
+
 struct FusedDev {
   int nelt;
   long npts;
@@ -280,13 +316,14 @@ struct AdjointDev {
   const double* u_prev;  // forward u_{i-1}
   const double* k_cur;   // forward k_i
   const double* k_prev;  // forward k_{i-1} (unused when a == 0)
-  const double* coef;    // dt hbm1 (npts), dt ebm1 (npts)
+  const double* hbm1;
+  const double* ebm1;
   const double* bm1;
   double* deps;          // accumulated dJ/deps per node
   const int* nbr;
   const double* egeom;
   const double* slot;    // [16][nxzfl] static face-slot coefficients as (hi, lo) float pairs
-  double a, b_next, inv_dt;
+  double a, bdt_next, inv_dt;  // bdt_next = b_{i-1} dt
   double Dw[kMaxNx * kMaxNx];  // D(m,i) w_m at [m + NX*i]
   double w[kMaxNx];
 };
@@ -409,6 +446,7 @@ struct Context {
   bool uniform = true;
   int fused_grid = 0;
   FusedDev fargs{};
+  Fp64Dev dargs{};  // fused FP64 form, affine meshes
   MixedDev margs{};
   float* d_egm = nullptr;
   // PML: plain form uses d_pml_sigma/d_eps/d_mu/d_pmlptr/d_pml_res (full
@@ -453,8 +491,8 @@ struct Context {
   int adj_stride = 0;
   int adj_host_snapshots = 0;  // pinned host snapshot slots the binomial schedule may add
   bool adj_mixed_recompute = false;  // fused FP64: the sqrt schedule's segments recomputed in mixed stages
-  // mixed form: the FP64 face coefficients (4 per face node, as FusedDev::fcoef)
-  // for the adjoint's face-slot table; empty when uniform
+  // the FP64 face coefficients (4 per face node: Y02, C02Y, Z02, C02Z) for the
+  // adjoint's face-slot table; empty when uniform
   std::vector<double> host_fcoef64;
 
   // plain form
@@ -498,13 +536,19 @@ int plain_incident(Context* c);
 int incident_upload(Context* c, double rktime);
 int plain_gs(Context* c, double* d_u, int nfld);
 
-// kernel launchers (nekgpu_fused.cu)
+// kernel launchers (nekgpu_fused.cu, the FP32 form kept for comparison)
 int fused_setup(Context* c);  // grid size / smem attributes
 int fused_stage(Context* c, int rkstep, double time, double dt);
-// one stage with explicit state / RK-register buffers (no ping-pong bookkeeping)
-int fused_stage_buffers(Context* c, int rkstep, double time, double dt, const double* u_in,
-                        double* u_out, double* k_in, double* k_out);
 int scale_coef(Context* c, double dt);
+
+// nekgpu_fp64.cu: the fused FP64 stage on affine meshes
+int fp64_stage(Context* c, int rkstep, double time, double dt);
+// one stage with explicit state / RK-register buffers (no ping-pong bookkeeping)
+int fp64_stage_buffers(Context* c, int rkstep, double time, double dt, const double* u_in,
+                       double* u_out, const double* k_in, double* k_out);
+void fixed_table(const double* D, int n, FixedD& t);
+
+int num_sms(Context* c);
 
 // nekgpu_mixed.cu
 int mixed_stage(Context* c, int rkstep, double time, double dt);
@@ -548,11 +592,9 @@ int stage2d(Context* c, int rkstep, double time, double dt);
 
 // nekgpu_adjoint.cu
 int adjoint_stage(Context* c, const AdjointDev& a);
-// w = b * coef * ub (the stage weights of the last stage of the last step)
-int adjoint_seed(Context* c, double* w, const double* ub, const double* coef, double b);
-// coef = dt hbm1 | dt ebm1 (2 npts), the FP64 inverse-mass scale of the
-// reverse stages, for a context whose own coefficients are float pairs
-int adjoint_coef64(Context* c, double* coef, double dt);
+// w = bdt * (hbm1 | ebm1) * ub (the stage weights of the last stage of the
+// last step; bdt = b_5 dt)
+int adjoint_seed(Context* c, double* w, const double* ub, double bdt);
 
 // nekgpu_noalloc.cu: cem_error norms with a fixed device scratch array
 int norms_noalloc(Context* c, const double* exact_dev, double l2[6], double linf[6]);
