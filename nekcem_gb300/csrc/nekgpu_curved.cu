@@ -10,13 +10,27 @@
 // launched before the stage kernel, which then adds flux, lift, source,
 // inverse mass and RK update in one pass.
 //
-// One block of N3 threads per element at a time (thread per node); the
-// element's six field components sit in shared memory for the derivative
-// contractions, which take D from shared memory.  The metrics add 72 bytes
-// per node and stage to the affine kernel's traffic; the face geometry
-// 4 doubles and the partner index per face node.
+// What bounds it: the FP64 pipe (two lanes per clock and SM).  The 18
+// contractions per node run in 64-bit integer arithmetic (nekgpu_fixed.cuh),
+// one thread per GLL line; the node's weight w3 multiplies the curl once, as
+// the lift is added, and the areas are inside the face coefficients.  That leaves ~90 FP64 operations per node at
+// N=7 (curl 36, flux 32, finish 18) of the ~230 of a form with FP64
+// contractions: 57 us per stage for 990 elements at N=5 (135 before; FP64 pipe
+// 73 % busy), 117 for 1000 at N=7.
+//
+// One block per element at a time, thread per node: state in shared memory;
+// face nodes' fluxes summed per node, axis by axis so that no two threads
+// meet at one; then for each direction the six derivatives to
+// shared memory and, per node, their products with the direction's three
+// metrics into the residual held in registers.  The metrics add 72 bytes per
+// node and stage to the affine kernel's traffic; the face geometry 4 doubles
+// and the partner index per face node.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
+#include "nekgpu_fixed.cuh"
 #include "nekgpu_internal.h"
 
 namespace nekgpu {
@@ -24,172 +38,252 @@ namespace nekgpu {
 namespace {
 
 template <int NX>
-__device__ __forceinline__ int face_vol_c(int f, int a, int b) {
+__device__ __forceinline__ void face_node(int f, int a, int b, int& i, int& j, int& k) {
   // slot order s=-1, r=+1, s=+1, r=-1, t=-1, t=+1 (pff)
-  switch (f) {
-    case 0: return a + NX * NX * b;
-    case 1: return NX - 1 + NX * a + NX * NX * b;
-    case 2: return a + NX * (NX - 1) + NX * NX * b;
-    case 3: return NX * a + NX * NX * b;
-    case 4: return a + NX * b;
-    default: return a + NX * b + NX * NX * (NX - 1);
+  const int ax = f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2);
+  const int fix = f == 0 || f == 3 || f == 4 ? 0 : NX - 1;
+  i = ax == 0 ? fix : a;
+  j = ax == 1 ? fix : (ax == 0 ? a : b);
+  k = ax == 2 ? fix : b;
+}
+
+constexpr int round32(int a) { return (a + 31) / 32 * 32; }
+
+template <int NX>
+struct KCfg {
+  static constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
+  static constexpr int RS = NX | 1, SZ = RS * NX, N3P = NX * SZ;  // odd rows
+  static constexpr int NT = round32(N3 > 6 * N2 ? N3 : 6 * N2);  // a thread per node, line and face node
+  static constexpr int kMinBlocks = NT > 256 ? 2 : (NT > 160 ? 3 : 4);
+  static constexpr size_t smem = 4 * 6 * (size_t)N3P * 8;  // state, derivatives A and B, lifted flux
+};
+
+// the six derivatives along DIR to s_d: one thread per (component, line)
+template <int NX, int DIR>
+__device__ __forceinline__ void curved_lines(const double* s_u, double* s_d, const CurvedDev& a) {
+  using C = KCfg<NX>;
+  const int task = threadIdx.x;
+  if (task >= 6 * C::N2) return;
+  const int c = task / C::N2, lam = task - c * C::N2, la = lam % NX, lb = lam / NX;
+  const int base = c * C::N3P + (DIR == 0 ? C::RS * la + C::SZ * lb
+                                          : (DIR == 1 ? la + C::SZ * lb : la + C::RS * lb));
+  constexpr int step = DIR == 0 ? 1 : (DIR == 1 ? C::RS : C::SZ);
+  FixedLine<NX> f;
+  {
+    double u[NX];
+#pragma unroll
+    for (int l = 0; l < NX; ++l) u[l] = s_u[base + step * l];
+    fixed_line<NX>(u, f);
+  }
+  if (a.fd.ok && !f.special) {
+#pragma unroll
+    for (int i = 0; i < NX; ++i)
+      s_d[base + step * i] = fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
+        hi = a.fd.hi[i + NX * l];
+        lo = a.fd.lo[i + NX * l];
+        hi8 = a.fd.hi8[i + NX * l];
+      });
+  } else {  // a line out of the integer form's range: in FP64
+#pragma unroll 1
+    for (int i = 0; i < NX; ++i) {
+      double x = a.D[i] * s_u[base];
+#pragma unroll 1
+      for (int l = 1; l < NX; ++l) x = fma(a.D[i + NX * l], s_u[base + step * l], x);
+      s_d[base + step * i] = x;
+    }
   }
 }
 
 template <int NX>
-__global__ void __launch_bounds__((NX * NX * NX + 31) / 32 * 32)
-    k_curved_stage(const CurvedDev a) {
-  constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
-  constexpr int NT = (N3 + 31) / 32 * 32;
-  __shared__ double s_u[6 * N3];
-  __shared__ double s_D[N2];
-  __shared__ double s_w3[N3];
-  __shared__ double s_flux[6 * NF];
+__global__ void __launch_bounds__(KCfg<NX>::NT, KCfg<NX>::kMinBlocks)
+    k_curved_stage(const __grid_constant__ CurvedDev a) {
+  using C = KCfg<NX>;
+  constexpr int N2 = C::N2, N3 = C::N3, NF = C::NF, N3P = C::N3P;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* s_u = reinterpret_cast<double*>(smem);
+  double* s_A = s_u + 6 * N3P;
+  double* s_B = s_A + 6 * N3P;
+  double* s_L = s_B + 6 * N3P;
   const int tid = threadIdx.x;
   const long P = a.npts;
   const bool node = tid < N3;
   const int vi = tid % NX, vj = (tid / NX) % NX, vk = tid / N2;
+  const int pn = vi + C::RS * vj + C::SZ * vk;  // stored node
+  const bool on_face = node && (vi == 0 || vi == NX - 1 || vj == 0 || vj == NX - 1 || vk == 0 || vk == NX - 1);
   const bool first_stage = (a.a == 0.0);
-  for (int t = tid; t < N2; t += NT) s_D[t] = a.D[t];
-  for (int t = tid; t < N3; t += NT) s_w3[t] = a.w3[t];
 
+  // a programmatic dependent of the previous launch: nothing it wrote is read
+  // before it has completed; the next one may launch from the last element on
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   for (int e = blockIdx.x; e < a.nelt; e += gridDim.x) {
-    __syncthreads();  // the previous element's shared data is consumed
+    if (e + (int)gridDim.x >= a.nelt) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const long g = (long)e * N3 + tid;
     if (node) {
-      const long g = (long)e * N3 + tid;
-#pragma unroll
-      for (int c = 0; c < 6; ++c) s_u[c * N3 + tid] = a.u_in[c * P + g];
-    }
-    __syncthreads();
-
-    // ---- weighted curl with the general metrics ---------------------------
-    // (or, with the dealiased curl, its volume term computed before)
-    double res[6];
-    if (node && a.vres) {
-      const long g = (long)e * N3 + tid;
-#pragma unroll
-      for (int c = 0; c < 6; ++c) res[c] = a.vres[c * P + g];
-    } else if (node) {
-      double dr[6], ds[6], dt[6];
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const double* u = s_u + c * N3;
-        double sr = s_D[vi] * u[NX * vj + N2 * vk];
-        double ss = s_D[vj] * u[vi + N2 * vk];
-        double st = s_D[vk] * u[vi + NX * vj];
-#pragma unroll
-        for (int l = 1; l < NX; ++l) {
-          sr = fma(s_D[vi + NX * l], u[l + NX * vj + N2 * vk], sr);
-          ss = fma(s_D[vj + NX * l], u[vi + NX * l + N2 * vk], ss);
-          st = fma(s_D[vk + NX * l], u[vi + NX * vj + N2 * l], st);
-        }
-        const double w = s_w3[tid];
-        dr[c] = sr * w;
-        ds[c] = ss * w;
-        dt[c] = st * w;
-      }
-      const long g = (long)e * N3 + tid;
-      const double rx = a.metrics[g], ry = a.metrics[P + g], rz = a.metrics[2 * P + g];
-      const double sx = a.metrics[3 * P + g], sy = a.metrics[4 * P + g], sz = a.metrics[5 * P + g];
-      const double tx = a.metrics[6 * P + g], ty = a.metrics[7 * P + g], tz = a.metrics[8 * P + g];
-      // w = curl(u1, u2, u3) with d/dx = rx d/dr + sx d/ds + tx d/dt, etc.
-      auto curl = [&](int c1, int c2, int c3, double* w) {
-        w[0] = (dr[c3] * ry + ds[c3] * sy + dt[c3] * ty) - (dr[c2] * rz + ds[c2] * sz + dt[c2] * tz);
-        w[1] = (dr[c1] * rz + ds[c1] * sz + dt[c1] * tz) - (dr[c3] * rx + ds[c3] * sx + dt[c3] * tx);
-        w[2] = (dr[c2] * rx + ds[c2] * sx + dt[c2] * tx) - (dr[c1] * ry + ds[c1] * sy + dt[c1] * ty);
-      };
-      double wE[3], wH[3];
-      curl(0, 1, 2, wE);  // resE = W curl H
-      curl(3, 4, 5, wH);  // resH = -W curl E
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        res[c] = -wH[c];
-        res[3 + c] = wE[c];
+        s_u[c * N3P + pn] = a.u_in[c * P + g];
       }
     }
-
-    // ---- upwind flux per face node ----------------------------------------
-    for (int t = tid; t < NF; t += NT) {
-      const int f = t / N2, ab = t - f * N2;
-      const int v = face_vol_c<NX>(f, ab % NX, ab / NX);
-      const long js = (long)e * NF + t, L = a.nxzfl;
+    // ---- upwind flux of the thread's face node, lifted -------------------------
+    double F[6];
+    int fax = -1, fv = 0;
+    bool later = false;  // the node lies on a face of an axis before this one
+    __syncthreads();
+    if (tid < NF) {
+      const int f = tid / N2, ab = tid - f * N2;
+      int i, j, k;
+      face_node<NX>(f, ab % NX, ab / NX, i, j, k);
+      fv = i + C::RS * j + C::SZ * k;
+      fax = f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2);
+      later = (fax > 0 && (i == 0 || i == NX - 1)) || (fax > 1 && (j == 0 || j == NX - 1));
+      const long js = (long)e * NF + tid, L = a.nxzfl;
       const int pv = a.partner[js];
+      const double nx = a.face[js], ny = a.face[L + js], nz = a.face[2 * L + js];
       double dH[3], dE[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const double hm = s_u[c * N3 + v], em = s_u[(c + 3) * N3 + v];
+        const double em = s_u[(c + 3) * N3P + fv];
         if (pv >= 0) {
-          dH[c] = a.u_in[c * P + pv] - hm;
+          dH[c] = a.u_in[c * P + pv] - s_u[c * N3P + fv];
           dE[c] = a.u_in[(c + 3) * P + pv] - em;
         } else {  // PEC mirror: H+ = H-, E+ = -E-
           dH[c] = 0.0;
           dE[c] = -2.0 * em;
         }
       }
-      const double nx = a.face[js], ny = a.face[L + js], nz = a.face[2 * L + js];
-      const double area = a.face[3 * L + js];
-      double Y02 = -0.5, C02Y = 0.5, Z02 = 0.5, C02Z = 0.5;
-      if (a.fcoef) {
-        Y02 = a.fcoef[js]; C02Y = a.fcoef[L + js]; Z02 = a.fcoef[2 * L + js]; C02Z = a.fcoef[3 * L + js];
-      }
-      // n x [E], n x [H] (the gs sums of -n x E, -n x H), then the upwind terms
-      const double nE[3] = {ny * dE[2] - nz * dE[1], nz * dE[0] - nx * dE[2], nx * dE[1] - ny * dE[0]};
-      const double nH[3] = {ny * dH[2] - nz * dH[1], nz * dH[0] - nx * dH[2], nx * dH[1] - ny * dH[0]};
-      const double fu[3] = {ny * nH[2] - nz * nH[1], nz * nH[0] - nx * nH[2], nx * nH[1] - ny * nH[0]};
-      const double fw[3] = {ny * nE[2] - nz * nE[1], nz * nE[0] - nx * nE[2], nx * nE[1] - ny * nE[0]};
+      // n x [E], n x [H] (the gs sums of -n x E, -n x H) and the upwind terms
+      // n x (n x [u]); the area is in the coefficients
+      const double n[3] = {nx, ny, nz};
+      double xE[3], xH[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        s_flux[c * NF + t] = area * (Y02 * nE[c] - C02Y * fu[c]);
-        s_flux[(3 + c) * NF + t] = area * (Z02 * nH[c] - C02Z * fw[c]);
+        const int p = (c + 1) % 3, q = (c + 2) % 3;
+        xE[c] = fma(n[p], dE[q], -(n[q] * dE[p]));
+        xH[c] = fma(n[p], dH[q], -(n[q] * dH[p]));
+      }
+      if (a.fcoef) {
+        const double Y02 = a.fcoef[js], C02Y = a.fcoef[L + js], Z02 = a.fcoef[2 * L + js],
+                     C02Z = a.fcoef[3 * L + js];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int p = (c + 1) % 3, q = (c + 2) % 3;
+          F[c] = fma(Y02, xE[c], -(C02Y * fma(n[p], xH[q], -(n[q] * xH[p]))));
+          F[3 + c] = fma(Z02, xH[c], -(C02Z * fma(n[p], xE[q], -(n[q] * xE[p]))));
+        }
+      } else {  // Y02 = -1/2, C02Y = Z02 = C02Z = 1/2 times the area
+        const double h = a.face[3 * L + js];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int p = (c + 1) % 3, q = (c + 2) % 3;
+          F[c] = -h * fma(n[p], xH[q], fma(-n[q], xH[p], xE[c]));
+          F[3 + c] = h * fma(-n[p], xE[q], fma(n[q], xE[p], xH[c]));
+        }
       }
     }
-    __syncthreads();
-
-    if (node) {
-      // ---- lift in face-slot order ---------------------------------------
-      auto add = [&](int f, int ab) {
+    // ---- lift, and the weighted curl resE += W curl H, resH -= W curl E ---------
+    // d/dx_ax = sum over directions of metric(dir, ax) d/d_dir.  The lines of
+    // one direction run beside the lift of one axis (its two faces share no
+    // node) and the products of the direction before:
+    //   lines r -> A, lift r | lines s -> B, lift s, A | lines t -> A, lift t, B | A
+    double res[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    auto lift = [&](int ax) {
+      if (fax == ax)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) res[c] += s_flux[c * NF + f * N2 + ab];
-      };
-      if (vj == 0) add(0, vi + NX * vk);
-      if (vi == NX - 1) add(1, vj + NX * vk);
-      if (vj == NX - 1) add(2, vi + NX * vk);
-      if (vi == 0) add(3, vj + NX * vk);
-      if (vk == 0) add(4, vi + NX * vj);
-      if (vk == NX - 1) add(5, vi + NX * vj);
-      // ---- volume source (usersrc), mass-weighted ------------------------
+        for (int c = 0; c < 6; ++c) {
+          double* q = s_L + c * N3P + fv;
+          *q = ax > 0 && later ? *q + F[c] : F[c];
+        }
+    };
+    auto products = [&](int dir, const double* s_d) {
+      if (!node) return;
+      double m[3];
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) m[ax] = a.metrics[(3 * dir + ax) * P + g];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {  // a component enters the curl's two others
+        const int p1 = (q + 1) % 3, p2 = (q + 2) % 3;
+        const double h = s_d[q * N3P + pn], v = s_d[(3 + q) * N3P + pn];
+        res[3 + p2] = fma(-m[p1], h, res[3 + p2]);
+        res[3 + p1] = fma(m[p2], h, res[3 + p1]);
+        res[p2] = fma(m[p1], v, res[p2]);
+        res[p1] = fma(-m[p2], v, res[p1]);
+      }
+    };
+    const bool curl = a.vres == nullptr;  // else the dealiased volume term, computed before
+    lift(0);
+    if (curl) curved_lines<NX, 0>(s_u, s_A, a);
+    __syncthreads();
+    lift(1);
+    if (curl) {
+      curved_lines<NX, 1>(s_u, s_B, a);
+      products(0, s_A);
+    }
+    __syncthreads();
+    lift(2);
+    if (curl) {
+      curved_lines<NX, 2>(s_u, s_A, a);
+      products(1, s_B);
+    }
+    __syncthreads();
+    if (curl) {
+      products(2, s_A);
+      const double w3 = node ? a.w3[tid] : 0.0;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) res[c] = fma(w3, res[c], on_face ? s_L[c * N3P + pn] : 0.0);
+    } else if (node) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) res[c] = a.vres[c * P + g] + (on_face ? s_L[c * N3P + pn] : 0.0);
+    }
+    if (node) {
+      // ---- volume source (usersrc) ---------------------------------------
       if (a.src_elem) {
         const int so = a.src_elem[e];
-        if (so >= 0) res[5] += a.src_w[(long)so * N3 + tid] * a.src_ft;
+        if (so >= 0) res[5] = fma(a.src_w[(long)so * N3 + tid], a.src_ft, res[5]);
       }
       // ---- inverse mass + low-storage RK ---------------------------------
-      const long g = (long)e * N3 + tid;
       const double ch = a.coef[g], ce = a.coef[P + g];
+      double kk[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) kk[c] = first_stage ? 0.0 : a.k[c * P + g];
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
         const double r = res[c] * (c < 3 ? ch : ce);
-        const double kn = first_stage ? r : fma(a.a, a.k[c * P + g], r);
+        const double kn = first_stage ? r : fma(a.a, kk[c], r);
         a.k[c * P + g] = kn;
-        a.u_out[c * P + g] = fma(a.b, kn, s_u[c * N3 + tid]);
+        a.u_out[c * P + g] = fma(a.b, kn, s_u[c * N3P + pn]);
       }
     }
+    // (the next element's state overwrites s_u: only this thread's node of it
+    // is still read above)
   }
 }
 
 template <int NX>
 int launch_curved(Context* c, const CurvedDev& a) {
-  constexpr int NT = (NX * NX * NX + 31) / 32 * 32;
+  using C = KCfg<NX>;
   static int grid = 0;
   if (!grid) {
-    int per_sm = 0, sms = 0;
-    if (check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_curved_stage<NX>, NT, 0)))
+    if (check_cuda(cudaFuncSetAttribute(k_curved_stage<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)C::smem)))
       return NEKGPU_ERR_CUDA;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    int per_sm = 0;
+    if (check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_curved_stage<NX>, C::NT,
+                                                                 C::smem)))
+      return NEKGPU_ERR_CUDA;
     if (per_sm < 1) return NEKGPU_ERR_UNSUPPORTED;
-    grid = per_sm * sms;
+    grid = per_sm * num_sms(c);
   }
-  const int g = c->nelt < grid ? c->nelt : grid;
-  k_curved_stage<NX><<<g, NT, 0, c->stream>>>(a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(c->nelt, grid));
+  cfg.blockDim = dim3(C::NT);
+  cfg.dynamicSmemBytes = C::smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (check_cuda(cudaLaunchKernelEx(&cfg, k_curved_stage<NX>, a))) return NEKGPU_ERR_CUDA;
   c->last_launches += 1;
   return check_cuda(cudaGetLastError());
 }

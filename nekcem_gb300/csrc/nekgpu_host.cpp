@@ -352,15 +352,16 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
     if (std::fabs(t - m->w3mn[v]) > 1e-12 * std::fabs(t)) return NEKGPU_ERR_MESH;
   }
   cp.egeom.assign(9 * (size_t)nelt, 0.0);
+  cp.lift.assign(6 * (size_t)nelt, 0.0);
   const double* mt[9] = {m->rxmn, m->rymn, m->rzmn, m->sxmn, m->symn, m->szmn, m->txmn, m->tymn, m->tzmn};
   for (int e = 0; e < nelt; ++e) {
     const long o = n3 * e;
     double diag[3] = {0, 0, 0};
     const int di[3] = {0, 4, 8};
     for (int d = 0; d < 3; ++d) {
-      double s = 0;
-      for (long v = 0; v < n3; ++v) s += mt[di[d]][o + v];
-      diag[d] = s / n3;
+      double s = 0;  // the mean as the first value plus the mean deviation: exact for equal values
+      for (long v = 0; v < n3; ++v) s += mt[di[d]][o + v] - mt[di[d]][o];
+      diag[d] = mt[di[d]][o] + s / n3;
       if (!(diag[d] > 0)) return NEKGPU_ERR_MESH;
     }
     const double scale = std::max(diag[0], std::max(diag[1], diag[2]));
@@ -375,7 +376,7 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
     cp.egeom[9 * e + 2] = diag[2];
     for (int f = 0; f < 6; ++f) {
       const int ax = kSlotAxis[f], sd = kSlotSide[f];
-      double s = 0;
+      double s = 0, sl = 0, l0 = 0;
       for (int b = 0; b < n; ++b)
         for (int a = 0; a < n; ++a) {
           const long j = a + (long)n * b + n2 * (f + 6L * e);
@@ -386,8 +387,12 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
             if (std::fabs(nv[d] - want) > tol) return NEKGPU_ERR_MESH;
           }
           s += m->aream[j] / (cp.w[a] * cp.w[b]);
+          const double l = m->aream[j] / m->w3mn[face_vol(f, a, b, n)];
+          if (a == 0 && b == 0) l0 = l;
+          sl += l - l0;
         }
       s /= n2;
+      cp.lift[6 * e + f] = l0 + sl / n2;
       for (int b = 0; b < n; ++b)
         for (int a = 0; a < n; ++a) {
           const long j = a + (long)n * b + n2 * (f + 6L * e);
@@ -730,6 +735,7 @@ void compact_from_box(const nekgpu_box* bx, const BoxArrays& A, Compact& cp) {
   const double ascale[3] = {ys * zt, xr * zt, xr * ys};
   cp.egeom.resize(9 * (size_t)nelt);
   cp.nbr.resize(6 * (size_t)nelt);
+  cp.lift.resize(6 * (size_t)nelt);
   for (long e = 0; e < nelt; ++e) {
     const long ec[3] = {e % nel[0], (e / nel[0]) % nel[1], e / ((long)nel[0] * nel[1])};
     cp.egeom[9 * e + 0] = ys * zt;
@@ -737,6 +743,7 @@ void compact_from_box(const nekgpu_box* bx, const BoxArrays& A, Compact& cp) {
     cp.egeom[9 * e + 2] = xr * ys;
     for (int f = 0; f < 6; ++f) {
       cp.egeom[9 * e + 3 + f] = ascale[kSlotAxis[f]];
+      cp.lift[6 * e + f] = ascale[kSlotAxis[f]] / w[0];
       cp.nbr[6 * e + f] = (int)box_partner(bx, nel, ec, f);
     }
   }
@@ -974,8 +981,7 @@ int upload_fused(Context* c, const Compact& cp) {
       std::vector<double> f(cp.fcoef);
       const size_t n2 = (size_t)c->nx * c->nx;
       for (size_t j = 0; j < f.size() / 4; ++j) {
-        const double* g = &cp.egeom[9 * (j / (6 * n2))];
-        const double lf = g[3 + (j / n2) % 6] / (cp.w[0] * g[0]);
+        const double lf = cp.lift[j / n2] / cp.egeom[9 * (j / (6 * n2))];
         for (int q = 0; q < 4; ++q) f[4 * j + q] *= lf;
       }
       double* d;
@@ -1063,7 +1069,7 @@ int upload_fused(Context* c, const Compact& cp) {
   }
   if ((st = A.put(&c->d_egeom, cp.egeom))) return st;
   if (c->form == NEKGPU_FUSED64) {
-    // per element: sy/rx, tz/rx, and with the lift factor l = A_f/(w_end*rx)
+    // per element: sy/rx, tz/rx, and with the lift factor l = area/(w3*rx)
     // l/2 per slot, then l C0/2 (the flux coefficients of uniform media)
     std::vector<double> egn(14 * (size_t)c->nelt);
     for (int e = 0; e < c->nelt; ++e) {
@@ -1072,7 +1078,7 @@ int upload_fused(Context* c, const Compact& cp) {
       o[0] = g[1] / g[0];
       o[1] = g[2] / g[0];
       for (int f = 0; f < 6; ++f) {
-        o[2 + f] = 0.5 * (g[3 + f] / (cp.w[0] * g[0]));
+        o[2 + f] = 0.5 * (cp.lift[6 * (size_t)e + f] / g[0]);
         o[8 + f] = o[2 + f] * cp.C0;
       }
     }
@@ -1178,9 +1184,12 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   if ((st = upload_common(c, A, bm1, eb, hb))) return st;
   if ((st = A.get(&c->d_coef, 2 * npts))) return st;
   std::vector<double> base(2 * npts);
+  // the mixed form's residual is res/w3
+  const bool norm = c->form == NEKGPU_MIXED;
   for (long g = 0; g < npts; ++g) {
-    base[g] = hb[g];
-    base[npts + g] = eb[g];
+    const double w = norm ? m->w3mn[g % n3] : 1.0;
+    base[g] = hb[g] * w;
+    base[npts + g] = eb[g] * w;
   }
   if ((st = A.put(&c->d_cbase, base))) return st;
   c->coef_dt = std::nan("");
@@ -1192,16 +1201,22 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
     face[j] = m->unxm[j];
     face[nxzfl + j] = m->unym[j];
     face[2 * nxzfl + j] = m->unzm[j];
-    face[3 * nxzfl + j] = m->aream[j];
+    const double area = norm ? m->aream[j] / m->w3mn[(m->cemface[j] - 1) % n3] : m->aream[j];
+    face[3 * nxzfl + j] = 0.5 * area;
     const double Y0 = m->Y_0[j], Y1 = m->Y_1[j], Z0 = m->Z_0[j], Z1 = m->Z_1[j];
     const double o[4] = {-0.5 / Y0 * Y1, 0.5 / Y0 * m->C0, 0.5 / Z0 * Z1, 0.5 / Z0 * m->C0};
-    for (int q = 0; q < 4; ++q) fcoef[q * nxzfl + j] = o[q];
+    for (int q = 0; q < 4; ++q) fcoef[q * nxzfl + j] = area * o[q];
     uniform = uniform && o[0] == -0.5 && o[1] == 0.5 && o[2] == 0.5 && o[3] == 0.5;
   }
   CurvedDev& a = c->cargs;
   a = CurvedDev{};
   double* d;
   int* di;
+  if (norm)  // as (hi, lo) float pairs in the same 8 bytes
+    for (double& v : metrics) {
+      const float p[2] = {(float)v, (float)(v - (double)(float)v)};
+      std::memcpy(&v, p, 8);
+    }
   if ((st = A.put(&d, metrics))) return st;
   a.metrics = d;
   if ((st = A.put(&d, std::vector<double>(m->w3mn, m->w3mn + n3)))) return st;
@@ -1220,6 +1235,7 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   a.k = c->d_k;
   a.coef = c->d_coef;
   for (long i = 0; i < n2; ++i) a.D[i] = m->dxm1[i];
+  fixed_table(a.D, n, a.fd);
   c->host_w3.assign(m->w3mn, m->w3mn + n3);
   c->curved = true;
   // the fused arguments carry the source weights for the curved kernel too
@@ -2483,11 +2499,12 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
     }
     int* d_off;
     if ((st = A.put(&d_off, off))) return st;
-    if (c->form != NEKGPU_MIXED_NAIVE && !c->curved) {
-      // normalised like the residual: weight / (w3 * rx)
+    if (c->curved ? c->form == NEKGPU_MIXED : c->form != NEKGPU_MIXED_NAIVE) {
+      // normalised like the residual: weight / (w3 * rx), on curved meshes / w3
       for (int e = 0; e < c->nelt; ++e)
         if (off[e] >= 0)
-          for (long v = 0; v < n3; ++v) wd[off[e] * n3 + v] /= c->host_w3[v] * c->host_rx[e];
+          for (long v = 0; v < n3; ++v)
+            wd[off[e] * n3 + v] /= c->host_w3[v] * (c->curved ? 1.0 : c->host_rx[e]);
     }
     if (c->form == NEKGPU_MIXED && !c->curved) {
       // as (hi, lo) float pairs (~2^-48 of the weight)

@@ -32,6 +32,7 @@ struct Compact {
   std::vector<double> w3;       // nx^3 (as given by the caller)
   std::vector<double> egeom;    // per element: rx, sy, tz, area scale per slot (6)
   std::vector<int> nbr;         // 6*nelt: partner element, -1 PEC mirror
+  std::vector<double> lift;     // 6 per element: area/w3 of the slot's nodes (= A_f/w_end)
   std::vector<double> ebm1, hbm1;   // npts
   std::vector<double> bm1;          // npts
   std::vector<double> fcoef;    // 4*nxzfl: Y02, C02Y, Z02, C02Z per face node
@@ -337,18 +338,21 @@ struct CurvedDev {
   const double* u_in;
   double* u_out;
   double* k;
-  const double* coef;     // 2*npts: dt*hbm1 then dt*ebm1
+  // the mixed form's residual is res/w3: its coef, face, fcoef and src_w hold
+  // that factor, and its coef and metrics are (hi, lo) float pairs
+  const double* coef;     // 2*npts: dt*hbm1 then dt*ebm1 (mixed: times w3)
   const double* metrics;  // 9*npts: rx, ry, rz, sx, sy, sz, tx, ty, tz (cofactors)
   const double* w3;       // nx^3
-  const double* face;     // 4*nxzfl: unx, uny, unz, area
-  const double* fcoef;    // 4*nxzfl: Y02, C02Y, Z02, C02Z
+  const double* face;     // 4*nxzfl: unx, uny, unz, area/2 (mixed: over w3)
+  const double* fcoef;    // 4*nxzfl: area (mixed: over w3) times Y02, C02Y, Z02, C02Z; null when uniform
   const int* partner;     // nxzfl: volume node across the face, -1 on PEC faces
   const int* src_elem;    // nelt or null
-  const double* src_w;    // nx^3 per source element
+  const double* src_w;    // nx^3 per source element (mixed: over w3)
   double src_ft;
   double a, b;
   const double* vres;     // 6*npts volume term from the dealiased curl, or null: the curl in-kernel
-  double D[kMaxNx * kMaxNx];  // D(i,j) at [i + nx*j]
+  FixedD fd;
+  double D[kMaxFixed * kMaxFixed];  // D(i,j) at [i + nx*j]
 };
 
 // 2-D TE / TM stage (nekgpu_2d.cu): the reference's ldim = 2 arrays as given
@@ -584,7 +588,7 @@ int mixed_upload_D(int nx, const float* tab, size_t count);
 
 // nekgpu_curved.cu: one fused FP64 stage on a curvilinear mesh
 int curved_stage(Context* c, int rkstep, double time, double dt);
-// mixed stage on a curvilinear mesh (curved arrays, FP64 coefficients)
+// mixed stage on a curvilinear mesh (curved arrays, metrics and coefficients as pairs)
 int mixed_curved_stage(Context* c, int rkstep, double time, double dt);
 
 // nekgpu_2d.cu: one 2-D TE / TM stage in the reference's arithmetic

@@ -1030,14 +1030,19 @@ int launch_mixed(Context* c, const MixedDev& a, bool pdl) {
 // per-node metrics (maxwell_wght_curl, src/cem_maxwell.F:1428-1497), the
 // upwind flux with per-face-node normals and areas (cem_maxwell_flux3d,
 // src/cem_maxwell.F:922-1002) and the partner's values read directly, lift,
-// volume source, inverse mass and RK update -- the arrays of the curved FP64
-// form (CurvedDev), converted to float pairs on the fly by integer
-// operations.  The derivatives are exact-hi FP32 contractions as in the
+// volume source, inverse mass and RK update, the residual over w3 as in the
+// curved FP64 form.  The derivatives are exact-hi FP32 contractions as in the
 // affine kernel (the element's 10-bit grid per component, D in its Dh, Df,
-// Dm pieces); metrics, weights, normals, areas, face coefficients, source
-// weights and the inverse mass enter as float pairs in float-float
-// arithmetic; the RK update is FP64.  One block of NX^3 threads per element
-// (thread per node); the state of the thread's node stays in registers.
+// Dm pieces, one thread per GLL line); metrics and inverse mass come as float
+// pairs (made once on the host, or per dt) and enter in float-float
+// arithmetic, an H and an E component per packed instruction; the flux is
+// FP64 (the FP64 pipe is idle meanwhile), joined as float pairs; the RK
+// update is FP64.
+//
+// One block per element at a time, thread per node, line and face node, as in
+// k_curved_stage.  With a thread per node forming its own 18 derivatives from
+// shared memory and the flux in float pairs (128 registers, one block per SM)
+// the 12^3-element N=7 box took 148 us per stage; 125 us so (FP64 pipe 53 % busy, issue 41 %).
 // ===========================================================================
 struct PairF {
   float h, l;
@@ -1055,202 +1060,271 @@ __device__ __forceinline__ PairF padd(PairF a, PairF b) {
   two_sum(a.h, b.h, s, t);
   return PairF{s, (a.l + b.l) + t};
 }
-__device__ __forceinline__ PairF pneg(PairF a) { return PairF{-a.h, -a.l}; }
-__device__ __forceinline__ PairF psub(PairF a, PairF b) { return padd(a, pneg(b)); }
-// a x b for pair 3-vectors
-__device__ __forceinline__ void pcross(const PairF* a, const PairF* b, PairF* o) {
-  o[0] = psub(pmul(a[1], b[2]), pmul(a[2], b[1]));
-  o[1] = psub(pmul(a[2], b[0]), pmul(a[0], b[2]));
-  o[2] = psub(pmul(a[0], b[1]), pmul(a[1], b[0]));
+
+// two float pairs side by side, and acc += m * d with one pair m for both:
+// the product's error terms and the two-sum's to the low parts
+struct Pair2 {
+  float2 h, l;
+};
+__device__ __forceinline__ void pfma2(Pair2& acc, PairF m, const Pair2& d) {
+  const float2 mh = make_float2(m.h, m.h), ml = make_float2(m.l, m.l);
+  const float2 neg = make_float2(-1.0f, -1.0f);
+  const float2 p = __fmul2_rn(mh, d.h);
+  float2 e = __ffma2_rn(mh, d.h, __fmul2_rn(p, neg));
+  e = __ffma2_rn(mh, d.l, e);
+  e = __ffma2_rn(ml, d.h, e);
+  const float2 s = __fadd2_rn(acc.h, p);  // two-sum
+  const float2 bb = __ffma2_rn(acc.h, neg, s);
+  const float2 t = __fadd2_rn(__ffma2_rn(__ffma2_rn(bb, neg, s), neg, acc.h), __ffma2_rn(bb, neg, p));
+  acc.h = s;
+  acc.l = __fadd2_rn(__fadd2_rn(acc.l, e), t);
 }
 
 template <int NX>
 struct CMCfg {
   static constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
-  static constexpr int NT = (N3 + 31) / 32 * 32, NW = NT / 32;
-  static constexpr size_t off_F = 6 * (size_t)N3 * 8;            // float2 split pairs [c][v]
-  static constexpr size_t off_D = off_F + 6 * (size_t)NF * 8;    // float2 flux pairs [c][face node]
-  static constexpr size_t off_Dm = off_D + (size_t)N2 * 8;       // (Dh, Df) [i + NX l]
-  static constexpr size_t off_wmax = off_Dm + (size_t)N2 * 4;    // Dm [i + NX l]
-  static constexpr size_t off_E = off_wmax + NW * 6 * 4;
-  static constexpr size_t smem = off_E + 8 * 4;
+  static constexpr int RS = NX | 1, SZ = RS * NX, N3P = NX * SZ;  // odd rows
+  static constexpr int NT = round32(cmax(N3, NF)), NW = NT / 32;
+  static constexpr int kMinBlocks = NT > 256 ? 2 : (NT > 160 ? 3 : 4);
+  // four areas: split pairs, derivative pairs A and B (B first holds the FP64
+  // state), lifted flux pairs
+  static constexpr size_t area = 6 * (size_t)N3P * 8;
+  static constexpr size_t off_wmax = 4 * area;
+  static constexpr size_t smem = off_wmax + NW * 6 * 4;
 };
 
+// outputs [I0, I0 + NXP) of one line: hi = sum Dh uh (exact), lo = the rest
+template <int NX, int I0, int NXP>
+__device__ __forceinline__ void curved_line_outputs(const float2* u, float2* d, int step) {
+  constexpr int H = (NX + 1) / 2, HP = (NXP + 1) / 2, J0 = I0 / 2;
+  float2 x[NXP], y[HP];
+#pragma unroll
+  for (int j = 0; j < NXP; ++j) x[j] = __fmul2_rn(c_mixD[NX][0][I0 + j], u[0]);
+#pragma unroll
+  for (int j = 0; j < HP; ++j) y[j] = __fmul2_rn(c_mixD[NX][1][J0 + j], make_float2(u[0].x, u[0].x));
+#pragma unroll
+  for (int l = 1; l < NX; ++l) {
+    const float2 uu = make_float2(u[l].x, u[l].x);
+#pragma unroll
+    for (int j = 0; j < NXP; ++j) x[j] = __ffma2_rn(c_mixD[NX][0][I0 + j + NX * l], u[l], x[j]);
+#pragma unroll
+    for (int j = 0; j < HP; ++j) y[j] = __ffma2_rn(c_mixD[NX][1][J0 + j + H * l], uu, y[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NXP; ++j)
+    d[step * (I0 + j)] = make_float2(x[j].x, x[j].y + ((j & 1) ? y[j / 2].y : y[j / 2].x));
+}
+
 template <int NX>
-__global__ void __launch_bounds__(CMCfg<NX>::NT, 1) k_mixed_curved(const CurvedDev a) {
+__global__ void __launch_bounds__(CMCfg<NX>::NT, CMCfg<NX>::kMinBlocks)
+    k_mixed_curved(const __grid_constant__ CurvedDev a) {
   using C = CMCfg<NX>;
-  constexpr int N2 = C::N2, N3 = C::N3, NF = C::NF, NT = C::NT;
+  constexpr int N2 = C::N2, N3 = C::N3, NF = C::NF, N3P = C::N3P;
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s_u2 = reinterpret_cast<float2*>(smem);
-  float2* s_F = reinterpret_cast<float2*>(smem + C::off_F);
-  float2* s_Dhf = reinterpret_cast<float2*>(smem + C::off_D);
-  float* s_Dm = reinterpret_cast<float*>(smem + C::off_Dm);
+  float2* s_A = reinterpret_cast<float2*>(smem + C::area);
+  float2* s_B = reinterpret_cast<float2*>(smem + 2 * C::area);
+  float2* s_L = reinterpret_cast<float2*>(smem + 3 * C::area);
+  double* s_u64 = reinterpret_cast<double*>(smem + 2 * C::area);
   unsigned* s_wmax = reinterpret_cast<unsigned*>(smem + C::off_wmax);
-  unsigned* s_E = reinterpret_cast<unsigned*>(smem + C::off_E);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long P = a.npts;
+  const long P = a.npts, L = a.nxzfl;
   const bool node = tid < N3;
   const int vi = tid % NX, vj = (tid / NX) % NX, vk = tid / N2;
+  const int pn = vi + C::RS * vj + C::SZ * vk;
+  const bool on_face = node && (vi == 0 || vi == NX - 1 || vj == 0 || vj == NX - 1 || vk == 0 || vk == NX - 1);
   const bool first_stage = (a.a == 0.0);
-  constexpr int H = (NX + 1) / 2;
-  for (int t = tid; t < N2; t += NT) {
-    const int i = t % NX, l = t / NX;
-    s_Dhf[t] = c_mixD[NX][0][t];
-    const float2 m = c_mixD[NX][1][i / 2 + H * l];
-    s_Dm[t] = (i & 1) ? m.y : m.x;
-  }
+  // the thread's face node
+  const int f = tid / N2, fab = tid - f * N2;
+  const int fax = tid < NF ? slot_axis(f) : -1;
+  const int fvol = face_vol<NX>(f, fab % NX, fab / NX);
+  const int fi = fvol % NX, fj = (fvol / NX) % NX;
+  const int fv = fi + C::RS * fj + C::SZ * (fvol / N2);
+  const bool later = (fax > 0 && (fi == 0 || fi == NX - 1)) || (fax > 1 && (fj == 0 || fj == NX - 1));
+  // a programmatic dependent of the previous launch, as k_mixed_stage
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   for (int e = blockIdx.x; e < a.nelt; e += gridDim.x) {
-    __syncthreads();  // the previous element's shared data is consumed
+    if (e + (int)gridDim.x >= a.nelt) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const long g = (long)e * N3 + tid;
     double u[6];
-    unsigned em[6];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      u[c] = node ? a.u_in[c * P + g] : 0.0;
-      em[c] = ((unsigned)__double2hiint(u[c]) >> 20) & 0x7FFu;
-      em[c] = __reduce_max_sync(0xffffffffu, em[c]);
-    }
-    if (lane == 0)
+    for (int c = 0; c < 6; ++c) u[c] = node ? a.u_in[c * P + g] : 0.0;
+    // the face node's partner values
+    const long js = (long)e * NF + tid;
+    int pv = -1;
+    double up[6];
+    if (tid < NF) {
+      pv = a.partner[js];
+      if (pv >= 0)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) s_wmax[warp * 6 + c] = em[c];
-    __syncthreads();
-    if (tid < 6) {
-      unsigned m = 0;
-      for (int w = 0; w < C::NW; ++w) m = max(m, s_wmax[w * 6 + tid]);
-      s_E[tid] = min(max(m, 906u), 1158u);
+        for (int c = 0; c < 6; ++c) up[c] = a.u_in[c * P + pv];
     }
-    __syncthreads();
-    if (node) {  // split: uh on the element's 10-bit grid of the component, ul = u - uh
-      const float M = 12582912.0f;
+    {  // the component's largest exponent in the element
+      unsigned em[6];
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const int E = (int)s_E[c];
-        const float qv = __int_as_float((E - 905) << 23);
-        const float qi = __int_as_float((1159 - E) << 23);
-        const float uf = d2f_hi(u[c]), ulo = d2f_lo(u[c]);
-        const float uh = (__fadd_rn(__fmaf_rn(uf, qi, M), -M)) * qv;
-        s_u2[c * N3 + tid] = make_float2(uh, __fadd_rn(__fsub_rn(uf, uh), ulo));
+        if (node) s_u64[c * N3P + pn] = u[c];
+        em[c] = ((unsigned)__double2hiint(u[c]) >> 20) & 0x7FFu;
+        em[c] = __reduce_max_sync(0xffffffffu, em[c]);
       }
+      if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) s_wmax[warp * 6 + c] = em[c];
     }
     __syncthreads();
-    // ---- upwind flux per face node, float pairs ---------------------------
-    for (int t = tid; t < NF; t += NT) {
-      const int f = t / N2, ab = t - f * N2;
-      const int v = face_vol<NX>(f, ab % NX, ab / NX);
-      const long js = (long)e * NF + t, L = a.nxzfl;
-      const int pv = a.partner[js];
-      PairF JH[3], JE[3];
+    // split: uh on the element's 10-bit grid of the component, ul = u - uh
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      unsigned m = lane < C::NW ? s_wmax[lane * 6 + c] : 0u;
+      m = __reduce_max_sync(0xffffffffu, m);
+      const int E = (int)min(max(m, 906u), 1158u);
+      const float M = 12582912.0f;
+      const float qv = __int_as_float((E - 905) << 23);
+      const float qi = __int_as_float((1159 - E) << 23);
+      const float uf = d2f_hi(u[c]), ulo = d2f_lo(u[c]);
+      const float uh = (__fadd_rn(__fmaf_rn(uf, qi, M), -M)) * qv;
+      if (node) s_u2[c * N3P + pn] = make_float2(uh, __fadd_rn(__fsub_rn(uf, uh), ulo));
+    }
+    // ---- upwind flux of the face node, FP64 (k_curved_stage) --------------------
+    float2 F[6];
+    if (tid < NF) {
+      double dH[3], dE[3], fl[6];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float2 h = s_u2[c * N3 + v], ev = s_u2[(c + 3) * N3 + v];
-        if (pv >= 0) {
-          const float2 jh = jump_pair(a.u_in[c * P + pv], h), je = jump_pair(a.u_in[(c + 3) * P + pv], ev);
-          JH[c] = PairF{jh.x, jh.y};
-          JE[c] = PairF{je.x, je.y};
-        } else {  // PEC mirror: [H] = 0, [E] = -2E exactly
-          JH[c] = PairF{0.0f, 0.0f};
-          JE[c] = PairF{-2.0f * ev.x, -2.0f * ev.y};
+        const double em = s_u64[(c + 3) * N3P + fv];
+        dH[c] = pv >= 0 ? up[c] - s_u64[c * N3P + fv] : 0.0;
+        dE[c] = pv >= 0 ? up[c + 3] - em : -2.0 * em;  // PEC mirror
+      }
+      const double n[3] = {a.face[js], a.face[L + js], a.face[2 * L + js]};
+      double xE[3], xH[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int p = (c + 1) % 3, q = (c + 2) % 3;
+        xE[c] = fma(n[p], dE[q], -(n[q] * dE[p]));
+        xH[c] = fma(n[p], dH[q], -(n[q] * dH[p]));
+      }
+      if (a.fcoef) {
+        const double Y02 = a.fcoef[js], C02Y = a.fcoef[L + js], Z02 = a.fcoef[2 * L + js],
+                     C02Z = a.fcoef[3 * L + js];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int p = (c + 1) % 3, q = (c + 2) % 3;
+          fl[c] = fma(Y02, xE[c], -(C02Y * fma(n[p], xH[q], -(n[q] * xH[p]))));
+          fl[3 + c] = fma(Z02, xH[c], -(C02Z * fma(n[p], xE[q], -(n[q] * xE[p]))));
+        }
+      } else {  // Y02 = -1/2, C02Y = Z02 = C02Z = 1/2 times the area
+        const double h = a.face[3 * L + js];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int p = (c + 1) % 3, q = (c + 2) % 3;
+          fl[c] = -h * fma(n[p], xH[q], fma(-n[q], xH[p], xE[c]));
+          fl[3 + c] = h * fma(-n[p], xE[q], fma(n[q], xE[p], xH[c]));
         }
       }
-      const PairF n[3] = {pr(a.face[js]), pr(a.face[L + js]), pr(a.face[2 * L + js])};
-      const PairF area = pr(a.face[3 * L + js]);
-      PairF Y02{-0.5f, 0.0f}, C02Y{0.5f, 0.0f}, Z02{0.5f, 0.0f}, C02Z{0.5f, 0.0f};
-      if (a.fcoef) {
-        Y02 = pr(a.fcoef[js]); C02Y = pr(a.fcoef[L + js]);
-        Z02 = pr(a.fcoef[2 * L + js]); C02Z = pr(a.fcoef[3 * L + js]);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) F[c] = make_float2(d2f_hi(fl[c]), d2f_lo(fl[c]));
+    }
+    // The lines of one direction run beside the lift of one axis (its two
+    // faces share no node) and the products of the direction before:
+    //   lines r -> A, lift r | lines s -> B, lift s, A | lines t -> A, lift t, B | A
+    const float2* met = reinterpret_cast<const float2*>(a.metrics);
+    Pair2 acc[3];  // (resE_i, resH_i) as pairs, resE += curl H, resH -= curl E
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c].h = acc[c].l = make_float2(0.0f, 0.0f);
+    auto lift = [&](int ax) {
+      if (fax == ax)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          float2* q = s_L + c * N3P + fv;
+          PairF v{F[c].x, F[c].y};
+          if (ax > 0 && later) v = padd(PairF{q->x, q->y}, v);
+          *q = make_float2(v.h, v.l);
+        }
+    };
+    auto lines = [&](int dir, float2* s_d) {
+      if (tid < 6 * N2) {
+        const int c = tid / N2, lam = tid - c * N2, la = lam % NX, lb = lam / NX;
+        const int base = c * N3P + (dir == 0 ? C::RS * la + C::SZ * lb : (dir == 1 ? la + C::SZ * lb : la + C::RS * lb));
+        const int step = dir == 0 ? 1 : (dir == 1 ? C::RS : C::SZ);
+        float2 ul[NX];
+#pragma unroll
+        for (int l = 0; l < NX; ++l) ul[l] = s_u2[base + step * l];
+        constexpr int HALF = NX > 4 ? (NX + 3) / 4 * 2 : NX;  // even: two batches of outputs
+        curved_line_outputs<NX, 0, HALF>(ul, s_d + base, step);
+        if constexpr (HALF < NX) curved_line_outputs<NX, HALF, NX - HALF>(ul, s_d + base, step);
       }
-      // n x [E], n x [H] (the gs sums of -n x E, -n x H), then the upwind terms
-      PairF nE[3], nH[3], fu[3], fw[3];
-      pcross(n, JE, nE);
-      pcross(n, JH, nH);
-      pcross(n, nH, fu);
-      pcross(n, nE, fw);
+    };
+    auto products = [&](int dir, const float2* s_d) {
+      if (!node) return;
+      PairF m[3];
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) {
+        const float2 v = met[(3 * dir + ax) * P + g];
+        m[ax] = PairF{v.x, v.y};
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int p1 = (q + 1) % 3, p2 = (q + 2) % 3;
+        const float2 h = s_d[q * N3P + pn], v = s_d[(3 + q) * N3P + pn];
+        const Pair2 d{make_float2(h.x, -v.x), make_float2(h.y, -v.y)};
+        pfma2(acc[p2], PairF{-m[p1].h, -m[p1].l}, d);
+        pfma2(acc[p1], m[p2], d);
+      }
+    };
+    __syncthreads();
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      float2* into = dir == 1 ? s_B : s_A;
+      lift(dir);
+      lines(dir, into);
+      if (dir > 0) products(dir - 1, dir == 1 ? s_A : s_B);
+      __syncthreads();
+    }
+    products(2, s_A);
+    if (on_face)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const PairF fh = pmul(area, psub(pmul(Y02, nE[c]), pmul(C02Y, fu[c])));
-        const PairF fe = pmul(area, psub(pmul(Z02, nH[c]), pmul(C02Z, fw[c])));
-        s_F[c * NF + t] = make_float2(fh.h, fh.l);
-        s_F[(3 + c) * NF + t] = make_float2(fe.h, fe.l);
+        const float2 fh = s_L[c * N3P + pn], fe = s_L[(3 + c) * N3P + pn];
+        const PairF e1 = padd(PairF{acc[c].h.x, acc[c].l.x}, PairF{fe.x, fe.y});
+        const PairF h1 = padd(PairF{acc[c].h.y, acc[c].l.y}, PairF{fh.x, fh.y});
+        acc[c].h = make_float2(e1.h, h1.h);
+        acc[c].l = make_float2(e1.l, h1.l);
       }
-    }
-    __syncthreads();
-    if (!node) continue;
-    // ---- derivatives (exact-hi contractions) and the weighted curl -----------
-    // d_dir u_c at the node as a pair: hi = sum Dh uh (exact), lo = the rest
-    auto deriv = [&](int c, int dir) {
-      const float2* pu = s_u2 + c * N3;
-      const int row = dir == 0 ? vi : (dir == 1 ? vj : vk);
-      float2 x = make_float2(0.0f, 0.0f);
-      float m = 0.0f;
+    if (node) {
+      // ---- volume source (usersrc) ------------------------------------------------
+      float Rh[6], Rl[6];
 #pragma unroll
-      for (int l = 0; l < NX; ++l) {
-        const int q = dir == 0 ? l + NX * vj + N2 * vk
-                               : (dir == 1 ? vi + NX * l + N2 * vk : vi + NX * vj + N2 * l);
-        const float2 uu = pu[q];
-        x = __ffma2_rn(s_Dhf[row + NX * l], uu, x);
-        m = fmaf(s_Dm[row + NX * l], uu.x, m);
+      for (int c = 0; c < 3; ++c) {
+        Rh[c] = acc[c].h.y; Rl[c] = acc[c].l.y;
+        Rh[3 + c] = acc[c].h.x; Rl[3 + c] = acc[c].l.x;
       }
-      return PairF{x.x, x.y + m};
-    };
-    // curl_k = eps(k, ax, q) d u_q / d x_ax with d/dx_ax = sum_dir metric(dir, ax) d/d_dir,
-    // accumulated direction by direction (one row of D live at a time): the
-    // two axes other than q give
-    //   w[(q+2)%3] -= metric(dir, (q+1)%3) du_q/d_dir,  w[(q+1)%3] += metric(dir, (q+2)%3) du_q/d_dir
-    PairF w[6] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f},
-                  {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};  // curl H, curl E
-#pragma unroll
-    for (int dir = 0; dir < 3; ++dir) {
-      const PairF m3[3] = {pr(a.metrics[(3 * dir) * P + g]), pr(a.metrics[(3 * dir + 1) * P + g]),
-                           pr(a.metrics[(3 * dir + 2) * P + g])};  // r|s|t x, y, z
+      if (a.src_elem) {
+        const int so = a.src_elem[e];
+        if (so >= 0) {
+          const PairF w = pr(a.src_w[(long)so * N3 + tid]), t = pr(a.src_ft);
+          add_pair_product(Rh[5], Rl[5], make_float2(w.h, w.l), make_float2(t.h, t.l));
+        }
+      }
+      // ---- inverse mass (pair product) and the FP64 RK update -----------------------
+      const float2* cf = reinterpret_cast<const float2*>(a.coef);
+      const float2 ch = cf[g], ce = cf[P + g];
+      double kk[6], uu[6];  // all twelve loads before the stores (k may be read and written)
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const int q = c % 3, o = c - q;
-        const PairF d = deriv(c, dir);
-        w[o + (q + 2) % 3] = psub(w[o + (q + 2) % 3], pmul(d, m3[(q + 1) % 3]));
-        w[o + (q + 1) % 3] = padd(w[o + (q + 1) % 3], pmul(d, m3[(q + 2) % 3]));
+        kk[c] = first_stage ? 0.0 : a.k[c * P + g];
+        uu[c] = a.u_in[c * P + g];
       }
-    }
-    const PairF w3 = pr(a.w3[tid]);
-    PairF res[6];  // resH = -W curl E, resE = W curl H
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      res[q] = pneg(pmul(w3, w[3 + q]));
-      res[3 + q] = pmul(w3, w[q]);
-    }
-    // ---- lift in face-slot order ---------------------------------------------
-    auto add = [&](int f, int ab) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const float2 F = s_F[c * NF + f * N2 + ab];
-        res[c] = padd(res[c], PairF{F.x, F.y});
+        const float2 w = c < 3 ? ch : ce;
+        const PairF p = pmul(PairF{Rh[c], Rl[c]}, PairF{w.x, w.y});
+        float s, t;
+        two_sum(p.h, p.l, s, t);
+        const double r = pair_to_double(s, t);
+        const double kn = first_stage ? r : fma(a.a, kk[c], r);
+        a.k[c * P + g] = kn;
+        a.u_out[c * P + g] = fma(a.b, kn, uu[c]);
       }
-    };
-    if (vj == 0) add(0, vi + NX * vk);
-    if (vi == NX - 1) add(1, vj + NX * vk);
-    if (vj == NX - 1) add(2, vi + NX * vk);
-    if (vi == 0) add(3, vj + NX * vk);
-    if (vk == 0) add(4, vi + NX * vj);
-    if (vk == NX - 1) add(5, vi + NX * vj);
-    // ---- volume source (usersrc), mass-weighted ----------------------------------
-    if (a.src_elem) {
-      const int so = a.src_elem[e];
-      if (so >= 0) res[5] = padd(res[5], pmul(pr(a.src_w[(long)so * N3 + tid]), pr(a.src_ft)));
-    }
-    // ---- inverse mass (pair product, one DADD) and the FP64 RK update ------------
-    const PairF ch = pr(a.coef[g]), ce = pr(a.coef[P + g]);
-    double kk[6], uu[6];  // all twelve loads before the stores (k may be read and written)
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      kk[c] = first_stage ? 0.0 : a.k[c * P + g];
-      uu[c] = a.u_in[c * P + g];
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const PairF p = pmul(res[c], c < 3 ? ch : ce);
-      const double r = f2d(p.h) + f2d(p.l);
-      const double kn = first_stage ? r : fma(a.a, kk[c], r);
-      a.k[c * P + g] = kn;
-      a.u_out[c * P + g] = fma(a.b, kn, uu[c]);
     }
   }
 }
@@ -1263,15 +1337,23 @@ int launch_mixed_curved(Context* c, const CurvedDev& a) {
     if (check_cuda(cudaFuncSetAttribute(k_mixed_curved<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)C::smem)))
       return NEKGPU_ERR_CUDA;
-    int per_sm = 0, sms = 0;
+    int per_sm = 0;
     if (check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mixed_curved<NX>, C::NT, C::smem)))
       return NEKGPU_ERR_CUDA;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     if (per_sm < 1) return NEKGPU_ERR_UNSUPPORTED;
-    grid = per_sm * sms;
+    grid = per_sm * num_sms(c);
   }
-  const int g = c->nelt < grid ? c->nelt : grid;
-  k_mixed_curved<NX><<<g, C::NT, C::smem, c->stream>>>(a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(c->nelt < grid ? c->nelt : grid);
+  cfg.blockDim = dim3(C::NT);
+  cfg.dynamicSmemBytes = C::smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (check_cuda(cudaLaunchKernelEx(&cfg, k_mixed_curved<NX>, a))) return NEKGPU_ERR_CUDA;
   c->last_launches += 1;
   return check_cuda(cudaGetLastError());
 }
@@ -1383,10 +1465,10 @@ int mixed_stage_range(Context* c, int rkstep, double time, double dt, int e0, in
   return st;
 }
 
-// One mixed stage on a curvilinear mesh (the curved form's arrays, FP64
-// coefficients scaled once per dt).
+// One mixed stage on a curvilinear mesh (the curved form's arrays, the
+// metrics and the coefficients, scaled once per dt, as float pairs).
 int mixed_curved_stage(Context* c, int rkstep, double time, double dt) {
-  int st = scale_coef(c, dt);
+  int st = scale_coef_pairs(c, dt);
   if (st) return st;
   CurvedDev a = c->cargs;
   a.u_in = c->d_u[c->cur];
