@@ -100,10 +100,10 @@ __device__ __forceinline__ int pnode(int v) {  // stored index of node v = i + N
 }
 
 // Field component of the k-th partner value of face f: all six with the
-// extension terms, else H and E along the two axes tangential to f.
-template <bool EXT>
+// face terms (EXT 2), else H and E along the two axes tangential to f.
+template <int EXT>
 __device__ __forceinline__ int partner_comp(int f, int k) {
-  if (EXT) return k;
+  if (EXT == 2) return k;
   const int ax = slot_axis(f);
   const int tang = (k & 1) ? (ax == 2 ? 1 : 2) : (ax == 0 ? 1 : 0);
   return (k < 2 ? 0 : 3) + tang;
@@ -277,39 +277,26 @@ __device__ __forceinline__ void line_phase(const double* s_u, double* s_R, const
 }
 
 // PML (pml_step, src/cem_maxwell_pml.F:508-590) at one node of a PML element:
-// the auxiliary residuals from res/bm1 = R * (w3 rx / bm1), their RK update
-// (src/cem_maxwell.F:1942-1955), and the PML terms added to R.
+// the auxiliary fields' RK update (src/cem_maxwell.F:1942-1955) and the PML
+// terms added to R; the coefficients are those of PmlDev (seven FP64
+// operations per component; ten from sigma, mu and bm1).
 template <int N3>
 __device__ __forceinline__ void pml_node(const Fp64Dev& a, int l, int v, const double* u,
                                          bool first_stage, double* R) {
   const long nn = a.pml.n, q = (long)l * N3 + v;
-  const double* pd = a.pml.data;
-  const double sxp = pd[q], syp = pd[nn + q], szp = pd[2 * nn + q];
-  const double sigx = pd[3 * nn + q], sigy = pd[4 * nn + q], sigz = pd[5 * nn + q];
-  const double mu = pd[6 * nn + q], fac = pd[9 * nn + q], inv = pd[10 * nn + q];
-  double* aux = a.pml.aux;
-  double* kx = a.pml.k;
-  const double bn[3] = {aux[q], aux[nn + q], aux[2 * nn + q]};
-  const double dn[3] = {aux[3 * nn + q], aux[4 * nn + q], aux[5 * nn + q]};
-  double rp[6], t[6];
-  rp[0] = R[0] * fac - syp * bn[0];
-  rp[1] = R[1] * fac - szp * bn[1];
-  rp[2] = R[2] * fac - sxp * bn[2];
-  rp[3] = R[3] * fac - syp * dn[0];
-  rp[4] = R[4] * fac - szp * dn[1];
-  rp[5] = R[5] * fac - sxp * dn[2];
-  t[0] = -syp * bn[0] + sxp * bn[0] - szp * mu * u[0];
-  t[1] = -szp * bn[1] + syp * bn[1] - sxp * mu * u[1];
-  t[2] = -sxp * bn[2] + szp * bn[2] - syp * mu * u[2];
-  t[3] = -syp * dn[0] + sxp * dn[0] - sigz * u[3];
-  t[4] = -szp * dn[1] + syp * dn[1] - sigx * u[4];
-  t[5] = -sxp * dn[2] + szp * dn[2] - sigy * u[5];
+  const double* pd = a.pml.data + q;
+  double* aux = a.pml.aux + q;
+  double* kx = a.pml.k + q;
+  const double fac = pd[12 * nn];
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
-    R[c] += t[c] * inv;  // res += t bm1
-    const double kv = first_stage ? a.dt * rp[c] : fma(a.a, kx[c * nn + q], a.dt * rp[c]);
-    kx[c * nn + q] = kv;
-    aux[c * nn + q] = fma(a.b, kv, c < 3 ? bn[c] : dn[c - 3]);
+    const int d = c % 3;
+    const double f = aux[c * nn];
+    const double rp = fma(R[c], fac, -(pd[d * nn] * f));
+    const double kv = first_stage ? a.dt * rp : fma(a.a, kx[c * nn], a.dt * rp);
+    R[c] = fma(pd[(3 + d) * nn], f, fma(-pd[(c < 3 ? 6 : 9) * nn + d * nn], u[c], R[c]));
+    kx[c * nn] = kv;
+    aux[c * nn] = fma(a.b, kv, f);
   }
 }
 
@@ -393,17 +380,17 @@ __device__ __noinline__ void face_extras(const Fp64Dev& a, int e, int t, int f, 
   }
 }
 
-template <int NX, bool EXT>
+template <int NX, int EXT>
 constexpr int fp64_min_blocks() {
   return NX == 9 || EXT ? 2 : (NX == 8 ? 3 : 4);
 }
 
-template <int NX, bool EXT, bool SPLIT>
+template <int NX, int EXT, bool SPLIT>
 __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
     k_fp64_stage(const __grid_constant__ Fp64Dev a, int nsplit, int og) {
   using C = DCfg<NX>;
   constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF;
-  constexpr int NPC = EXT ? 6 : 4;
+  constexpr int NPC = EXT == 2 ? 6 : 4;
   extern __shared__ __align__(16) unsigned char smem[];
   double* s_u = reinterpret_cast<double*>(smem);
   double* s_R = reinterpret_cast<double*>(smem + C::off_R);
@@ -480,23 +467,29 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
       // [E] = -2 E)
       const int ta = ax == 0 ? 1 : 0, tb = ax == 2 ? 1 : 2;
       double JHa, JHb, JEa, JEb;
-      if (EXT) {
+      if (EXT == 2) {
         double h[3], ev[3], JH[3], JE[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           h[c] = s_u[c * C::N3P + pv];
           ev[c] = s_u[(3 + c) * C::N3P + pv];
           JH[c] = pe >= 0 ? nbv[q][c] - h[c] : 0.0;
-          JE[c] = pe >= 0 ? nbv[q][EXT ? 3 + c : 0] - ev[c] : -2.0 * ev[c];
+          JE[c] = pe >= 0 ? nbv[q][EXT == 2 ? 3 + c : 0] - ev[c] : -2.0 * ev[c];
         }
         if (a.inc_elem || a.gr.elem) {
           double hp[3], ep[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             hp[c] = pe >= 0 ? nbv[q][c] : 0.0;
-            ep[c] = pe >= 0 ? nbv[q][EXT ? 3 + c : 0] : 0.0;
+            ep[c] = pe >= 0 ? nbv[q][EXT == 2 ? 3 + c : 0] : 0.0;
           }
-          face_extras<NX>(a, e, j, f, pe, h, ev, hp, ep, first_stage, JH, JE);
+          double jh[3], je[3];
+          face_extras<NX>(a, e, j, f, pe, h, ev, hp, ep, first_stage, jh, je);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            JH[c] = jh[c];
+            JE[c] = je[c];
+          }
         }
         JHa = ax == 0 ? JH[1] : JH[0];
         JHb = ax == 2 ? JH[1] : JH[2];
@@ -545,8 +538,8 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
     __syncthreads();
     // ---- PML, currents, source, inverse mass, RK update, node by node ----------
     const int so = a.src_elem ? a.src_elem[e] : -1;
-    const int pml_l = (EXT && a.pml.slot) ? a.pml.slot[e] : -1;
-    const int disp_l = (EXT && a.disp.slot) ? a.disp.slot[e] : -1;
+    const int pml_l = (EXT > 0 && a.pml.slot) ? a.pml.slot[e] : -1;
+    const int disp_l = (EXT > 0 && a.disp.slot) ? a.disp.slot[e] : -1;
 #pragma unroll 1
     for (int v = tid + sl.k0 * N2; v < sl.k1 * N2; v += NT) {
       const int pv = pnode<NX>(v);
@@ -560,8 +553,8 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
         R[c] = s_R[c * C::N3P + pv];
         u[c] = s_u[c * C::N3P + pv];
       }
-      if (EXT && pml_l >= 0) pml_node<N3>(a, pml_l, v, u, first_stage, R);
-      if (EXT && disp_l >= 0) disp_node<N3>(a, disp_l, v, u, first_stage, R);
+      if (EXT > 0 && pml_l >= 0) pml_node<N3>(a, pml_l, v, u, first_stage, R);
+      if (EXT > 0 && disp_l >= 0) disp_node<N3>(a, disp_l, v, u, first_stage, R);
       if (so >= 0) R[5] = fma(a.src_w[(long)so * N3 + v], a.src_ft, R[5]);
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
@@ -575,7 +568,7 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
   }
 }
 
-template <int NX, bool EXT, bool SPLIT>
+template <int NX, int EXT, bool SPLIT>
 int launch(Context* c, const Fp64Dev& a, bool pdl, int nsplit, int og) {
   using C = DCfg<NX>;
   constexpr size_t smem = C::smem(SPLIT);
@@ -613,7 +606,7 @@ int launch(Context* c, const Fp64Dev& a, bool pdl, int nsplit, int og) {
 // two, 12.7 in four, 13.4 unsplit).  With more elements the slabs only repeat
 // the staging and the t-lines' conversions (100 elements, N=7: 13.4 us
 // unsplit, 14.6 in two).
-template <int NX, bool EXT>
+template <int NX, int EXT>
 int dispatch_split(Context* c, const Fp64Dev& a, bool pdl) {
   // outputs per task of a split line: three at NX = 9 (10.0 against 10.6 us
   // with five), halves otherwise (64 elements, N=7: 10.8 us, 12.1 with three,
@@ -623,7 +616,7 @@ int dispatch_split(Context* c, const Fp64Dev& a, bool pdl) {
   return ns >= 2 ? launch<NX, EXT, true>(c, a, pdl, ns, og) : launch<NX, EXT, false>(c, a, pdl, 1, NX);
 }
 
-template <bool EXT>
+template <int EXT>
 int dispatch(Context* c, const Fp64Dev& a, bool pdl) {
   switch (c->nx) {
     case 3: return dispatch_split<3, EXT>(c, a, pdl);
@@ -644,8 +637,8 @@ int fp64_launch(Context* c, Fp64Dev& a, int rkstep, double time, double dt, bool
   a.src_elem = c->fargs.src_elem;
   a.src_w = reinterpret_cast<const double*>(c->fargs.src_w);
   if (c->src.enabled) a.src_ft = source_ft(c->src, time + dt * c->rk_c[rkstep - 1]);
-  const bool ext = a.pml.slot || a.disp.slot || a.inc_elem || a.gr.elem;
-  return ext ? dispatch<true>(c, a, pdl) : dispatch<false>(c, a, pdl);
+  if (a.inc_elem || a.gr.elem) return dispatch<2>(c, a, pdl);
+  return a.pml.slot || a.disp.slot ? dispatch<1>(c, a, pdl) : dispatch<0>(c, a, pdl);
 }
 
 }  // namespace

@@ -896,15 +896,18 @@ int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
     slot[e] = (int)l;
     for (long v = 0; v < n3; ++v) {
       const long j = e * n3 + v, q = l * n3 + v;
+      const double nrm = cp.bm1[j] / (cp.w3[v] * cp.egeom[9 * e]);
       for (int ax = 0; ax < 3; ++ax) {
-        d[ax * nn + q] = p.sigma[j + ax * npts] / p.eps[j];
-        d[(3 + ax) * nn + q] = p.sigma[j + ax * npts];
+        const double sig2 = p.sigma[j + ((ax + 2) % 3) * npts];
+        const double s0 = p.sigma[j + ax * npts] / p.eps[j];
+        const double s1 = p.sigma[j + ((ax + 1) % 3) * npts] / p.eps[j];
+        d[ax * nn + q] = s1;
+        d[(3 + ax) * nn + q] = nrm * (s0 - s1);
+        d[(6 + ax) * nn + q] = nrm * (sig2 / p.eps[j] * p.mu[j]);
+        d[(9 + ax) * nn + q] = nrm * sig2;
+        d[(13 + ax) * nn + q] = p.sigma[j + ax * npts];
       }
-      d[6 * nn + q] = p.mu[j];
-      d[7 * nn + q] = cp.bm1[j];
-      d[8 * nn + q] = 1.0 / cp.bm1[j];
-      d[9 * nn + q] = cp.w3[v] * cp.egeom[9 * e] / cp.bm1[j];
-      d[10 * nn + q] = cp.bm1[j] / (cp.w3[v] * cp.egeom[9 * e]);
+      d[12 * nn + q] = cp.w3[v] * cp.egeom[9 * e] / cp.bm1[j];
     }
   }
   int st;
@@ -2014,8 +2017,8 @@ int nekgpu_get_array(nekgpu_ctx* c, const char* name, double* out) {
     for (long v = 0; v < n3; ++v) {
       const long q = l * n3 + v, g = (long)c->pml_elems[l] * n3 + v;
       for (int cc = 0; cc < 3; ++cc) {
-        if (sg)  // sigma = (sigma/eps) * eps is not stored; sigma itself is q = 3..5
-          out[cc * P + g] = h[(3 + cc) * nn + q];
+        if (sg)
+          out[cc * P + g] = h[(13 + cc) * nn + q];
         else
           out[cc * P + g] = h[((dn ? 3 : 0) + cc) * nn + q];
       }

@@ -136,11 +136,14 @@ struct PlainDev {
 };
 
 // PML data of the fused forms, compact over the PML elements (slot l holds
-// element pml_elem[l]); per node of a PML element, [q][l*N3 + v]:
-//   q = 0..2 sigma/eps (x, y, z), 3..5 sigma (x, y, z), 6 mu, 7 bm1, 8 1/bm1,
-//   9 w3*rx/bm1 (the mixed form's normalised residual R: res/bm1 = R * [9]),
-//   10 bm1/(w3*rx) (a residual term t enters R as t * [10])
-constexpr int kPmlData = 11;
+// element pml_elem[l]).  With s = sigma/eps and, for component c = x, y, z of
+// B and of D, s0, s1, s2 its values along c and the two next axes, pml_step
+// (src/cem_maxwell_pml.F:508-590) is, f the auxiliary field,
+//   df/dt = res/bm1 - s1 f,   res += bm1 ((s0 - s1) f - s2 mu H | - sigma_2 E).
+// Per node of a PML element, [q][l*N3 + v]: q = 0..2 s1; with the residual
+// R = res/(w3 rx) and n = bm1/(w3 rx), 3..5 n (s0 - s1), 6..8 n s2 mu, 9..11
+// n sigma_2, 12 1/n; 13..15 sigma along x, y, z (read back by the host only).
+constexpr int kPmlData = 16;
 struct PmlDev {
   const int* slot;        // nelt: PML slot of the element, -1 outside
   const double* data;     // kPmlData * n

@@ -40,6 +40,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "nekgpu_internal.h"
 #include "nekgpu_pair.cuh"
 
@@ -159,10 +161,14 @@ __device__ __forceinline__ int opaque_tid() {
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
 constexpr int round32(int a) { return (a + 31) / 32 * 32; }
 
-// TPL: threads per line task (2: each computes half of a line's outputs, for
-// meshes with fewer elements than SMs, where the time per stage is one
-// element's latency)
-template <int NX, int TPL = 1>
+// First k-layer of slab s of S (even, so that the outputs' float pairs of D
+// stay whole), and the slab of a part of a line's outputs alike
+template <int NX, int S>
+__host__ __device__ constexpr int slab_lo(int s) {
+  return s >= S ? NX : (s * NX / S) & ~1;
+}
+
+template <int NX>
 struct MCfg {
   static constexpr int N2 = NX * NX, N3 = N2 * NX;
   // Node layout of the FP32 pair arrays.  NX = 8: unpadded, node
@@ -176,20 +182,20 @@ struct MCfg {
   static constexpr int N3P = NX * SZ;
   static constexpr int NF = 6 * N2;
   static constexpr int NTASK = 4 * N2;  // line tasks per direction
-  static constexpr int NT = round32(cmax(NTASK * TPL, (N3 + 1) / 2));
+  static constexpr int NT = round32(cmax(NTASK, (N3 + 1) / 2));
   static constexpr int NW = NT / 32;
   static constexpr int NPT = (N3 + NT - 1) / NT;
   static constexpr int FPT = (NF + NT - 1) / NT;
-  static constexpr int TPT = (NTASK * TPL + NT - 1) / NT;
+  static constexpr int TPT = (NTASK + NT - 1) / NT;
   static constexpr bool kTma = (N3 % 2) == 0;
   // odd node counts: the next element staged by per-thread 8-byte async
   // copies where that measured faster (N=8 +3 %, N=6 +0.9 %; N=4, N=2 load
   // synchronously: -0.5 %, -1.8 % with the async copies)
   static constexpr bool kAsync = !kTma && NX >= 7;
   // L1 prefetch of the finish's loads where it measured faster: in the t-line
-  // tasks that finish (N=6 +2.5 %, N=4 +0.4 %; N=5 -1.9 %: it spills there)
+  // tasks that finish (N=6 +2.5 %, N=5 +1.7 %, N=4 +0.4 %)
   // and for the next node of the node-by-node finish (N=8 +1.4 %; N=7 -2.2 %)
-  static constexpr bool kPfLine = NX == 5 || NX == 7;
+  static constexpr bool kPfLine = NX == 5 || NX == 6 || NX == 7;
   static constexpr bool kPfNode = NX == 9;
   // Where the components finish (inverse mass, RK update) without the
   // extension terms: true = the t-line tasks finish H1, H2, E1, E2 on their
@@ -273,21 +279,26 @@ __device__ __forceinline__ void rk_finish_cf(const MixedDev& a, int c, long g, f
   a.k_out[c * P + g] = kn;
   a.u_out[c * P + g] = fma(a.b, kn, __ldg(a.u_in + c * P + g));
 }
-// All six components of node g: the node's RK register and state loaded
+// All six components of node v of the element whose first node is ge (the
+// rows' bases are uniform: 32-bit offsets): the node's RK register and state loaded
 // first (twelve loads in flight; the stores of one component would otherwise
 // keep the next component's loads behind them, k_out possibly being k), then
 // the six updates as in rk_finish_cf.
 template <bool IA>
-__device__ __forceinline__ void rk_finish_node(const MixedDev& a, long g, const float* Rh,
-                                               const float* Rl, float2 cfH, float2 cfE,
-                                               bool first_stage) {
+__device__ __forceinline__ void rk_finish_node(const MixedDev& a, long ge, unsigned v, const float* Rh,
+                                               const float* Rl, bool first_stage) {
   const long P = a.npts;
   double kk[6], uu[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
-    kk[c] = first_stage ? 0.0 : a.k[c * P + g];
-    uu[c] = __ldg(a.u_in + c * P + g);
+    const double* kp = a.k + (c * P + ge);
+    const double* up = a.u_in + (c * P + ge);
+    kk[c] = first_stage ? 0.0 : kp[v];
+    uu[c] = __ldg(up + v);
   }
+  const float2* ch = a.coef + ge;
+  const float2* ce = a.coef + (P + ge);
+  const float2 cfH = ch[v], cfE = ce[v];
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
     const float2 cf = c < 3 ? cfH : cfE;
@@ -304,8 +315,10 @@ __device__ __forceinline__ void rk_finish_node(const MixedDev& a, long g, const 
       r = f2d(p) + f2d(ee);
     }
     const double kn = first_stage ? r : fma(a.a, kk[c], r);
-    a.k_out[c * P + g] = kn;
-    a.u_out[c * P + g] = fma(a.b, kn, uu[c]);
+    double* ko = a.k_out + (c * P + ge);
+    double* uo = a.u_out + (c * P + ge);
+    ko[v] = kn;
+    uo[v] = fma(a.b, kn, uu[c]);
   }
 }
 template <bool IA>
@@ -349,11 +362,11 @@ __device__ __forceinline__ void add_jump(float2& J, double d) {
 }
 
 // Field component of the k-th parked partner value of face f: all six with
-// the extension terms, else H and E along the two axes tangential to f
+// the face terms (EXT 2), else H and E along the two axes tangential to f
 // (k = 0, 1: H; k = 2, 3: E; lower axis first).
-template <bool EXT>
+template <int EXT>
 __device__ __forceinline__ int partner_comp(int f, int k) {
-  if (EXT) return k;
+  if (EXT == 2) return k;
   const int ax = slot_axis(f);
   const int tang = (k & 1) ? (ax == 2 ? 1 : 2) : (ax == 0 ? 1 : 0);
   return (k < 2 ? 0 : 3) + tang;
@@ -369,16 +382,23 @@ __device__ __forceinline__ float2 jump_pair(double p, float2 own) {
   return make_float2(s, (d2f_lo(p) - own.y) + t);
 }
 
-// Outputs I0 .. I0+NXP-1 of one line task (all NX of them, or one half when
-// two threads share the line): the contraction, the rho factor, the lifted
+// two_sum(a, sg * b) for sg = +-1
+__device__ __forceinline__ void signed_sum(float a, float sg, float b, float& s, float& e) {
+  s = fmaf(sg, b, a);
+  const float bb = s - a;
+  e = (a - (s - bb)) + fmaf(sg, b, -bb);
+}
+
+// Outputs I0 .. I0+NXP-1 of one line task (all NX of them, or the part of one
+// of the threads that share the line): the contraction, the rho factor, the lifted
 // flux at the line's ends and the accumulation into the residual pairs (or,
 // FIN, the finish).
-template <int NX, int DIR, bool FIN, int TPL, int I0, int NXP>
+template <int NX, int DIR, bool FIN, int I0, int NXP>
 __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2 flux_m,
                                              float2 flux_p, bool cubic, float rh, float rl,
                                              float sg, bool init, int la, int lb, int rt,
                                              const MixedDev& a, int e, bool first_stage) {
-  using C = MCfg<NX, TPL>;
+  using C = MCfg<NX>;
   // packed in float pairs:
   //   (hi_i, lo_i)   += (Dh, Df)(i,l) * (uh, ul)_l      hi exact
   //   (m_i, m_i+1)   += (Dm(i,l), Dm(i+1,l)) * (uh, uh)_l
@@ -409,20 +429,26 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
       h = p;
       r = ee;
     }
-    h *= sg;
-    r *= sg;
-    if (i == 0 || i == NX - 1) {  // the lifted flux pair of the end's face
+    const bool end = i == 0 || i == NX - 1;
+    if (end || (!FIN && init)) {
+      h *= sg;
+      r *= sg;
+    }
+    if (end) {  // the lifted flux pair of the end's face
       const float2 F = i == 0 ? flux_m : flux_p;
       float s, t;
       two_sum(h, F.x, s, t);
       h = s;
       r = (r + F.y) + t;
     }
+    // the sign of an inner output rides on the additions (sg h is exact)
+    const float sa = end ? 1.0f : sg;
     float2* Rp = R0 + line_node<NX, DIR>(la, lb, i);
     if (FIN) {
       const float2 old = *Rp;
       float sum, err;
-      two_sum(old.x, h, sum, err);
+      signed_sum(old.x, sa, h, sum, err);
+      r *= sa;
       const int vol = DIR == 0 ? i + NX * la + C::N2 * lb
                                : (DIR == 1 ? la + NX * i + C::N2 * lb : la + NX * lb + C::N2 * i);
       rk_finish<C::kIntAdd>(a, rt, (long)e * C::N3 + vol, sum, (old.y + r) + err, first_stage);
@@ -431,8 +457,8 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
     } else {
       const float2 old = *Rp;
       float sum, err;
-      two_sum(old.x, h, sum, err);
-      *Rp = make_float2(sum, (old.y + r) + err);
+      signed_sum(old.x, sa, h, sum, err);
+      *Rp = make_float2(sum, fmaf(sa, r, old.y) + err);
     }
   }
 }
@@ -443,23 +469,27 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
 // task's residual component (s_F, stored in this direction's slot order) is
 // added to their low parts.  FIN (last direction): the residual of the
 // task's component is complete at the line's nodes, so the task finishes
-// them (inverse mass, RK update) instead of storing the pairs.  TPL = 2: two
-// threads per line, each with half of its outputs (the halves in separate
-// warps, so the branch on the half is warp-uniform).
-template <int NX, int DIR, bool FIN, int TPL = 1>
+// them (inverse mass, RK update) instead of storing the pairs.  S > 1: the
+// block's k-slab only -- r- and s-lines inside the slab, S threads on each
+// with the outputs of one part (part-major: warp-uniform at NX = 8), t-lines
+// with the slab's outputs.
+template <int NX, int DIR, bool FIN, int S>
 __device__ __forceinline__ void line_phase(const float2* s_u2, float2* s_R2, const float2* s_F,
                                            bool cubic, float rh, float rl, const MixedDev& a,
-                                           int e, bool first_stage) {
-  using C = MCfg<NX, TPL>;
-  static_assert(TPL == 1 || (TPL == 2 && !FIN && NX % 4 == 0), "two threads per line: NX = 4k, no FIN");
+                                           int e, bool first_stage, int slab) {
+  using C = MCfg<NX>;
   const int tid = opaque_tid();
+  const int k0 = S == 1 ? 0 : slab_lo<NX, S>(slab), k1 = S == 1 ? NX : slab_lo<NX, S>(slab + 1);
+  const int nl = S > 1 && DIR < 2 ? NX * (k1 - k0) : C::N2;  // lines per component
+  const int ntask = 4 * nl * (DIR < 2 ? S : 1);
+  constexpr int ROUNDS = S > 1 ? (4 * C::N2 * (DIR < 2 ? 2 : 1) + C::NT - 1) / C::NT : C::TPT;
 #pragma unroll
-  for (int q = 0; q < C::TPT; ++q) {
+  for (int q = 0; q < ROUNDS; ++q) {
     const int task = tid + q * C::NT;
-    if (task < C::NTASK * TPL) {
-      const int part = TPL == 1 ? 0 : task / C::NTASK;
-      const int lt = task - part * C::NTASK;
-      const int slot = lt / C::N2, lam = lt - slot * C::N2;
+    if (task < ntask) {
+      const int part = S > 1 ? (DIR < 2 ? task / (4 * nl) : slab) : 0;
+      const int lt = S > 1 && DIR < 2 ? task - part * 4 * nl : task;
+      const int slot = lt / nl, lam = lt - slot * nl + (S > 1 && DIR < 2 ? NX * k0 : 0);
       const int la = lam % NX, lb = lam / NX;
       const int comp = kLineComp[DIR][slot], rt = kLineRes[DIR][slot];
       const float sg = kLineSign[DIR][slot];
@@ -469,6 +499,7 @@ __device__ __forceinline__ void line_phase(const float2* s_u2, float2* s_R2, con
         const long P = a.npts;
 #pragma unroll
         for (int i = 0; i < NX; ++i) {
+          if (S > 1 && (i < k0 || i >= k1)) continue;
           const int vol = DIR == 0 ? i + NX * la + C::N2 * lb
                                    : (DIR == 1 ? la + NX * i + C::N2 * lb : la + NX * lb + C::N2 * i);
           const long g = (long)e * C::N3 + vol;
@@ -485,65 +516,63 @@ __device__ __forceinline__ void line_phase(const float2* s_u2, float2* s_R2, con
 #pragma unroll
       for (int l = 0; l < NX; ++l) u[l] = pu[line_node<NX, DIR>(la, lb, l)];
       float2* R0 = s_R2 + rt * C::N3P;
-      if constexpr (TPL == 1) {
-        line_outputs<NX, DIR, FIN, TPL, 0, NX>(u, R0, flux_m, flux_p, cubic, rh, rl, sg, init, la, lb,
-                                               rt, a, e, first_stage);
-      } else if (part == 0) {
-        line_outputs<NX, DIR, FIN, TPL, 0, NX / 2>(u, R0, flux_m, flux_p, cubic, rh, rl, sg, init, la,
-                                                   lb, rt, a, e, first_stage);
+      auto outputs = [&](auto p) {
+        constexpr int I0 = slab_lo<NX, S>(decltype(p)::value), NP = slab_lo<NX, S>(decltype(p)::value + 1) - I0;
+        line_outputs<NX, DIR, FIN, I0, NP>(u, R0, flux_m, flux_p, cubic, rh, rl, sg, init, la, lb, rt,
+                                           a, e, first_stage);
+      };
+      if constexpr (S == 1) {
+        outputs(std::integral_constant<int, 0>{});
+      } else if constexpr (S == 2) {
+        if (part == 0) outputs(std::integral_constant<int, 0>{});
+        else outputs(std::integral_constant<int, 1>{});
+      } else if constexpr (S == 3) {
+        if (part == 0) outputs(std::integral_constant<int, 0>{});
+        else if (part == 1) outputs(std::integral_constant<int, 1>{});
+        else outputs(std::integral_constant<int, 2>{});
       } else {
-        line_outputs<NX, DIR, FIN, TPL, NX / 2, NX / 2>(u, R0, flux_m, flux_p, cubic, rh, rl, sg, init,
-                                                        la, lb, rt, a, e, first_stage);
+        static_assert(S == 4, "one to four slabs");
+        if (part == 0) outputs(std::integral_constant<int, 0>{});
+        else if (part == 1) outputs(std::integral_constant<int, 1>{});
+        else if (part == 2) outputs(std::integral_constant<int, 2>{});
+        else outputs(std::integral_constant<int, 3>{});
       }
     }
   }
 }
 
 // PML (pml_step, src/cem_maxwell_pml.F:508-590) at one node of a PML element,
-// in FP64: the auxiliary residuals from res/bm1 = R * (w3 rx / bm1), their RK
-// update (src/cem_maxwell.F:1942-1955), and the PML terms of res added to the
-// normalised residual pair R as FP32 pairs.
+// in FP64: the auxiliary fields' RK update (src/cem_maxwell.F:1942-1955), and
+// the PML terms added to the normalised residual pair R as FP32 pairs; the
+// coefficients are those of PmlDev.
 template <int N3>
 __device__ __forceinline__ void pml_node(const MixedDev& a, int l, int v, long g, bool first_stage,
-                                      float* Rh, float* Rl) {
+                                         float* Rh, float* Rl) {
   const long nn = a.pml.n, q = (long)l * N3 + v, P = a.npts;
-  const double* pd = a.pml.data;
-  const double sxp = pd[q], syp = pd[nn + q], szp = pd[2 * nn + q];
-  const double sigx = pd[3 * nn + q], sigy = pd[4 * nn + q], sigz = pd[5 * nn + q];
-  const double mu = pd[6 * nn + q], fac = pd[9 * nn + q], inv = pd[10 * nn + q];
-  double* aux = a.pml.aux;
-  double* kx = a.pml.k;
-  double bn[3], dn[3], hn[3], en[3], rp[6];
-  for (int c = 0; c < 3; ++c) {
-    bn[c] = aux[c * nn + q];
-    dn[c] = aux[(3 + c) * nn + q];
-    hn[c] = __ldg(a.u_in + c * P + g);
-    en[c] = __ldg(a.u_in + (3 + c) * P + g);
-  }
-  double rb[6];
-  for (int c = 0; c < 6; ++c) rb[c] = (f2d(Rh[c]) + f2d(Rl[c])) * fac;
-  rp[0] = rb[0] - syp * bn[0];
-  rp[1] = rb[1] - szp * bn[1];
-  rp[2] = rb[2] - sxp * bn[2];
-  rp[3] = rb[3] - syp * dn[0];
-  rp[4] = rb[4] - szp * dn[1];
-  rp[5] = rb[5] - sxp * dn[2];
-  double t[6];
-  t[0] = -syp * bn[0] + sxp * bn[0] - szp * mu * hn[0];
-  t[1] = -szp * bn[1] + syp * bn[1] - sxp * mu * hn[1];
-  t[2] = -sxp * bn[2] + szp * bn[2] - syp * mu * hn[2];
-  t[3] = -syp * dn[0] + sxp * dn[0] - sigz * en[0];
-  t[4] = -szp * dn[1] + syp * dn[1] - sigx * en[1];
-  t[5] = -sxp * dn[2] + szp * dn[2] - sigy * en[2];
+  const double* pd = a.pml.data + q;
+  double* aux = a.pml.aux + q;
+  double* kx = a.pml.k + q;
+  const double fac = pd[12 * nn];
+  double f[6], kk[6], u[6];  // loaded before the stores (which they could not pass)
+#pragma unroll
   for (int c = 0; c < 6; ++c) {
-    const double dR = t[c] * inv;  // res += t bm1  ->  R += t bm1 / (w3 rx)
+    f[c] = aux[c * nn];
+    kk[c] = first_stage ? 0.0 : kx[c * nn];
+    u[c] = __ldg(a.u_in + c * P + g);
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const int d = c % 3;
     float s, e;
+    two_sum(Rh[c], Rl[c], s, e);
+    const double rp = fma(pair_to_double(s, e), fac, -(pd[d * nn] * f[c]));
+    const double kv = first_stage ? a.dt * rp : fma(a.a, kk[c], a.dt * rp);
+    const double dR = fma(pd[(3 + d) * nn], f[c], -(pd[(c < 3 ? 6 : 9) * nn + d * nn] * u[c]));
     two_sum(Rh[c], d2f_hi(dR), s, e);
     Rh[c] = s;
     Rl[c] = (Rl[c] + d2f_lo(dR)) + e;
-    const double kv = first_stage ? a.dt * rp[c] : fma(a.a, kx[c * nn + q], a.dt * rp[c]);
-    kx[c * nn + q] = kv;
-    aux[c * nn + q] = fma(a.b, kv, c < 3 ? bn[c] : dn[c - 3]);
+    kx[c * nn] = kv;
+    aux[c * nn] = fma(a.b, kv, f[c]);
   }
 }
 
@@ -581,24 +610,74 @@ __device__ __forceinline__ void disp_node(const MixedDev& a, int l, int v, long 
   }
 }
 
+// Incident field (userinc) and graphene sheet (userfsrc) terms of face node t
+// of element e added to its jumps JH, JE (FP64 differences; listed elements
+// only): the incident field on the own side of a listed face node, or on the
+// partner's side when the partner's slot is listed; the sheet's currents on
+// both sides as n x [H] - J, i.e. [H] + n x J.
+template <int NF>
+__device__ __noinline__ void face_extras(const MixedDev& a, int e, int t, int f, int pe, double* hm,
+                                         double* em, double* hp, double* ep, bool first_stage,
+                                         float2* JH, float2* JE) {
+  const int io = a.inc_elem ? a.inc_elem[e] : -1;
+  if (io >= 0) {
+    const double* iv = a.inc_val + (long)io * 12 * NF + t;
+    for (int c = 0; c < 3; ++c) {
+      const double ho = iv[c * NF], eo = iv[(3 + c) * NF], hq = iv[(6 + c) * NF], eq = iv[(9 + c) * NF];
+      if (pe >= 0) {
+        add_jump(JH[c], hq - ho);
+        add_jump(JE[c], eq - eo);
+      } else {
+        add_jump(JE[c], -2.0 * eo);
+      }
+      hm[c] += ho;
+      em[c] += eo;
+      hp[c] += hq;
+      ep[c] += eq;
+    }
+  }
+  if (!a.gr.elem) return;
+  const int gr = a.gr.elem[e];
+  const int go = gr >= 0 ? a.gr.own[(long)gr * NF + t] : -1;
+  const int gp = gr >= 0 ? a.gr.part[(long)gr * NF + t] : -1;
+  if (go < 0 && gp < 0) return;
+  double nv[3], nm[3], J[3] = {0.0, 0.0, 0.0};
+  for (int c = 0; c < 3; ++c) {
+    nv[c] = c == slot_axis(f) ? (double)slot_side(f) : 0.0;
+    nm[c] = -nv[c];
+  }
+  if (go >= 0) graphene_slot(a.gr, go, nv, hm, em, true, first_stage, a.a, a.b, a.dt, J);
+  if (gp >= 0 && pe >= 0) graphene_slot(a.gr, gp, nm, hp, ep, false, first_stage, a.a, a.b, a.dt, J);
+  if (pe >= 0) {  // a PEC face keeps its mirror flux
+    add_jump(JH[0], nv[1] * J[2] - nv[2] * J[1]);
+    add_jump(JH[1], nv[2] * J[0] - nv[0] * J[2]);
+    add_jump(JH[2], nv[0] * J[1] - nv[1] * J[0]);
+  }
+}
+
 // Blocks per SM the launch is built for: three at NX = 8 (62 KB of shared
 // memory with the face flux as float pairs: a fourth does not fit; up to 80
 // registers), six at NX = 6 (160 threads, 32 KB, 64 registers), two at NX = 9
-// (384 threads, 94 KB), three otherwise and with the extension branches.
-template <int NX, bool EXT, int TPL = 1>
+// (384 threads, 94 KB), three otherwise and with the extension branches
+// (two, with 128 registers and no spills, take 95 instead of 60 us per stage
+// on 8^3 elements with PML at N=8).
+template <int NX, int EXT, int S>
 constexpr int mixed_min_blocks() {
-  return TPL == 2 ? 1 : (NX == 9 ? 2 : (EXT ? 3 : (NX == 6 ? 6 : 3)));
+  return NX == 9 ? 2 : (EXT || S > 1 ? 3 : (NX == 6 ? 6 : 3));
 }
 
-// EXT: the variant with the PML, dispersive-current, incident-field and
-// graphene branches
-template <int NX, bool EXT, int TPL = 1>
-__global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, TPL>())
+// EXT: 0 plain, 1 with the PML and dispersive-current terms of the nodes, 2
+// with the incident-field and graphene terms of the faces too.  S > 1: an element's k-slabs go to S blocks, for meshes
+// with few elements: every block stages and splits the whole element (the
+// t-lines need it) and works out the nodes of its slab, so the blocks share
+// nothing; the arithmetic of a node is the same.
+template <int NX, int EXT, int S>
+__global__ void __launch_bounds__(MCfg<NX>::NT, mixed_min_blocks<NX, EXT, S>())
     k_mixed_stage(const MixedDev a) {
-  using C = MCfg<NX, TPL>;
+  using C = MCfg<NX>;
   constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF, N3P = C::N3P;
   constexpr int NPT = C::NPT, FPT = C::FPT;
-  constexpr bool FIN = !EXT && C::kFin;  // the extension terms need all six at a node
+  constexpr bool FIN = EXT == 0 && C::kFin;  // the extension terms need all six at a node
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s_F = reinterpret_cast<float2*>(smem + C::off_F);
   unsigned* s_wmax = reinterpret_cast<unsigned*>(smem + C::off_wmax);
@@ -654,28 +733,43 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
   };
   unsigned parity = 0;
   int buf = 0;  // area of the element's staged state and residual pairs
-  if (C::kTma && tid == 0 && a.e_begin + (int)blockIdx.x < a.e_end) issue_tma(a.e_begin + blockIdx.x, 0);
-  if (C::kAsync && a.e_begin + (int)blockIdx.x < a.e_end) issue_async(a.e_begin + blockIdx.x, 0, tid);
+  // tasks: element w/S, slab w%S
+  const int w0 = a.e_begin * S + (int)blockIdx.x, w1 = a.e_end * S;
+  if (C::kTma && tid == 0 && w0 < w1) issue_tma(w0 / S, 0);
+  if (C::kAsync && w0 < w1) issue_async(w0 / S, 0, tid);
 
-  for (int e = a.e_begin + blockIdx.x; e < a.e_end; e += gridDim.x, buf ^= 1) {
+  for (int w = w0; w < w1; w += gridDim.x, buf ^= 1) {
     int tid = opaque_tid();
-    if (e + (int)gridDim.x >= a.e_end) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int e = w / S, slab = S == 1 ? 0 : w % S;
+    const int k0 = S == 1 ? 0 : slab_lo<NX, S>(slab), k1 = S == 1 ? NX : slab_lo<NX, S>(slab + 1);
+    if (w + (int)gridDim.x >= w1) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     double* s_u64 = reinterpret_cast<double*>(smem + buf * C::SA);
     float2* s_R2 = reinterpret_cast<float2*>(smem + buf * C::SA);
     float2* s_u2 = reinterpret_cast<float2*>(smem + (buf ^ 1) * C::SA);
-    const int en = e + gridDim.x;
+    const int wn = w + gridDim.x, en = wn / S;
     const int* nbr = a.nbr + 6 * e;
     const float* eg = a.egm + 16 * e;
     // ---- early loads: partner face nodes (kept in registers until the flux)
     // The flux of a face uses the components tangential to it: without the
     // extension terms only those four are loaded (H and E along the two
     // other axes); the graphene sheets need all six.
-    constexpr int NPC = EXT ? 6 : 4;
+    constexpr int NPC = EXT == 2 ? 6 : 4;
+    // face task q of the slab: the face node t (slot f, in-face place ab) of
+    // the element, or -1; S > 1: side-face rows of the slab, then the t faces
+    const int per = NX * (k1 - k0);
+    auto face_task = [&](int tid, int q) {
+      const int t = tid + q * NT;
+      if (S == 1) return t < NF ? t : -1;
+      if (t < 4 * per) return t / per * N2 + NX * k0 + t % per;
+      const int r = t - 4 * per, n4 = k0 == 0 ? N2 : 0;
+      if (r < n4) return 4 * N2 + r;
+      return k1 == NX && r < n4 + N2 ? 5 * N2 + r - n4 : -1;
+    };
     double nbv[FPT][NPC];
 #pragma unroll
     for (int q = 0; q < FPT; ++q) {
-      const int t = tid + q * NT;
-      if (t < NF) {
+      const int t = face_task(tid, q);
+      if (t >= 0) {
         const int f = t / N2, ab = t - f * N2;
         const int pe = nbr[f];
         if (pe >= 0) {
@@ -763,15 +857,15 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
     double* s_nbv = s_u64;
 #pragma unroll
     for (int q = 0; q < FPT; ++q) {
-      const int t = tid + q * NT;
-      if (t < NF && nbr[t / N2] >= 0)
+      const int t = face_task(tid, q);
+      if (t >= 0 && nbr[t / N2] >= 0)
 #pragma unroll
         for (int k = 0; k < NPC; ++k) s_nbv[k * NF + t] = nbv[q][k];
     }
 #pragma unroll
     for (int q = 0; q < FPT; ++q) {
-      const int t = tid + q * NT;
-      if (t < NF) {
+      const int t = face_task(tid, q);
+      if (t >= 0) {
         const int f = t / N2, ab = t - f * N2;
         const int fa = ab % NX, fb = ab / NX;
         const int pv = pnode<NX>(face_vol<NX>(f, fa, fb));
@@ -780,68 +874,41 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
         const int ax = slot_axis(f), ta = ax == 0 ? 1 : 0;  // the tangential axes ta < tb
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          if (!EXT && c == ax) {  // the normal component: not in the flux
+          if (EXT < 2 && c == ax) {  // the normal component: not in the flux
             JH[c] = JE[c] = make_float2(0.0f, 0.0f);
             continue;
           }
           const float2 h = s_u2[c * N3P + pv], ev = s_u2[(c + 3) * N3P + pv];
           if (pe >= 0) {
-            const int kh = EXT ? c : (c == ta ? 0 : 1), ke = EXT ? c + 3 : kh + 2;
+            const int kh = EXT == 2 ? c : (c == ta ? 0 : 1), ke = EXT == 2 ? c + 3 : kh + 2;
             JH[c] = jump_pair(s_nbv[kh * NF + t], h);
             JE[c] = jump_pair(s_nbv[ke * NF + t], ev);
           } else {  // PEC mirror H+ = H-, E+ = -E-: [H] = 0, [E] = -2E exactly
             JH[c] = make_float2(0.0f, 0.0f);
             JE[c] = make_float2(-2.0f * ev.x, -2.0f * ev.y);
           }
-          if (EXT && a.inc_elem) {
-            // userinc: the incident field on the own side of a listed face
-            // node, or on the partner's side when the partner's slot is listed
-            const int io = a.inc_elem[e];
-            if (io >= 0) {  // (FP64 differences: listed elements only)
-              const double* iv = a.inc_val + (long)io * 12 * NF + t;
-              if (pe >= 0) {
-                add_jump(JH[c], iv[(6 + c) * NF] - iv[c * NF]);
-                add_jump(JE[c], iv[(9 + c) * NF] - iv[(3 + c) * NF]);
-              } else {
-                add_jump(JE[c], -2.0 * iv[(3 + c) * NF]);
-              }
-            }
-          }
         }
-        if (EXT && a.gr.elem) {
-          // graphene (userfsrc): the sheet's currents on both sides of the
-          // face node enter as n x [H] - J, i.e. [H] + n x J (FP64)
-          const int gr = a.gr.elem[e];
-          const int go = gr >= 0 ? a.gr.own[(long)gr * NF + t] : -1;
-          const int gp = gr >= 0 ? a.gr.part[(long)gr * NF + t] : -1;
-          if (go >= 0 || gp >= 0) {
-            double nv[3] = {0.0, 0.0, 0.0}, nm[3];
-            nv[slot_axis(f)] = (double)slot_side(f);
-            double fhm[3], fem[3], fhp[3], fep[3];
-            const int io = a.inc_elem ? a.inc_elem[e] : -1;
-            for (int c = 0; c < 3; ++c) {
-              nm[c] = -nv[c];
-              const float2 h = s_u2[c * N3P + pv], ev = s_u2[(c + 3) * N3P + pv];
-              fhm[c] = f2d(h.x) + f2d(h.y);
-              fem[c] = f2d(ev.x) + f2d(ev.y);
-              fhp[c] = pe >= 0 ? s_nbv[c * NF + t] : 0.0;  // EXT: all six parked
-              fep[c] = pe >= 0 ? s_nbv[(c + 3) * NF + t] : 0.0;
-              if (io >= 0) {
-                const double* iv = a.inc_val + (long)io * 12 * NF + t;
-                fhm[c] += iv[c * NF];
-                fem[c] += iv[(3 + c) * NF];
-                fhp[c] += iv[(6 + c) * NF];
-                fep[c] += iv[(9 + c) * NF];
-              }
-            }
-            double J[3] = {0.0, 0.0, 0.0};
-            if (go >= 0) graphene_slot(a.gr, go, nv, fhm, fem, true, first_stage, a.a, a.b, a.dt, J);
-            if (gp >= 0 && pe >= 0) graphene_slot(a.gr, gp, nm, fhp, fep, false, first_stage, a.a, a.b, a.dt, J);
-            if (pe >= 0) {  // a PEC face keeps its mirror flux
-              add_jump(JH[0], nv[1] * J[2] - nv[2] * J[1]);
-              add_jump(JH[1], nv[2] * J[0] - nv[0] * J[2]);
-              add_jump(JH[2], nv[0] * J[1] - nv[1] * J[0]);
-            }
+        if (EXT == 2 && (a.inc_elem || a.gr.elem)) {
+          double hm[3], em[3], hp[3], ep[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const float2 h = s_u2[c * N3P + pv], ev = s_u2[(c + 3) * N3P + pv];
+            hm[c] = f2d(h.x) + f2d(h.y);
+            em[c] = f2d(ev.x) + f2d(ev.y);
+            hp[c] = pe >= 0 ? s_nbv[c * NF + t] : 0.0;
+            ep[c] = pe >= 0 ? s_nbv[(EXT == 2 ? c + 3 : 0) * NF + t] : 0.0;
+          }
+          float2 jh[3], je[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            jh[c] = JH[c];
+            je[c] = JE[c];
+          }
+          face_extras<NF>(a, e, t, f, pe, hm, em, hp, ep, first_stage, jh, je);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            JH[c] = jh[c];
+            JE[c] = je[c];
           }
         }
         // coefficient pairs Y02, C02Y, Z02, C02Z (hi in the first float4 of
@@ -895,24 +962,25 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
     {
       const bool cubic = eg[0] == 1.0f && eg[1] == 0.0f && eg[2] == 1.0f && eg[3] == 0.0f;
       const float r1h = eg[0], r1l = eg[1], r2h = eg[2], r2l = eg[3];
-      line_phase<NX, 0, false, TPL>(s_u2, s_R2, s_F, cubic, 0.0f, 0.0f, a, e, first_stage);
+      line_phase<NX, 0, false, S>(s_u2, s_R2, s_F, cubic, 0.0f, 0.0f, a, e, first_stage, slab);
       __syncthreads();
-      line_phase<NX, 1, false, TPL>(s_u2, s_R2, s_F, cubic, r1h, r1l, a, e, first_stage);
+      line_phase<NX, 1, false, S>(s_u2, s_R2, s_F, cubic, r1h, r1l, a, e, first_stage, slab);
       __syncthreads();
       // without the extension terms each component can finish on its own
       // (MCfg::kFin): H3, E3 (no t-derivative) are complete since the s-lines
-      line_phase<NX, 2, FIN, TPL>(s_u2, s_R2, s_F, cubic, r2h, r2l, a, e, first_stage);
+      line_phase<NX, 2, FIN, S>(s_u2, s_R2, s_F, cubic, r2h, r2l, a, e, first_stage, slab);
     }
     if constexpr (FIN) {
       tid = opaque_tid();
       const int so = a.src_elem ? a.src_elem[e] : -1;
       constexpr int NPT2 = (2 * N3 + NT - 1) / NT;
+      const int nv = S == 1 ? N3 : N2 * (k1 - k0);
 #pragma unroll
       for (int q = 0; q < NPT2; ++q) {
-        const int w = tid + q * NT;
-        if (w < 2 * N3) {
-          const int c = w < N3 ? 2 : 5;
-          const int v = w < N3 ? w : w - N3;
+        const int w2 = tid + q * NT;
+        if (w2 < 2 * nv) {
+          const int c = w2 < nv ? 2 : 5;
+          const int v = (w2 < nv ? w2 : w2 - nv) + (S == 1 ? 0 : N2 * k0);
           const float2 rr = s_R2[c * N3P + pnode<NX>(v)];
           float Rh = rr.x, Rl = rr.y;
           if (c == 5 && so >= 0) add_pair_product(Rh, Rl, a.src_w[(long)so * N3 + v], a.src_ft2);
@@ -920,33 +988,34 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
         }
       }
       __syncthreads();  // the split pairs are consumed: the next element may land
-      if (C::kTma && tid == 0 && en < a.e_end) {
+      if (C::kTma && tid == 0 && wn < w1) {
         fence_proxy_async_smem();
         issue_tma(en, buf ^ 1);
       }
-      if (C::kAsync && en < a.e_end) issue_async(en, buf ^ 1, tid);
+      if (C::kAsync && wn < w1) issue_async(en, buf ^ 1, tid);
     } else {
       tid = opaque_tid();
       __syncthreads();
       // the split pairs are consumed: the next element's state lands in their
       // area while this one finishes (the next element's own barriers order
       // these reads of the residual pairs before its split overwrites them)
-      if (C::kTma && tid == 0 && en < a.e_end) {
+      if (C::kTma && tid == 0 && wn < w1) {
         fence_proxy_async_smem();
         issue_tma(en, buf ^ 1);
       }
-      if (C::kAsync && en < a.e_end) issue_async(en, buf ^ 1, tid);
+      if (C::kAsync && wn < w1) issue_async(en, buf ^ 1, tid);
       // ---- source, inverse mass, RK update ----------------------------------------
       // All six components of a node at once (the PML and dispersive terms
       // couple them to the node's auxiliary fields).
       const int so = a.src_elem ? a.src_elem[e] : -1;
-      const int pml_l = (EXT && a.pml.slot) ? a.pml.slot[e] : -1;
-      const int disp_l = (EXT && a.disp.slot) ? a.disp.slot[e] : -1;
+      const int pml_l = (EXT > 0 && a.pml.slot) ? a.pml.slot[e] : -1;
+      const int disp_l = (EXT > 0 && a.disp.slot) ? a.disp.slot[e] : -1;
+      const int v1 = S == 1 ? N3 : N2 * k1;
 #pragma unroll
       for (int q = 0; q < NPT; ++q) {
-        const int v = tid + q * NT;
-        if (v >= N3) continue;
-        if (C::kPfNode && q + 1 < NPT && v + NT < N3) {  // the next node's loads into L1 meanwhile
+        const int v = tid + q * NT + (S == 1 ? 0 : N2 * k0);
+        if (v >= v1) continue;
+        if (C::kPfNode && q + 1 < NPT && v + NT < v1) {  // the next node's loads into L1 meanwhile
           const long g2 = (long)e * N3 + v + NT;
 #pragma unroll
           for (int c = 0; c < 6; ++c) {
@@ -962,13 +1031,10 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, T
           Rh[c] = rr.x;
           Rl[c] = rr.y;
         }
-        if (EXT && pml_l >= 0) pml_node<N3>(a, pml_l, v, (long)e * N3 + v, first_stage, Rh, Rl);
-        if (EXT && disp_l >= 0) disp_node<N3>(a, disp_l, v, (long)e * N3 + v, first_stage, Rh, Rl);
+        if (EXT > 0 && pml_l >= 0) pml_node<N3>(a, pml_l, v, (long)e * N3 + v, first_stage, Rh, Rl);
+        if (EXT > 0 && disp_l >= 0) disp_node<N3>(a, disp_l, v, (long)e * N3 + v, first_stage, Rh, Rl);
         if (so >= 0) add_pair_product(Rh[5], Rl[5], a.src_w[(long)so * N3 + v], a.src_ft2);
-        // the node's two coefficient pairs, H and E, once for its six components
-        const long g = (long)e * N3 + v;
-        const float2 cfH = a.coef[g], cfE = a.coef[P + g];
-        rk_finish_node<C::kIntAdd>(a, g, Rh, Rl, cfH, cfE, first_stage);
+        rk_finish_node<C::kIntAdd>(a, (long)e * N3, v, Rh, Rl, first_stage);
       }
     }
   }
@@ -983,45 +1049,71 @@ __global__ void k_scale_coef_pairs(float2* coef, const double* base, long n2, do
   coef[i] = make_float2(d2f_hi(v), d2f_lo(v));
 }
 
-template <int NX, bool EXT, int TPL = 1>
+template <int NX, int EXT, int S>
 int launch_mixed(Context* c, const MixedDev& a, bool pdl) {
-  using C = MCfg<NX, TPL>;
-  auto kern = k_mixed_stage<NX, EXT, TPL>;
-  static bool ready = false;
+  using C = MCfg<NX>;
+  auto kern = k_mixed_stage<NX, EXT, S>;
   static int grid = 0;
-  if (!ready) {
+  if (!grid) {
     if (check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)C::smem)))
       return NEKGPU_ERR_CUDA;
-    int per_sm = 0, sms = 0;
+    int per_sm = 0;
     if (check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, C::smem)))
       return NEKGPU_ERR_CUDA;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     if (per_sm < 1) return NEKGPU_ERR_UNSUPPORTED;
-    grid = per_sm * sms;
-    ready = true;
+    grid = per_sm * num_sms(c);
   }
-  const int n = a.e_end - a.e_begin;
+  const int n = (a.e_end - a.e_begin) * S;
   if (n <= 0) return NEKGPU_OK;
   const int g = n < grid ? n : grid;
   c->fused_grid = g;
-  if (pdl) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(g);
-    cfg.blockDim = dim3(C::NT);
-    cfg.dynamicSmemBytes = C::smem;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (check_cuda(cudaLaunchKernelEx(&cfg, kern, a))) return NEKGPU_ERR_CUDA;
-  } else {
-    kern<<<g, C::NT, C::smem, c->stream>>>(a);
-  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g);
+  cfg.blockDim = dim3(C::NT);
+  cfg.dynamicSmemBytes = C::smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  if (check_cuda(cudaLaunchKernelEx(&cfg, kern, a))) return NEKGPU_ERR_CUDA;
   c->last_launches += 1;
   return check_cuda(cudaGetLastError());
+}
+
+// Slabs per element (k_mixed_stage): the most slabs the order has, else two,
+// while the tasks stay within what the SMs take side by side without slowing
+// each other -- one per SM at N=7 and 8, more for smaller elements.  us per
+// stage, unsplit / two / most slabs: 64 elements N=7 9.4 / 7.0 / 9.1 (four),
+// 27 elements N=7 9.4 / 6.8 / 6.5, N=8 13.1 / 11.7 / 9.6, 100 elements N=6
+// 11.7 / 12.2 / 11.4 (three), N=5 9.1 / 8.9 / 6.8, 180 elements N=5 9.9 / 9.8
+// / 10.1, 294 elements N=3 8.6 / 9.5.
+template <int NX, int EXT>
+int launch_mixed_split(Context* c, const MixedDev& a, bool pdl) {
+  constexpr int SM = EXT == 2 ? 1 : (NX >= 8 ? 4 : (NX >= 6 ? 3 : (NX >= 4 ? 2 : 1)));
+  constexpr int kPerSm = NX >= 8 ? 1 : (NX == 7 ? 2 : (NX == 3 ? 6 : 3));
+  const int n = a.e_end - a.e_begin, room = kPerSm * num_sms(c);
+  if constexpr (SM > 2)
+    if (n * SM <= room) return launch_mixed<NX, EXT, SM>(c, a, pdl);
+  if constexpr (SM > 1)
+    if (n * 2 <= room) return launch_mixed<NX, EXT, 2>(c, a, pdl);
+  return launch_mixed<NX, EXT, 1>(c, a, pdl);
+}
+
+template <int EXT>
+int dispatch_mixed(Context* c, const MixedDev& a, bool pdl) {
+  switch (c->nx) {
+    case 3: return launch_mixed_split<3, EXT>(c, a, pdl);
+    case 4: return launch_mixed_split<4, EXT>(c, a, pdl);
+    case 5: return launch_mixed_split<5, EXT>(c, a, pdl);
+    case 6: return launch_mixed_split<6, EXT>(c, a, pdl);
+    case 7: return launch_mixed_split<7, EXT>(c, a, pdl);
+    case 8: return launch_mixed_split<8, EXT>(c, a, pdl);
+    case 9: return launch_mixed_split<9, EXT>(c, a, pdl);
+    default: return NEKGPU_ERR_UNSUPPORTED;
+  }
 }
 
 // ===========================================================================
@@ -1440,29 +1532,13 @@ int mixed_stage_range(Context* c, int rkstep, double time, double dt, int e0, in
     const float hi = (float)ft;
     a.src_ft2 = make_float2(hi, (float)(ft - (double)hi));
   }
-  const bool ext = a.pml.slot || a.disp.slot || a.inc_elem || a.gr.elem;
   if (a.inc_elem && (st = incident_upload(c, time + dt * c->rk_c[rkstep - 1]))) return st;
   if (a.gr.elem) {
     a.gr.f_in = c->d_gr_f[c->gr_cur];
     a.gr.f_out = c->d_gr_f[c->gr_cur ^ 1];
   }
-  switch (c->nx) {
-    case 3: st = ext ? launch_mixed<3, true>(c, a, pdl) : launch_mixed<3, false>(c, a, pdl); break;
-    case 4: st = ext ? launch_mixed<4, true>(c, a, pdl) : launch_mixed<4, false>(c, a, pdl); break;
-    case 5: st = ext ? launch_mixed<5, true>(c, a, pdl) : launch_mixed<5, false>(c, a, pdl); break;
-    case 6: st = ext ? launch_mixed<6, true>(c, a, pdl) : launch_mixed<6, false>(c, a, pdl); break;
-    case 7: st = ext ? launch_mixed<7, true>(c, a, pdl) : launch_mixed<7, false>(c, a, pdl); break;
-    case 8:
-      // fewer elements than SMs: two threads per line (one element per SM
-      // either way; the element's latency is the stage's time)
-      st = ext ? launch_mixed<8, true>(c, a, pdl)
-               : (e1 - e0 <= num_sms(c) ? launch_mixed<8, false, 2>(c, a, pdl)
-                                         : launch_mixed<8, false>(c, a, pdl));
-      break;
-    case 9: st = ext ? launch_mixed<9, true>(c, a, pdl) : launch_mixed<9, false>(c, a, pdl); break;
-    default: return NEKGPU_ERR_UNSUPPORTED;
-  }
-  return st;
+  if (a.inc_elem || a.gr.elem) return dispatch_mixed<2>(c, a, pdl);
+  return a.pml.slot || a.disp.slot ? dispatch_mixed<1>(c, a, pdl) : dispatch_mixed<0>(c, a, pdl);
 }
 
 // One mixed stage on a curvilinear mesh (the curved form's arrays, the
@@ -1523,16 +1599,7 @@ int mixed_stage_dev(Context* c, MixedDev a, int rkstep, double time, double dt, 
     const float hi = (float)ft;
     a.src_ft2 = make_float2(hi, (float)(ft - (double)hi));
   }
-  switch (c->nx) {
-    case 3: return launch_mixed<3, false>(c, a, false);
-    case 4: return launch_mixed<4, false>(c, a, false);
-    case 5: return launch_mixed<5, false>(c, a, false);
-    case 6: return launch_mixed<6, false>(c, a, false);
-    case 7: return launch_mixed<7, false>(c, a, false);
-    case 8: return launch_mixed<8, false>(c, a, false);
-    case 9: return launch_mixed<9, false>(c, a, false);
-    default: return NEKGPU_ERR_UNSUPPORTED;
-  }
+  return dispatch_mixed<0>(c, a, false);
 }
 
 int mixed_stage(Context* c, int rkstep, double time, double dt) {
