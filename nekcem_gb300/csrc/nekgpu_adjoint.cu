@@ -21,25 +21,32 @@
 // projected out).  Every element gathers what lands on its own nodes, reading
 // the partner elements' face nodes, so all writes are element-local: no
 // atomics, and the adjoint state ping-pongs like the forward state.
-// The D^T contractions and the face terms run in double-float FP32
-// arithmetic (D w, the stage weights, the face-slot coefficients and the
-// jumps as (hi, lo) float pairs, products with their FMA error terms,
-// two-sum accumulation: ~2^-47 of the sum of the magnitudes, near FP64's
-// 2^-53) and join the FP64 arithmetic as one FP64 value each; the updates of
-// ub, w and deps are FP64.  The contractions and face terms were ~130 of the
-// ~166 FP64 operations per node.
+//
+// The kernel has the forward stage's form (nekgpu_fp64.cu): the weights w of
+// an element in shared memory, one thread per face node, then two phases of
+// line tasks (D^T w3 w in 64-bit integer arithmetic, nekgpu_fixed.cuh), both
+// adding to ub in shared memory, then node by node the updates of w and deps
+// in FP64.  The face terms (16 coefficients, the stage weights and the jumps)
+// run in double-float FP32 arithmetic: float pairs, products with their FMA
+// error terms, two-sum accumulation, ~2^-47 of the sum of the magnitudes, each
+// result joined into one FP64 value.
+//
+// What bounds it: the FP64 pipe (43 slots per node) and issue (2400
+// instructions per node, the face terms most of them).  With double-float
+// contractions per node and the face terms added per node by divergent warps
+// (~100 FP64 slots per node, 512 threads and one block per SM) the reverse
+// sweep of 100 steps of the 8^3-element N=7 box, the recomputation beside it,
+// took 45 ms; it takes 32 ms.
 #include <cuda_runtime.h>
 
 #include "nekgpu_internal.h"
+#include "nekgpu_lines.cuh"
 #include "nekgpu_pair.cuh"
 
 namespace nekgpu {
 
 namespace {
 
-__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
-__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
-__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
 // tangential axes in cyclic order: (e_a x x)_t1 = -x_t2, (e_a x x)_t2 = x_t1
 __host__ __device__ constexpr int tan1(int a) { return a == 0 ? 1 : (a == 1 ? 2 : 0); }
 __host__ __device__ constexpr int tan2(int a) { return a == 0 ? 2 : (a == 1 ? 0 : 1); }
@@ -70,90 +77,88 @@ __device__ __forceinline__ double pdbl(P2 a) {
 }
 
 template <int NX>
-__device__ __forceinline__ int face_vol(int f, int a, int b) {
-  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
-  const int ax = slot_axis(f);
-  return ax == 0 ? fixed + NX * a + NX * NX * b
-                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
+struct ACfg : ElemCfg<NX> {
+  using E = ElemCfg<NX>;
+  // weights w; ub, completed in place; products of two GLL weights: 56 KB at
+  // N=7, four blocks per SM
+  static constexpr size_t off_R = 6 * (size_t)E::N3P * 8, off_w = 2 * off_R;
+  static constexpr size_t smem = off_w + (size_t)E::N2 * 8;
+};
+
+// Phase PH of the transposed curl: every line adds its outputs, times the
+// line's factor metric * w * w, to ub.
+template <int NX, int PH>
+__device__ __forceinline__ void adjoint_lines(const double* s_w, double* s_R, const double* s_ww,
+                                              const double* eg, const AdjointDev& a) {
+  using C = ElemCfg<NX>;
+  constexpr int N2 = C::N2;
+#pragma unroll 1
+  for (int task = threadIdx.x; task < 6 * N2; task += C::NT) {
+    const int type = task / N2, lam = task - type * N2;
+    const LineType& lt = kLine[PH][type];
+    const int dir = lt.dir, la = lam % NX, lb = lam / NX;
+    const int base = dir == 0 ? C::RS * la + C::SZ * lb : (dir == 1 ? la + C::SZ * lb : la + C::RS * lb);
+    const int step = dir == 0 ? 1 : (dir == 1 ? C::RS : C::SZ);
+    const double rho = flip(eg[dir] * s_ww[lam], lt.neg != 0);
+    double* R = s_R + lt.res * C::N3P + base;
+    line_outputs<NX, false>(s_w + lt.comp * C::N3P + base, step, 0, NX, a.fd, a.Dw, nullptr,
+                            [&](int i, double x) { R[step * i] = fma(rho, x, R[step * i]); });
+  }
 }
 
 template <int NX>
-struct ACfg {
-  static constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
-  static constexpr int NT = ((N3 + 31) / 32) * 32;
-  static constexpr int FPT = (NF + NT - 1) / NT;
-  // shared: face results (5*NF) in FP64; the stage weights w and D w as
-  // float pairs (6*N3 + NX*NX)
-  static constexpr size_t smem = 5 * NF * sizeof(double) + (6 * N3 + NX * NX) * sizeof(float2);
-};
+constexpr int adjoint_min_blocks() {
+  return NX == 9 ? 2 : 4;
+}
 
 template <int NX>
-__global__ void __launch_bounds__(ACfg<NX>::NT) k_adjoint_stage(const AdjointDev a) {
+__global__ void __launch_bounds__(ACfg<NX>::NT, adjoint_min_blocks<NX>())
+    k_adjoint_stage(const __grid_constant__ AdjointDev a) {
   using C = ACfg<NX>;
-  constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF, FPT = C::FPT;
-  extern __shared__ double sm[];
-  double* s_fu = sm;                // [4][NF]  tangential face contributions to ub
-  double* s_fe = s_fu + 4 * NF;     // [NF]     face contributions to deps
-  float2* s_wp = reinterpret_cast<float2*>(s_fe + NF);  // [6][N3] w as (hi, lo)
-  float2* s_Dp = s_wp + 6 * N3;                          // D w as (hi, lo)
+  constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF, N3P = C::N3P;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* s_w = reinterpret_cast<double*>(smem);
+  double* s_R = reinterpret_cast<double*>(smem + C::off_R);
+  double* s_ww = reinterpret_cast<double*>(smem + C::off_w);
   const int tid = threadIdx.x;
   const long P = a.npts, PF = (long)a.nelt * NF;
-  const bool node = tid < N3;
-  const int vi = tid % NX, vj = (tid / NX) % NX, vk = tid / N2;
-  for (int t = tid; t < NX * NX; t += NT) {
-    s_Dp[t] = make_float2(d2f_hi(a.Dw[t]), d2f_lo(a.Dw[t]));
-  }
-  const double wi = a.w[vi], wj = a.w[vj], wk = a.w[vk];
+  for (int t = tid; t < N2; t += NT) s_ww[t] = a.w[t % NX] * a.w[t / NX];
+  const float2* kslot = reinterpret_cast<const float2*>(a.slot);
 
   for (int e = blockIdx.x; e < a.nelt; e += gridDim.x) {
-    const long g = (long)e * N3 + tid;
-    double ub[6], wn[6], mass = 0.0;
-    __syncthreads();  // s_wp / s_fu of the previous element are consumed
-    if (node) {
+    const long ge = (long)e * N3;
+    for (int v = tid; v < N3; v += NT) {
+      const int pv = pnode<NX>(v);
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        ub[c] = a.ub_in[c * P + g];
-        wn[c] = a.w_in[c * P + g];
-        s_wp[c * N3 + tid] = make_float2(d2f_hi(wn[c]), d2f_lo(wn[c]));
+        cp_async8(s_w + c * N3P + pv, a.w_in + c * P + ge + v);
+        cp_async8(s_R + c * N3P + pv, a.ub_in + c * P + ge + v);
       }
-#pragma unroll
-      for (int c = 3; c < 6; ++c) {
-        const double r = a.a == 0.0 ? a.k_cur[c * P + g]
-                                    : fma(-a.a, a.k_prev[c * P + g], a.k_cur[c * P + g]);
-        mass = fma(wn[c], r, mass);
-      }
-      mass *= -a.bm1[g] * a.inv_dt;
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // ---- face slots: transposed flux and impedance derivatives --------------
+    // (the face node's share of deps; its terms of the component that waits)
+    double fe[C::FPT], later[C::FPT][2];
 #pragma unroll
-    for (int q = 0; q < FPT; ++q) {
+    for (int q = 0; q < C::FPT; ++q) {
       const int t = tid + q * NT;
+      fe[q] = 0.0;
       if (t >= NF) continue;
       const int f = t / N2, ab = t - f * N2, fa = ab % NX, fb = ab / NX;
       const int ax = slot_axis(f), t1 = tan1(ax), t2 = tan2(ax);
-      const int vl = face_vol<NX>(f, fa, fb);
-      const long gn = (long)e * N3 + vl;
-      const long j = (long)e * NF + t;
-      // the slot's coefficients, the stage weights and the jumps as float
-      // pairs; sums of products in double-float arithmetic (as the D^T
-      // contractions), each result joined into one FP64 value
-      const float2* kslot = reinterpret_cast<const float2*>(a.slot);
-      P2 k[16];
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const float2 kv = kslot[m * PF + j];
-        k[m] = P2{kv.x, kv.y};
-      }
-      // own stage weights (tangential) from shared memory
-      const P2 nH1 = p2(s_wp[t1 * N3 + vl]), nH2 = p2(s_wp[t2 * N3 + vl]);
-      const P2 nE1 = p2(s_wp[(3 + t1) * N3 + vl]), nE2 = p2(s_wp[(3 + t2) * N3 + vl]);
-      P2 pH1{0.0f, 0.0f}, pH2{0.0f, 0.0f}, pE1{0.0f, 0.0f}, pE2{0.0f, 0.0f};
-      // jump u+ - u- of u_{i-1} (PEC: u-, the -2 of the mirror is in the coefficients)
-      const double oH1 = a.u_prev[t1 * P + gn], oH2 = a.u_prev[t2 * P + gn];
-      const double oE1 = a.u_prev[(3 + t1) * P + gn], oE2 = a.u_prev[(3 + t2) * P + gn];
-      P2 dH1 = p2(oH1), dH2 = p2(oH2), dE1 = p2(oE1), dE2 = p2(oE2);
+      const int vl = face_vol<NX>(f, fa, fb), pv = pnode<NX>(vl);
+      const long gn = ge + vl, j = (long)e * NF + t;
       const int pe = a.nbr[6 * e + f];
+      auto k = [&](int m) { return p2(kslot[m * PF + j]); };
+      // own stage weights, and the jump u+ - u- of u_{i-1} (PEC: u-, the -2 of
+      // the mirror is in the coefficients), tangential components
+      const P2 nH1 = p2(s_w[t1 * N3P + pv]), nH2 = p2(s_w[t2 * N3P + pv]);
+      const P2 nE1 = p2(s_w[(3 + t1) * N3P + pv]), nE2 = p2(s_w[(3 + t2) * N3P + pv]);
+      P2 pH1{0.0f, 0.0f}, pH2{0.0f, 0.0f}, pE1{0.0f, 0.0f}, pE2{0.0f, 0.0f};
+      P2 dH1 = p2(a.u_prev[t1 * P + gn]), dH2 = p2(a.u_prev[t2 * P + gn]);
+      P2 dE1 = p2(a.u_prev[(3 + t1) * P + gn]), dE2 = p2(a.u_prev[(3 + t2) * P + gn]);
       if (pe >= 0) {
         const long gp = (long)pe * N3 + face_vol<NX>(slot_opp(f), fa, fb);
         pH1 = p2(a.w_in[t1 * P + gp]);
@@ -165,97 +170,133 @@ __global__ void __launch_bounds__(ACfg<NX>::NT) k_adjoint_stage(const AdjointDev
         dE1 = padd(p2(a.u_prev[(3 + t1) * P + gp]), pneg(dE1));
         dE2 = padd(p2(a.u_prev[(3 + t2) * P + gp]), pneg(dE2));
       }
+      // Each component takes terms from the faces of its two tangential axes:
+      // from those of the axis after it (it is their t2) now, from the other
+      // axis' (their t1) after a barrier, so no two threads meet at a node.
+      double* R = s_R + t2 * N3P + pv;
       // k: 0 kH 1 kHx 2 kE 3 kEx | 4 pH 5 pHx 6 pE 7 pEx | 8..11 gA..gD | 12..15 hA..hD
-      s_fu[0 * NF + t] = pdbl(padd(padd(pmul(k[0], nH1), pneg(pmul(k[1], nE2))),
-                                   padd(pmul(k[4], pH1), pneg(pmul(k[5], pE2)))));
-      s_fu[1 * NF + t] = pdbl(padd(padd(pmul(k[0], nH2), pmul(k[1], nE1)),
-                                   padd(pmul(k[4], pH2), pmul(k[5], pE1))));
-      s_fu[2 * NF + t] = pdbl(padd(padd(pneg(pmul(k[3], nH2)), pmul(k[2], nE1)),
-                                   padd(pneg(pmul(k[7], pH2)), pmul(k[6], pE1))));
-      s_fu[3 * NF + t] = pdbl(padd(padd(pmul(k[3], nH1), pmul(k[2], nE2)),
-                                   padd(pmul(k[7], pH1), pmul(k[6], pE2))));
-      // fe = A.PdH + B.(e_a x dE) + C.(e_a x dH) + D.PdE with A = gA wH(n) + hA wH(p) ...
-      const P2 A1 = padd(pmul(k[8], nH1), pmul(k[12], pH1)), A2 = padd(pmul(k[8], nH2), pmul(k[12], pH2));
-      const P2 B1 = padd(pmul(k[9], nH1), pmul(k[13], pH1)), B2 = padd(pmul(k[9], nH2), pmul(k[13], pH2));
-      const P2 C1 = padd(pmul(k[10], nE1), pmul(k[14], pE1)), C2 = padd(pmul(k[10], nE2), pmul(k[14], pE2));
-      const P2 D1 = padd(pmul(k[11], nE1), pmul(k[15], pE1)), D2 = padd(pmul(k[11], nE2), pmul(k[15], pE2));
-      P2 fe = pmul(A1, dH1);
-      fe = padd(fe, pmul(A2, dH2));
-      fe = padd(fe, pneg(pmul(B1, dE2)));
-      fe = padd(fe, pmul(B2, dE1));
-      fe = padd(fe, pneg(pmul(C1, dH2)));
-      fe = padd(fe, pmul(C2, dH1));
-      fe = padd(fe, pmul(D1, dE1));
-      fe = padd(fe, pmul(D2, dE2));
-      s_fe[t] = pdbl(fe);
-    }
-    __syncthreads();
-    if (!node) continue;
-    // ---- transposed weighted curl: D^T contractions of w3 w ------------------
-    const double* eg = a.egeom + 9 * e;
-    const double Rr = eg[0] * wj * wk, Ss = eg[1] * wi * wk, Tt = eg[2] * wi * wj;
-    // sum_m D(m,row) w_m z_m over one line of the stage weights, double-float
-    auto dot = [&](const float2* z, int zs, int row) -> double {
-      float S = 0.0f, E = 0.0f;
-#pragma unroll
-      for (int m = 0; m < NX; ++m) {
-        const float2 d = s_Dp[m + NX * row];
-        const float2 x = z[zs * m];
-        const float p = d.x * x.x;
-        float e = fmaf(d.x, x.x, -p);
-        e = fmaf(d.x, x.y, e);
-        e = fmaf(d.y, x.x, e);
-        float s, t;
-        two_sum(S, p, s, t);
-        S = s;
-        E += e + t;
+      {
+        const P2 kH = k(0), kHx = k(1), qH = k(4), qHx = k(5);
+        later[q][0] = pdbl(padd(padd(pmul(kH, nH1), pneg(pmul(kHx, nE2))),
+                                padd(pmul(qH, pH1), pneg(pmul(qHx, pE2)))));
+        R[0] += pdbl(padd(padd(pmul(kH, nH2), pmul(kHx, nE1)),
+                          padd(pmul(qH, pH2), pmul(qHx, pE1))));
       }
-      float s, t;
-      two_sum(S, E, s, t);
-      return pair_to_double(s, t);
-    };
-    auto dtr = [&](int c) { return dot(s_wp + c * N3 + NX * vj + N2 * vk, 1, vi); };
-    auto dts = [&](int c) { return dot(s_wp + c * N3 + vi + N2 * vk, NX, vj); };
-    auto dtt = [&](int c) { return dot(s_wp + c * N3 + vi + NX * vj, N2, vk); };
-    double out[6];
-    out[0] = fma(Tt, dtt(4), fma(-Ss, dts(5), ub[0]));
-    out[1] = fma(Rr, dtr(5), fma(-Tt, dtt(3), ub[1]));
-    out[2] = fma(Ss, dts(3), fma(-Rr, dtr(4), ub[2]));
-    out[3] = fma(Ss, dts(2), fma(-Tt, dtt(1), ub[3]));
-    out[4] = fma(Tt, dtt(0), fma(-Rr, dtr(2), ub[4]));
-    out[5] = fma(Rr, dtr(1), fma(-Ss, dts(0), ub[5]));
-    // ---- face contributions, in face-slot order ------------------------------
-    double fe = 0.0;
-    auto add = [&](int f, int ab) {
-      const int t = f * N2 + ab, ax = slot_axis(f);
-      out[tan1(ax)] += s_fu[0 * NF + t];
-      out[tan2(ax)] += s_fu[1 * NF + t];
-      out[3 + tan1(ax)] += s_fu[2 * NF + t];
-      out[3 + tan2(ax)] += s_fu[3 * NF + t];
-      fe += s_fe[t];
-    };
-    if (vj == 0) add(0, vi + NX * vk);
-    if (vi == NX - 1) add(1, vj + NX * vk);
-    if (vj == NX - 1) add(2, vi + NX * vk);
-    if (vi == 0) add(3, vj + NX * vk);
-    if (vk == 0) add(4, vi + NX * vj);
-    if (vk == NX - 1) add(5, vi + NX * vj);
-    const double cH = a.bdt_next * a.hbm1[g], cE = a.bdt_next * a.ebm1[g];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      a.ub_out[c * P + g] = out[c];
-      a.w_out[c * P + g] = fma(a.a, wn[c], (c < 3 ? cH : cE) * out[c]);
+      {
+        const P2 kE = k(2), kEx = k(3), qE = k(6), qEx = k(7);
+        later[q][1] = pdbl(padd(padd(pneg(pmul(kEx, nH2)), pmul(kE, nE1)),
+                                padd(pneg(pmul(qEx, pH2)), pmul(qE, pE1))));
+        R[3 * N3P] += pdbl(padd(padd(pmul(kEx, nH1), pmul(kE, nE2)),
+                                padd(pmul(qEx, pH1), pmul(qE, pE2))));
+      }
+      // fe = A.PdH + B.(e_a x dE) + C.(e_a x dH) + D.PdE with A = gA wH(n) + hA wH(p) ...
+      P2 F;
+      {
+        const P2 g = k(8), h = k(12);
+        F = pmul(padd(pmul(g, nH1), pmul(h, pH1)), dH1);
+        F = padd(F, pmul(padd(pmul(g, nH2), pmul(h, pH2)), dH2));
+      }
+      {
+        const P2 g = k(9), h = k(13);
+        F = padd(F, pneg(pmul(padd(pmul(g, nH1), pmul(h, pH1)), dE2)));
+        F = padd(F, pmul(padd(pmul(g, nH2), pmul(h, pH2)), dE1));
+      }
+      {
+        const P2 g = k(10), h = k(14);
+        F = padd(F, pneg(pmul(padd(pmul(g, nE1), pmul(h, pE1)), dH2)));
+        F = padd(F, pmul(padd(pmul(g, nE2), pmul(h, pE2)), dH1));
+      }
+      {
+        const P2 g = k(11), h = k(15);
+        F = padd(F, pmul(padd(pmul(g, nE1), pmul(h, pE1)), dE1));
+        F = padd(F, pmul(padd(pmul(g, nE2), pmul(h, pE2)), dE2));
+      }
+      fe[q] = pdbl(F);
     }
-    a.deps[g] += mass + fe;
+    // after the barrier the other component, and the faces' deps one axis after
+    // the other beside the phases (an axis' two faces share no node)
+    auto each_face = [&](auto fn) {
+#pragma unroll
+      for (int q = 0; q < C::FPT; ++q) {
+        const int t = tid + q * NT, f = t / N2;
+        if (t < NF) fn(q, slot_axis(f), face_vol<NX>(f, (t - f * N2) % NX, (t - f * N2) / NX));
+      }
+    };
+    auto face_deps = [&](int axis) {
+      each_face([&](int q, int ax, int vl) {
+        if (ax == axis) a.deps[ge + vl] += fe[q];
+      });
+    };
+    const double* eg = a.egeom + 9 * (long)e;
+    face_deps(0);
+    __syncthreads();
+    each_face([&](int q, int ax, int vl) {
+      double* R = s_R + tan1(ax) * N3P + pnode<NX>(vl);
+      R[0] += later[q][0];
+      R[3 * N3P] += later[q][1];
+    });
+    face_deps(1);
+    __syncthreads();
+    face_deps(2);
+    adjoint_lines<NX, 0>(s_w, s_R, s_ww, eg, a);
+    __syncthreads();
+    adjoint_lines<NX, 1>(s_w, s_R, s_ww, eg, a);
+    __syncthreads();
+    // ---- updates of ub, w and deps, node by node --------------------------------
+#pragma unroll 1
+    for (int v = tid; v < N3; v += NT) {
+      const int pv = pnode<NX>(v);
+      const long g = ge + v;
+      double kc[3], kp[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        kc[c] = a.k_cur[(3 + c) * P + g];
+        kp[c] = a.a == 0.0 ? 0.0 : a.k_prev[(3 + c) * P + g];
+      }
+      const double cH = a.bdt_next * a.hbm1[g], cE = a.bdt_next * a.ebm1[g];
+      const double bm = -a.bm1[g] * a.inv_dt, d0 = a.deps[g];
+      double mass = 0.0;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        const double wn = s_w[c * N3P + pv], out = s_R[c * N3P + pv];
+        if (c >= 3) mass = fma(wn, a.a == 0.0 ? kc[c - 3] : fma(-a.a, kp[c - 3], kc[c - 3]), mass);
+        a.ub_out[c * P + g] = out;
+        a.w_out[c * P + g] = fma(a.a, wn, (c < 3 ? cH : cE) * out);
+      }
+      a.deps[g] = fma(mass, bm, d0);
+    }
+    __syncthreads();  // the element's shared data is consumed
   }
 }
 
-__global__ void k_adjoint_seed(double* w, const double* ub, const double* hbm1, const double* ebm1,
-                               long P, double bdt) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= 6 * P) return;
-  const long g = i % P;
-  w[i] = bdt * (i < 3 * P ? hbm1[g] : ebm1[g]) * ub[i];
+// J = sum jw |E|^2 (one partial sum per block, kSeedBlocks of them), and the
+// seed ub = (0, 2 jw E), w = bdt * (hbm1 | ebm1) * ub
+constexpr int kSeedThreads = 256;
+__global__ void __launch_bounds__(kSeedThreads)
+    k_adjoint_seed(double* w, double* ub, const double* u, const double* jw, const double* ebm1, long P,
+                   double bdt, double* partial) {
+  __shared__ double s_sum[kSeedThreads];
+  double sum = 0.0;
+  for (long g = blockIdx.x * (long)kSeedThreads + threadIdx.x; g < P; g += (long)gridDim.x * kSeedThreads) {
+    const double j = jw[g], ce = bdt * ebm1[g];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double e = u[(3 + c) * P + g];
+      sum = fma(j * e, e, sum);
+      const double b = 2.0 * j * e;
+      ub[c * P + g] = 0.0;
+      w[c * P + g] = 0.0;
+      ub[(3 + c) * P + g] = b;
+      w[(3 + c) * P + g] = ce * b;
+    }
+  }
+  s_sum[threadIdx.x] = sum;
+  __syncthreads();
+  for (int h = kSeedThreads / 2; h > 0; h /= 2) {
+    if ((int)threadIdx.x < h) s_sum[threadIdx.x] += s_sum[threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) partial[blockIdx.x] = s_sum[0];
 }
 
 template <int NX>
@@ -297,10 +338,10 @@ int adjoint_stage(Context* c, const AdjointDev& a) {
   }
 }
 
-int adjoint_seed(Context* c, double* w, const double* ub, double bdt) {
-  const long n = 6 * c->npts;
-  k_adjoint_seed<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(w, ub, c->d_hbm1, c->d_ebm1,
-                                                                     c->npts, bdt);
+int adjoint_seed(Context* c, double* w, double* ub, const double* u, const double* jw, double bdt,
+                 double* partial) {
+  k_adjoint_seed<<<kSeedBlocks, kSeedThreads, 0, c->stream>>>(w, ub, u, jw, c->d_ebm1, c->npts, bdt,
+                                                              partial);
   c->last_launches += 1;
   return check_cuda(cudaGetLastError());
 }

@@ -40,20 +40,36 @@ int face_vol(int f, int a, int b, int n) {
   }
 }
 
-// Temporary device buffers of one call; freed on every exit path.
+// Temporary device buffers of one call; freed on every exit path.  reserve()
+// takes the call's whole plan in one allocation that get() hands out: a
+// gradient of 100 steps needs ~220 buffers, and 220 pairs of cudaMalloc and
+// cudaFree took 14 ms of its 80 (8^3 elements, N=7).
 struct Scratch {
   std::vector<void*> ptrs;
+  char* arena = nullptr;
+  size_t cap = 0, used = 0;
+  static size_t round(size_t bytes) { return (bytes + 255) / 256 * 256; }
   ~Scratch() {
     for (void* p : ptrs) cudaFree(p);
   }
-  double* get(size_t count) {
+  double* alloc(size_t bytes) {
     void* p = nullptr;
-    if (cudaMalloc(&p, count * sizeof(double)) != cudaSuccess) {
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
     ptrs.push_back(p);
     return (double*)p;
+  }
+  // (without room for it in one piece, get() allocates one by one)
+  void reserve(size_t bytes) {
+    if ((arena = (char*)alloc(bytes))) cap = bytes;
+  }
+  double* get(size_t count) {
+    const size_t bytes = round(count * sizeof(double));
+    if (used + bytes > cap) return alloc(count * sizeof(double));
+    used += bytes;
+    return (double*)(arena + used - bytes);
   }
 };
 
@@ -298,32 +314,29 @@ struct Sweep {
   AdjointDev a{};
   double J = 0.0;
   bool seeded = false;
-  std::vector<double> final_host;  // u(T), read back by the seed
+  bool keep_final = false;         // binomial schedule: its stages overwrite u(T) ...
+  std::vector<double> final_host;  // ... so the seed keeps a copy
 
-  // J and the adjoint seed from the final state: ub = (0, 2 jw E), w = b_5 dt M^-1 ub
+  // J and the adjoint seed from the final state (jw passes through deps)
   int seed(const double* u_final) {
     const long npts = c->npts, ns = 6 * npts;
-    std::vector<double>& uf = final_host;
-    std::vector<double> ubf(ns, 0.0);
-    uf.resize(ns);
-    if (check_cuda(cudaMemcpyAsync(uf.data(), u_final, ns * 8, cudaMemcpyDeviceToHost, c->stream)) ||
-        check_cuda(cudaStreamSynchronize(c->stream)))
+    double part[kSeedBlocks];
+    if (keep_final) final_host.resize(ns);
+    int st;
+    if (check_cuda(cudaMemcpyAsync(deps, jw, npts * 8, cudaMemcpyHostToDevice, c->stream)))
       return NEKGPU_ERR_CUDA;
-    double Jv = 0.0;
-    for (int q = 3; q < 6; ++q)
-      for (long g = 0; g < npts; ++g) {
-        const double e = uf[q * npts + g];
-        Jv += jw[g] * e * e;
-        ubf[q * npts + g] = 2.0 * jw[g] * e;
-      }
-    J = Jv;
-    if (check_cuda(cudaMemcpyAsync(ub[0], ubf.data(), ns * 8, cudaMemcpyHostToDevice, c->stream)) ||
+    if ((st = adjoint_seed(c, wb[0], ub[0], u_final, deps, c->rk_b[4] * dt, c->d_red))) return st;
+    if (check_cuda(cudaMemcpyAsync(part, c->d_red, sizeof(part), cudaMemcpyDeviceToHost, c->stream)) ||
+        (keep_final && check_cuda(cudaMemcpyAsync(final_host.data(), u_final, ns * 8,
+                                                  cudaMemcpyDeviceToHost, c->stream))) ||
         check_cuda(cudaMemsetAsync(deps, 0, npts * 8, c->stream)) ||
         check_cuda(cudaStreamSynchronize(c->stream)))
       return NEKGPU_ERR_CUDA;
+    J = 0.0;
+    for (double p : part) J += p;
     cu = 0;
     seeded = true;
-    return adjoint_seed(c, wb[0], ub[0], c->rk_b[4] * dt);
+    return NEKGPU_OK;
   }
 
   // the five reverse stages of step j from its stage states (U[0..4]) and
@@ -360,8 +373,9 @@ struct Sweep {
     const int n = c->nx;
     for (int i = 0; i < n; ++i) {
       a.w[i] = c->fargs.w[i];
-      for (int m = 0; m < n; ++m) a.Dw[m + n * i] = c->fargs.D[m + n * i] * c->fargs.w[m];
+      for (int m = 0; m < n; ++m) a.Dw[i + n * m] = c->fargs.D[m + n * i] * c->fargs.w[m];
     }
+    fixed_table(a.Dw, n, a.fd);
   }
 };
 
@@ -498,6 +512,10 @@ extern "C" int nekgpu_adjoint_gradient(nekgpu_ctx* c, int nsteps, double t0, dou
       t = t + dt;
     }
   }
+  {
+    const double states = nsets ? sqrt_states(nsets) : 15.0 + ndev;
+    mem.reserve((size_t)states * Scratch::round(ns * 8) + Scratch::round(npts * 8));
+  }
   w.ub[0] = mem.get(ns);
   w.ub[1] = mem.get(ns);
   w.wb[0] = mem.get(ns);
@@ -511,6 +529,7 @@ extern "C" int nekgpu_adjoint_gradient(nekgpu_ctx* c, int nsteps, double t0, dou
   if (nsets == 0) {
     // ---- binomial schedule -------------------------------------------------------
     Binomial bs{w};
+    w.keep_final = true;
     for (int r = 1; r <= 5; ++r)
       if (!(bs.SU[r] = mem.get(ns)) || !(bs.SK[r] = mem.get(ns))) return NEKGPU_ERR_NOMEM;
     bs.SK[0] = bs.SK[5];

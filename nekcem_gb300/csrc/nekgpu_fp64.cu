@@ -31,73 +31,21 @@
 #include <algorithm>
 #include <cmath>
 
-#include "nekgpu_fixed.cuh"
 #include "nekgpu_internal.h"
+#include "nekgpu_lines.cuh"
 
 namespace nekgpu {
 
 namespace {
 
-__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
-__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
-__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
-constexpr int cmax(int a, int b) { return a > b ? a : b; }
-constexpr int round32(int a) { return (a + 31) / 32 * 32; }
-
 template <int NX>
-__device__ __forceinline__ int face_vol(int f, int a, int b) {
-  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
-  const int ax = slot_axis(f);
-  return ax == 0 ? fixed + NX * a + NX * NX * b
-                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
-}
-
-// x with its sign flipped where neg (no FP64 instruction)
-__device__ __forceinline__ double flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
-}
-
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-
-template <int NX>
-struct DCfg {
-  static constexpr int N2 = NX * NX, N3 = N2 * NX, NF = 6 * N2;
-  // node (i,j,k) of the element arrays at i + RS*j + SZ*k, an odd row length:
-  // lines in every direction are read with at most two threads of a half warp
-  // on a bank
-  static constexpr int RS = NX | 1, SZ = RS * NX, N3P = NX * SZ;
-  static constexpr int NT = NX == 9 ? 384 : (NX == 8 ? 256 : round32(cmax(3 * N2, (N3 + 1) / 2)));
-  static constexpr int FPT = (NF + NT - 1) / NT;
+struct DCfg : ElemCfg<NX> {
+  using E = ElemCfg<NX>;
   // state, residual, flux [face][line slot][N2], D rows (split form)
-  static constexpr size_t off_R = 6 * (size_t)N3P * 8, off_F = 2 * off_R;
-  static constexpr size_t off_D = (off_F + 24 * (size_t)N2 * 8 + 15) / 16 * 16;
-  static constexpr size_t smem(bool split) { return off_D + (split ? N2 * 16 : 0); }
+  static constexpr size_t off_R = 6 * (size_t)E::N3P * 8, off_F = 2 * off_R;
+  static constexpr size_t off_D = (off_F + 24 * (size_t)E::N2 * 8 + 15) / 16 * 16;
+  static constexpr size_t smem(bool split) { return off_D + (split ? E::N2 * 16 : 0); }
 };
-
-// The line types of the two contraction phases: the first starts each of the
-// six residual components, the second completes it, so a phase has six
-// component-lines per line and one barrier ends it.  Residual index 0..2 =
-// H1..H3 (-curl E), 3..5 = E1..E3 (curl H); field 0..2 = H, 3..5 = E:
-//   E1 = ds Hz - dt Hy   E2 = dt Hx - dr Hz   E3 = dr Hy - ds Hx
-//   H1 = dt Ey - ds Ez   H2 = dr Ez - dt Ex   H3 = ds Ex - dr Ey
-// slot: the type's place among the four flux components of a face normal to
-// its direction.
-struct LineType {
-  int dir, comp, res, neg, slot;
-};
-__constant__ const LineType kLine[2][6] = {
-    {{0, 1, 5, 0, 0}, {0, 2, 4, 1, 1}, {0, 4, 2, 1, 2}, {0, 5, 1, 0, 3}, {1, 2, 3, 0, 1}, {1, 5, 0, 1, 3}},
-    {{1, 0, 5, 1, 0}, {1, 3, 2, 0, 2}, {2, 0, 4, 0, 0}, {2, 1, 3, 1, 1}, {2, 3, 1, 1, 2}, {2, 4, 0, 0, 3}}};
-
-template <int NX>
-__device__ __forceinline__ int pnode(int v) {  // stored index of node v = i + NX*j + NX^2*k
-  return (v % NX) + DCfg<NX>::RS * ((v / NX) % NX) + DCfg<NX>::SZ * (v / (NX * NX));
-}
 
 // Field component of the k-th partner value of face f: all six with the
 // face terms (EXT 2), else H and E along the two axes tangential to f.
@@ -184,45 +132,10 @@ __device__ __forceinline__ void line_task(int type, int lam, int i0, int i1, con
   // faces 3|1 (r), 0|2 (s), 4|5 (t)
   const double* Fm = s_F + ((dir == 0 ? 3 : (dir == 1 ? 0 : 4)) * 4 + lt.slot) * N2 + lam;
   const double* Fp = s_F + ((dir == 0 ? 1 : (dir == 1 ? 2 : 5)) * 4 + lt.slot) * N2 + lam;
-  FixedLine<NX> f;
-  {
-    double u[NX];
-#pragma unroll
-    for (int l = 0; l < NX; ++l) u[l] = pu[step * l];
-    fixed_line<NX>(u, f);
-  }
-  auto put = [&](int i, double x) {
+  line_outputs<NX, SPLIT>(pu, step, i0, i1, a.fd, a.D, s_D, [&](int i, double x) {
     const bool end = i == 0 || i == NX - 1;
     line_put<OP>(R + step * i, x, neg, rho, end, end ? (i == 0 ? *Fm : *Fp) : 0.0);
-  };
-  if (a.fd.ok && !f.special) {
-    if (!SPLIT) {
-#pragma unroll
-      for (int i = 0; i < NX; ++i)
-        put(i, fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
-              hi = a.fd.hi[i + NX * l];
-              lo = a.fd.lo[i + NX * l];
-              hi8 = a.fd.hi8[i + NX * l];
-            }));
-    } else {
-#pragma unroll 1
-      for (int i = i0; i < i1; ++i)
-        put(i, fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
-              const int4 d = s_D[i + NX * l];
-              hi = d.x;
-              lo = d.y;
-              hi8 = d.z;
-            }));
-    }
-  } else {  // a line out of the integer form's range: in FP64
-#pragma unroll 1
-    for (int i = i0; i < i1; ++i) {
-      double x = a.D[i] * pu[0];
-#pragma unroll 1
-      for (int l = 1; l < NX; ++l) x = fma(a.D[i + NX * l], pu[step * l], x);
-      put(i, x);
-    }
-  }
+  });
 }
 
 // Phase PH of the contractions over the slab: tasks (line type, line), in the

@@ -328,7 +328,8 @@ struct AdjointDev {
   const double* egeom;
   const double* slot;    // [16][nxzfl] static face-slot coefficients as (hi, lo) float pairs
   double a, bdt_next, inv_dt;  // bdt_next = b_{i-1} dt
-  double Dw[kMaxNx * kMaxNx];  // D(m,i) w_m at [m + NX*i]
+  double Dw[kMaxFixed * kMaxFixed];  // D(m,i) w_m at [i + NX*m], and in fixed point
+  FixedD fd;
   double w[kMaxNx];
 };
 
@@ -599,9 +600,12 @@ int stage2d(Context* c, int rkstep, double time, double dt);
 
 // nekgpu_adjoint.cu
 int adjoint_stage(Context* c, const AdjointDev& a);
-// w = bdt * (hbm1 | ebm1) * ub (the stage weights of the last stage of the
-// last step; bdt = b_5 dt)
-int adjoint_seed(Context* c, double* w, const double* ub, double bdt);
+// the adjoint's start from the final state u: ub = (0, 2 jw E), the stage
+// weights w = bdt * (hbm1 | ebm1) * ub of the last stage of the last step (bdt
+// = b_5 dt), and kSeedBlocks partial sums of J = sum jw |E|^2
+constexpr int kSeedBlocks = 304;
+int adjoint_seed(Context* c, double* w, double* ub, const double* u, const double* jw, double bdt,
+                 double* partial);
 
 // nekgpu_noalloc.cu: cem_error norms with a fixed device scratch array
 int norms_noalloc(Context* c, const double* exact_dev, double l2[6], double linf[6]);
