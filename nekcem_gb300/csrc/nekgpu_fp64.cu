@@ -200,16 +200,27 @@ __device__ __forceinline__ void pml_node(const Fp64Dev& a, int l, int v, const d
   const double* pd = a.pml.data + q;
   double* aux = a.pml.aux + q;
   double* kx = a.pml.k + q;
-  const double fac = pd[12 * nn];
+  // every load before the stores, which they could not pass
+  const double fac = __ldg(pd + 12 * nn);
+  double f[6], kk[6], s1[3], A[3], B[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    f[c] = aux[c * nn];
+    kk[c] = first_stage ? 0.0 : kx[c * nn];
+    B[c] = __ldg(pd + (6 + c) * nn);
+    if (c < 3) {
+      s1[c] = __ldg(pd + c * nn);
+      A[c] = __ldg(pd + (3 + c) * nn);
+    }
+  }
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
     const int d = c % 3;
-    const double f = aux[c * nn];
-    const double rp = fma(R[c], fac, -(pd[d * nn] * f));
-    const double kv = first_stage ? a.dt * rp : fma(a.a, kx[c * nn], a.dt * rp);
-    R[c] = fma(pd[(3 + d) * nn], f, fma(-pd[(c < 3 ? 6 : 9) * nn + d * nn], u[c], R[c]));
+    const double rp = fma(R[c], fac, -(s1[d] * f[c]));
+    const double kv = first_stage ? a.dt * rp : fma(a.a, kk[c], a.dt * rp);
+    R[c] = fma(A[d], f[c], fma(-B[c], u[c], R[c]));
     kx[c * nn] = kv;
-    aux[c * nn] = fma(a.b, kv, f);
+    aux[c * nn] = fma(a.b, kv, f[c]);
   }
 }
 
@@ -320,10 +331,11 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
   const int ntask = SPLIT ? a.nelt * nsplit : a.nelt;
   for (int w = blockIdx.x; w < ntask; w += gridDim.x) {
     if (w + (int)gridDim.x >= ntask) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    const int e = SPLIT ? w / nsplit : w;
+    const int q0 = SPLIT ? w / nsplit : w;
+    const int e = EXT > 0 && a.pml.order ? a.pml.order[q0] : q0;  // (PML elements first)
     Slab sl{0, NX};
     if (SPLIT) {
-      const int q = w - e * nsplit;
+      const int q = w - q0 * nsplit;
       sl = Slab{q * NX / nsplit, (q + 1) * NX / nsplit};
     }
     const int* nbr = a.nbr + 6 * (long)e;
@@ -338,7 +350,8 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     // what the finish reads, and the next element's state, on their way to L2
     if (!SPLIT) {
-      const int en = w + (int)gridDim.x < ntask ? w + gridDim.x : e;
+      const int wn = w + (int)gridDim.x;
+      const int en = wn < ntask ? (EXT > 0 && a.pml.order ? a.pml.order[wn] : wn) : e;
 #pragma unroll 1
       for (int t = tid; t < 14 * ((N3 + 15) / 16); t += NT) {
         const int q = t / ((N3 + 15) / 16), o = 16 * (t - q * ((N3 + 15) / 16));

@@ -552,7 +552,7 @@ __device__ __forceinline__ void pml_node(const MixedDev& a, int l, int v, long g
   const double* pd = a.pml.data + q;
   double* aux = a.pml.aux + q;
   double* kx = a.pml.k + q;
-  const double fac = pd[12 * nn];
+  const double fac = __ldg(pd + 12 * nn);
   double f[6], kk[6], u[6];  // loaded before the stores (which they could not pass)
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
@@ -565,9 +565,9 @@ __device__ __forceinline__ void pml_node(const MixedDev& a, int l, int v, long g
     const int d = c % 3;
     float s, e;
     two_sum(Rh[c], Rl[c], s, e);
-    const double rp = fma(pair_to_double(s, e), fac, -(pd[d * nn] * f[c]));
+    const double rp = fma(pair_to_double(s, e), fac, -(__ldg(pd + d * nn) * f[c]));
     const double kv = first_stage ? a.dt * rp : fma(a.a, kk[c], a.dt * rp);
-    const double dR = fma(pd[(3 + d) * nn], f[c], -(pd[(c < 3 ? 6 : 9) * nn + d * nn] * u[c]));
+    const double dR = fma(__ldg(pd + (3 + d) * nn), f[c], -(__ldg(pd + (6 + c) * nn) * u[c]));
     two_sum(Rh[c], d2f_hi(dR), s, e);
     Rh[c] = s;
     Rl[c] = (Rl[c] + d2f_lo(dR)) + e;
@@ -733,20 +733,21 @@ __global__ void __launch_bounds__(MCfg<NX>::NT, mixed_min_blocks<NX, EXT, S>())
   };
   unsigned parity = 0;
   int buf = 0;  // area of the element's staged state and residual pairs
-  // tasks: element w/S, slab w%S
+  // tasks: element w/S (with PML, of that mesh's order), slab w%S
+  auto element = [&](int w) { return EXT > 0 && a.pml.order ? a.pml.order[w / S] : w / S; };
   const int w0 = a.e_begin * S + (int)blockIdx.x, w1 = a.e_end * S;
-  if (C::kTma && tid == 0 && w0 < w1) issue_tma(w0 / S, 0);
-  if (C::kAsync && w0 < w1) issue_async(w0 / S, 0, tid);
+  if (C::kTma && tid == 0 && w0 < w1) issue_tma(EXT == 0 ? w0 / S : element(w0), 0);
+  if (C::kAsync && w0 < w1) issue_async(EXT == 0 ? w0 / S : element(w0), 0, tid);
 
   for (int w = w0; w < w1; w += gridDim.x, buf ^= 1) {
     int tid = opaque_tid();
-    const int e = w / S, slab = S == 1 ? 0 : w % S;
+    const int e = EXT == 0 ? w / S : element(w), slab = S == 1 ? 0 : w % S;
     const int k0 = S == 1 ? 0 : slab_lo<NX, S>(slab), k1 = S == 1 ? NX : slab_lo<NX, S>(slab + 1);
     if (w + (int)gridDim.x >= w1) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     double* s_u64 = reinterpret_cast<double*>(smem + buf * C::SA);
     float2* s_R2 = reinterpret_cast<float2*>(smem + buf * C::SA);
     float2* s_u2 = reinterpret_cast<float2*>(smem + (buf ^ 1) * C::SA);
-    const int wn = w + gridDim.x, en = wn / S;
+    const int wn = w + gridDim.x, en = EXT == 0 ? wn / S : (wn < w1 ? element(wn) : e);
     const int* nbr = a.nbr + 6 * e;
     const float* eg = a.egm + 16 * e;
     // ---- early loads: partner face nodes (kept in registers until the flux)
