@@ -1226,10 +1226,11 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   double* d;
   int* di;
   if (norm)  // as (hi, lo) float pairs in the same 8 bytes
-    for (double& v : metrics) {
-      const float p[2] = {(float)v, (float)(v - (double)(float)v)};
-      std::memcpy(&v, p, 8);
-    }
+    for (std::vector<double>* w : {&metrics, &face, &fcoef})
+      for (double& v : *w) {
+        const float p[2] = {(float)v, (float)(v - (double)(float)v)};
+        std::memcpy(&v, p, 8);
+      }
   if ((st = A.put(&d, metrics))) return st;
   a.metrics = d;
   if ((st = A.put(&d, std::vector<double>(m->w3mn, m->w3mn + n3)))) return st;

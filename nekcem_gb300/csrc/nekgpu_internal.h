@@ -344,7 +344,7 @@ struct CurvedDev {
   double* u_out;
   double* k;
   // the mixed form's residual is res/w3: its coef, face, fcoef and src_w hold
-  // that factor, and its coef and metrics are (hi, lo) float pairs
+  // that factor, and all but src_w are (hi, lo) float pairs
   const double* coef;     // 2*npts: dt*hbm1 then dt*ebm1 (mixed: times w3)
   const double* metrics;  // 9*npts: rx, ry, rz, sx, sy, sz, tx, ty, tz (cofactors)
   const double* w3;       // nx^3

@@ -1128,14 +1128,15 @@ int dispatch_mixed(Context* c, const MixedDev& a, bool pdl) {
 // affine kernel (the element's 10-bit grid per component, D in its Dh, Df,
 // Dm pieces, one thread per GLL line); metrics and inverse mass come as float
 // pairs (made once on the host, or per dt) and enter in float-float
-// arithmetic, an H and an E component per packed instruction; the flux is
-// FP64 (the FP64 pipe is idle meanwhile), joined as float pairs; the RK
-// update is FP64.
+// arithmetic, an H and an E component per packed instruction, as do normals,
+// areas and face coefficients in the flux of the FP64 jumps; the RK update is
+// FP64.
 //
 // One block per element at a time, thread per node, line and face node, as in
 // k_curved_stage.  With a thread per node forming its own 18 derivatives from
 // shared memory and the flux in float pairs (128 registers, one block per SM)
-// the 12^3-element N=7 box took 148 us per stage; 125 us so (FP64 pipe 53 % busy, issue 41 %).
+// the 12^3-element N=7 box took 148 us per stage; 106 us so (125 with the flux in FP64 throughout: its 42 FP64
+// slots per node did not overlap the FP32 work).
 // ===========================================================================
 struct PairF {
   float h, l;
@@ -1171,6 +1172,34 @@ __device__ __forceinline__ void pfma2(Pair2& acc, PairF m, const Pair2& d) {
   const float2 t = __fadd2_rn(__ffma2_rn(__ffma2_rn(bb, neg, s), neg, acc.h), __ffma2_rn(bb, neg, p));
   acc.h = s;
   acc.l = __fadd2_rn(__fadd2_rn(acc.l, e), t);
+}
+
+__device__ __forceinline__ Pair2 pmul2(const Pair2& a, const Pair2& b) {
+  const float2 neg = make_float2(-1.0f, -1.0f);
+  const float2 p = __fmul2_rn(a.h, b.h);
+  float2 e = __ffma2_rn(a.h, b.h, __fmul2_rn(p, neg));
+  e = __ffma2_rn(a.h, b.l, e);
+  return Pair2{p, __ffma2_rn(a.l, b.h, e)};
+}
+__device__ __forceinline__ Pair2 both(PairF m) {
+  return Pair2{make_float2(m.h, m.h), make_float2(m.l, m.l)};
+}
+__device__ __forceinline__ void padd2(Pair2& acc, const Pair2& b) {
+  const float2 neg = make_float2(-1.0f, -1.0f);
+  const float2 s = __fadd2_rn(acc.h, b.h);  // two-sum
+  const float2 bb = __ffma2_rn(acc.h, neg, s);
+  const float2 t = __fadd2_rn(__ffma2_rn(__ffma2_rn(bb, neg, s), neg, acc.h), __ffma2_rn(bb, neg, b.h));
+  acc.h = s;
+  acc.l = __fadd2_rn(__fadd2_rn(acc.l, b.l), t);
+}
+// a x b for a pair vector a and two pair vectors b side by side
+__device__ __forceinline__ void pcross2(const PairF* a, const Pair2* b, Pair2* o) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int p = (c + 1) % 3, q = (c + 2) % 3;
+    o[c] = pmul2(both(a[p]), b[q]);
+    padd2(o[c], pmul2(both(PairF{-a[q].h, -a[q].l}), b[p]));
+  }
 }
 
 template <int NX>
@@ -1278,44 +1307,48 @@ __global__ void __launch_bounds__(CMCfg<NX>::NT, CMCfg<NX>::kMinBlocks)
       const float uh = (__fadd_rn(__fmaf_rn(uf, qi, M), -M)) * qv;
       if (node) s_u2[c * N3P + pn] = make_float2(uh, __fadd_rn(__fsub_rn(uf, uh), ulo));
     }
-    // ---- upwind flux of the face node, FP64 (k_curved_stage) --------------------
+    // ---- upwind flux of the face node: jumps in FP64, then float pairs, the E
+    // and the H part side by side -------------------------------------------------
     float2 F[6];
     if (tid < NF) {
-      double dH[3], dE[3], fl[6];
+      Pair2 J[3];  // ([E], [H])
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double em = s_u64[(c + 3) * N3P + fv];
-        dH[c] = pv >= 0 ? up[c] - s_u64[c * N3P + fv] : 0.0;
-        dE[c] = pv >= 0 ? up[c + 3] - em : -2.0 * em;  // PEC mirror
+        const double dH = pv >= 0 ? up[c] - s_u64[c * N3P + fv] : 0.0;
+        const double dE = pv >= 0 ? up[c + 3] - em : -2.0 * em;  // PEC mirror
+        J[c] = Pair2{make_float2(d2f_hi(dE), d2f_hi(dH)), make_float2(d2f_lo(dE), d2f_lo(dH))};
       }
-      const double n[3] = {a.face[js], a.face[L + js], a.face[2 * L + js]};
-      double xE[3], xH[3];
+      const float2* fp = reinterpret_cast<const float2*>(a.face);
+      PairF n[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const int p = (c + 1) % 3, q = (c + 2) % 3;
-        xE[c] = fma(n[p], dE[q], -(n[q] * dE[p]));
-        xH[c] = fma(n[p], dH[q], -(n[q] * dH[p]));
+        const float2 v = fp[c * L + js];
+        n[c] = PairF{v.x, v.y};
       }
+      // factors of (n x [H], n x [E]) in (E, H): (Z02, Y02), and of the upwind
+      // terms n x (n x [u]), subtracted: (C02Z, C02Y); times the area, over w3
+      Pair2 K1, K2;
       if (a.fcoef) {
-        const double Y02 = a.fcoef[js], C02Y = a.fcoef[L + js], Z02 = a.fcoef[2 * L + js],
-                     C02Z = a.fcoef[3 * L + js];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int p = (c + 1) % 3, q = (c + 2) % 3;
-          fl[c] = fma(Y02, xE[c], -(C02Y * fma(n[p], xH[q], -(n[q] * xH[p]))));
-          fl[3 + c] = fma(Z02, xH[c], -(C02Z * fma(n[p], xE[q], -(n[q] * xE[p]))));
-        }
-      } else {  // Y02 = -1/2, C02Y = Z02 = C02Z = 1/2 times the area
-        const double h = a.face[3 * L + js];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int p = (c + 1) % 3, q = (c + 2) % 3;
-          fl[c] = -h * fma(n[p], xH[q], fma(-n[q], xH[p], xE[c]));
-          fl[3 + c] = h * fma(-n[p], xE[q], fma(n[q], xE[p], xH[c]));
-        }
+        const float2* cp = reinterpret_cast<const float2*>(a.fcoef);
+        const float2 Y = cp[js], CY = cp[L + js], Z = cp[2 * L + js], CZ = cp[3 * L + js];
+        K1 = Pair2{make_float2(Z.x, Y.x), make_float2(Z.y, Y.y)};
+        K2 = Pair2{make_float2(-CZ.x, -CY.x), make_float2(-CZ.y, -CY.y)};
+      } else {  // Y02 = -1/2, C02Y = Z02 = C02Z = 1/2
+        const float2 h = fp[3 * L + js];
+        K1 = Pair2{make_float2(h.x, -h.x), make_float2(h.y, -h.y)};
+        K2 = Pair2{make_float2(-h.x, -h.x), make_float2(-h.y, -h.y)};
       }
+      Pair2 X[3], U[3];
+      pcross2(n, J, X);
+      pcross2(n, X, U);
 #pragma unroll
-      for (int c = 0; c < 6; ++c) F[c] = make_float2(d2f_hi(fl[c]), d2f_lo(fl[c]));
+      for (int c = 0; c < 3; ++c) {
+        Pair2 f2 = pmul2(K1, Pair2{make_float2(X[c].h.y, X[c].h.x), make_float2(X[c].l.y, X[c].l.x)});
+        padd2(f2, pmul2(K2, U[c]));
+        F[c] = make_float2(f2.h.y, f2.l.y);
+        F[3 + c] = make_float2(f2.h.x, f2.l.x);
+      }
     }
     // The lines of one direction run beside the lift of one axis (its two
     // faces share no node) and the products of the direction before:
