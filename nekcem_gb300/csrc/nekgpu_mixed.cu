@@ -193,9 +193,9 @@ struct MCfg {
   // synchronously: -0.5 %, -1.8 % with the async copies)
   static constexpr bool kAsync = !kTma && NX >= 7;
   // L1 prefetch of the finish's loads where it measured faster: in the t-line
-  // tasks that finish (N=6 +2.5 %, N=5 +1.7 %, N=4 +0.4 %)
+  // tasks that finish (N=6 +2.5 %, N=5 +1.7 %; N=4 -1.9 %)
   // and for the next node of the node-by-node finish (N=8 +1.4 %; N=7 -2.2 %)
-  static constexpr bool kPfLine = NX == 5 || NX == 6 || NX == 7;
+  static constexpr bool kPfLine = NX == 6 || NX == 7;
   static constexpr bool kPfNode = NX == 9;
   // Where the components finish (inverse mass, RK update) without the
   // extension terms: true = the t-line tasks finish H1, H2, E1, E2 on their
@@ -382,13 +382,6 @@ __device__ __forceinline__ float2 jump_pair(double p, float2 own) {
   return make_float2(s, (d2f_lo(p) - own.y) + t);
 }
 
-// two_sum(a, sg * b) for sg = +-1
-__device__ __forceinline__ void signed_sum(float a, float sg, float b, float& s, float& e) {
-  s = fmaf(sg, b, a);
-  const float bb = s - a;
-  e = (a - (s - bb)) + fmaf(sg, b, -bb);
-}
-
 // Outputs I0 .. I0+NXP-1 of one line task (all NX of them, or the part of one
 // of the threads that share the line): the contraction, the rho factor, the lifted
 // flux at the line's ends and the accumulation into the residual pairs (or,
@@ -429,26 +422,20 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
       h = p;
       r = ee;
     }
-    const bool end = i == 0 || i == NX - 1;
-    if (end || (!FIN && init)) {
-      h *= sg;
-      r *= sg;
-    }
-    if (end) {  // the lifted flux pair of the end's face
+    h *= sg;
+    r *= sg;
+    if (i == 0 || i == NX - 1) {  // the lifted flux pair of the end's face
       const float2 F = i == 0 ? flux_m : flux_p;
       float s, t;
       two_sum(h, F.x, s, t);
       h = s;
       r = (r + F.y) + t;
     }
-    // the sign of an inner output rides on the additions (sg h is exact)
-    const float sa = end ? 1.0f : sg;
     float2* Rp = R0 + line_node<NX, DIR>(la, lb, i);
     if (FIN) {
       const float2 old = *Rp;
       float sum, err;
-      signed_sum(old.x, sa, h, sum, err);
-      r *= sa;
+      two_sum(old.x, h, sum, err);
       const int vol = DIR == 0 ? i + NX * la + C::N2 * lb
                                : (DIR == 1 ? la + NX * i + C::N2 * lb : la + NX * lb + C::N2 * i);
       rk_finish<C::kIntAdd>(a, rt, (long)e * C::N3 + vol, sum, (old.y + r) + err, first_stage);
@@ -457,8 +444,8 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
     } else {
       const float2 old = *Rp;
       float sum, err;
-      signed_sum(old.x, sa, h, sum, err);
-      *Rp = make_float2(sum, fmaf(sa, r, old.y) + err);
+      two_sum(old.x, h, sum, err);
+      *Rp = make_float2(sum, (old.y + r) + err);
     }
   }
 }
