@@ -73,9 +73,9 @@ __device__ __forceinline__ void fixed_line(const double* u, FixedLine<NX>& f) {
 }
 
 // b 2^(E - bias) rounded to FP64, |b| < 2^63, by integer operations: the
-// conversion instruction from 64-bit integers costs three FP64-pipe slots
-// (16^3 box at N=7: 311 us per stage with it, see below for this form).
-// Ties round away from zero.
+// conversion instruction from 64-bit integers takes an FP64-pipe slot per
+// output, 12 per node (16^3 box at N=7: 311 us per stage with it, 277 with
+// this form).  Ties round away from zero.
 __device__ __forceinline__ double fixed_join(long long b, int e) {
   const long long s = b >> 63;
   const unsigned long long mag = (unsigned long long)((b ^ s) - s);

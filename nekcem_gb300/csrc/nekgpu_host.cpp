@@ -1196,49 +1196,70 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   if ((st = A.get(&c->d_u[0], 6 * npts)) || (st = A.get(&c->d_u[1], 6 * npts))) return st;
   if ((st = upload_common(c, A, bm1, eb, hb))) return st;
   if ((st = A.get(&c->d_coef, 2 * npts))) return st;
-  std::vector<double> base(2 * npts);
-  // the mixed form's residual is res/w3
+  // the mixed form's residual is res/w3, and its metrics and face data are
+  // stored as (hi, lo) float pairs in the same 8 bytes
   const bool norm = c->form == NEKGPU_MIXED;
-  for (long g = 0; g < npts; ++g) {
-    const double w = norm ? m->w3mn[g % n3] : 1.0;
-    base[g] = hb[g] * w;
-    base[npts + g] = eb[g] * w;
-  }
+  std::vector<double> base(2 * npts);
+  for (long e = 0; e < m->nelt; ++e)
+    for (long v = 0; v < n3; ++v) {
+      const double w = norm ? m->w3mn[v] : 1.0;
+      base[e * n3 + v] = hb[e * n3 + v] * w;
+      base[npts + e * n3 + v] = eb[e * n3 + v] * w;
+    }
   if ((st = A.put(&c->d_cbase, base))) return st;
   c->coef_dt = std::nan("");
   const double* mt[9] = {m->rxmn, m->rymn, m->rzmn, m->sxmn, m->symn, m->szmn, m->txmn, m->tymn, m->tzmn};
-  std::vector<double> metrics(9 * (size_t)npts), face(4 * (size_t)nxzfl), fcoef(4 * (size_t)nxzfl);
-  for (int q = 0; q < 9; ++q) std::copy(mt[q], mt[q] + npts, metrics.begin() + q * npts);
+  const double* nr[3] = {m->unxm, m->unym, m->unzm};
+  // one row of `count` values to the device
+  std::vector<float> row(norm ? 2 * (size_t)std::max(npts, nxzfl) : 0);
+  auto put_row = [&](double* dst, const double* src, long count) -> int {
+    if (norm) {
+      for (long i = 0; i < count; ++i) {
+        row[2 * i] = (float)src[i];
+        row[2 * i + 1] = (float)(src[i] - (double)row[2 * i]);
+      }
+    }
+    return check_cuda(cudaMemcpy(dst, norm ? (const void*)row.data() : src, count * sizeof(double),
+                                 cudaMemcpyHostToDevice));
+  };
+  std::vector<double> area(nxzfl), half(nxzfl);
+  for (long e = 0; e < m->nelt; ++e)
+    for (int f = 0; f < 6; ++f)
+      for (int b = 0; b < n; ++b)
+        for (int a = 0; a < n; ++a) {
+          const long j = a + (long)n * b + n2 * (f + 6 * e);
+          area[j] = norm ? m->aream[j] / m->w3mn[face_vol(f, a, b, n)] : m->aream[j];
+          half[j] = 0.5 * area[j];
+        }
+  auto impedance = [&](int q, long j) {
+    const double Y0 = m->Y_0[j], Z0 = m->Z_0[j];
+    return q == 0 ? -0.5 / Y0 * m->Y_1[j] : q == 1 ? 0.5 / Y0 * m->C0
+         : q == 2 ? 0.5 / Z0 * m->Z_1[j] : 0.5 / Z0 * m->C0;
+  };
   bool uniform = true;
-  for (long j = 0; j < nxzfl; ++j) {
-    face[j] = m->unxm[j];
-    face[nxzfl + j] = m->unym[j];
-    face[2 * nxzfl + j] = m->unzm[j];
-    const double area = norm ? m->aream[j] / m->w3mn[(m->cemface[j] - 1) % n3] : m->aream[j];
-    face[3 * nxzfl + j] = 0.5 * area;
-    const double Y0 = m->Y_0[j], Y1 = m->Y_1[j], Z0 = m->Z_0[j], Z1 = m->Z_1[j];
-    const double o[4] = {-0.5 / Y0 * Y1, 0.5 / Y0 * m->C0, 0.5 / Z0 * Z1, 0.5 / Z0 * m->C0};
-    for (int q = 0; q < 4; ++q) fcoef[q * nxzfl + j] = area * o[q];
-    uniform = uniform && o[0] == -0.5 && o[1] == 0.5 && o[2] == 0.5 && o[3] == 0.5;
-  }
+  for (long j = 0; j < nxzfl && uniform; ++j)
+    uniform = impedance(0, j) == -0.5 && impedance(1, j) == 0.5 && impedance(2, j) == 0.5 &&
+              impedance(3, j) == 0.5;
   CurvedDev& a = c->cargs;
   a = CurvedDev{};
   double* d;
   int* di;
-  if (norm)  // as (hi, lo) float pairs in the same 8 bytes
-    for (std::vector<double>* w : {&metrics, &face, &fcoef})
-      for (double& v : *w) {
-        const float p[2] = {(float)v, (float)(v - (double)(float)v)};
-        std::memcpy(&v, p, 8);
-      }
-  if ((st = A.put(&d, metrics))) return st;
+  if ((st = A.get(&d, 9 * (size_t)npts))) return st;
+  for (int q = 0; q < 9; ++q)
+    if ((st = put_row(d + q * npts, mt[q], npts))) return st;
   a.metrics = d;
   if ((st = A.put(&d, std::vector<double>(m->w3mn, m->w3mn + n3)))) return st;
   a.w3 = d;
-  if ((st = A.put(&d, face))) return st;
+  if ((st = A.get(&d, 4 * (size_t)nxzfl))) return st;
+  for (int q = 0; q < 4; ++q)
+    if ((st = put_row(d + q * nxzfl, q < 3 ? nr[q] : half.data(), nxzfl))) return st;
   a.face = d;
   if (!uniform) {
-    if ((st = A.put(&d, fcoef))) return st;
+    if ((st = A.get(&d, 4 * (size_t)nxzfl))) return st;
+    for (int q = 0; q < 4; ++q) {
+      for (long j = 0; j < nxzfl; ++j) half[j] = area[j] * impedance(q, j);
+      if ((st = put_row(d + q * nxzfl, half.data(), nxzfl))) return st;
+    }
     a.fcoef = d;
   }
   if ((st = A.put(&di, partner))) return st;

@@ -564,7 +564,7 @@ int mixed_stage(Context* c, int rkstep, double time, double dt);
 // pair_to_double on n device pairs (default stream)
 int pair_join_selftest(const float* s, const float* t, double* out, long n);
 // one mixed stage between given buffers (u_in -> u_out, k_in -> k_out), as
-// fused_stage_buffers; the context's own state is untouched
+// fp64_stage_buffers; the context's own state is untouched
 int mixed_stage_buffers(Context* c, int rkstep, double time, double dt, const double* u_in,
                         double* u_out, double* k_in, double* k_out);
 // the same with explicit stage arguments (coefficient pairs already scaled),

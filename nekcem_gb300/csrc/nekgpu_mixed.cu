@@ -1,6 +1,6 @@
 // Mixed-precision Maxwell DG stage kernel for sm_103a (NEKGPU_MIXED).
 //
-// Same stage as nekgpu_fused.cu -- weighted curl from the GLL derivative
+// Same stage as nekgpu_fp64.cu -- weighted curl from the GLL derivative
 // contractions (src/nek5_grad.F:2-19, src/cem_maxwell.F:1428-1497), upwind
 // face flux with the partner-face read that replaces gs_op_fields
 // (src/cem_maxwell.F:922-1002, 1368-1426), lift (src/cem_maxwell.F:725-735),
@@ -33,7 +33,8 @@
 //    coefficient carries dt*(2/hx)/eps.
 //  * Pair residual.  The residual stays an unevaluated FP32 pair (hi, lo); it
 //    is multiplied by the FP64 coefficient as a float-float product, rounded
-//    to FP64 once (DADD) and enters the FP64 RK update (2 DFMA).
+//    to FP64 once (a DADD, or integer
+//    operations) and enters the FP64 RK update (2 DFMA).
 //
 // FP64 <-> FP32 conversions use integer instructions only: every FP64-pipe
 // instruction on GB300 (including F2F) runs at 2 lanes/clock/SM.
@@ -48,7 +49,6 @@
 namespace nekgpu {
 
 namespace {
-
 
 // (Rh, Rl) += w * f for float pairs w = (wh, wl), f = (fh, fl): the product's
 // rounding error and cross terms go to the low part (~2^-46 of |w f|), so a
@@ -95,8 +95,6 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned
       "l"(src), "r"(bytes), "r"(smem_addr(bar))
       : "memory");
 }
-// bulk prefetch of a global range into L2 (a hint: no completion to wait for);
-// address and size multiples of 16 bytes
 // 8-byte asynchronous global -> shared copies (element blocks whose size is
 // not a multiple of 16 bytes, where a bulk copy cannot start on every element)
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
@@ -108,6 +106,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void prefetch_l1(const void* p) {
   asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p));
 }
+// bulk prefetch of a global range into L2 (a hint: no completion to wait for);
+// address and size multiples of 16 bytes
 __device__ __forceinline__ void prefetch_l2(const void* src, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
@@ -1122,8 +1122,9 @@ int dispatch_mixed(Context* c, const MixedDev& a, bool pdl) {
 // One block per element at a time, thread per node, line and face node, as in
 // k_curved_stage.  With a thread per node forming its own 18 derivatives from
 // shared memory and the flux in float pairs (128 registers, one block per SM)
-// the 12^3-element N=7 box took 148 us per stage; 106 us so (125 with the flux in FP64 throughout: its 42 FP64
-// slots per node did not overlap the FP32 work).
+// the 12^3-element N=7 box took 148 us per stage; 106 us so (125 with the
+// flux in FP64 throughout: its 42 FP64 slots per node did not overlap the
+// FP32 work).
 // ===========================================================================
 struct PairF {
   float h, l;
