@@ -31,8 +31,9 @@
 // error terms, two-sum accumulation, ~2^-47 of the sum of the magnitudes, each
 // result joined into one FP64 value.
 //
-// What bounds it: the FP64 pipe (43 slots per node) and issue (2400
-// instructions per node, the face terms most of them).  With double-float
+// What bounds it: latencies at four blocks per SM, the FP64 pipe (41 slots per
+// node) 42 % and issue (75 warp instructions per node, the face terms most of
+// them) 38 % busy; 49 us per stage at 512 elements, N=7.  With double-float
 // contractions per node and the face terms added per node by divergent warps
 // (~100 FP64 slots per node, 512 threads and one block per SM) the reverse
 // sweep of 100 steps of the 8^3-element N=7 box, the recomputation beside it,
