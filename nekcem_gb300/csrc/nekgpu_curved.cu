@@ -73,7 +73,7 @@ __device__ __forceinline__ void curved_lines(const double* s_u, double* s_d, con
     double u[NX];
 #pragma unroll
     for (int l = 0; l < NX; ++l) u[l] = s_u[base + step * l];
-    fixed_line<NX>(u, f);
+    fixed_line<NX>(u, a.fd.maxexp, f);
   }
   if (a.fd.ok && !f.special) {
 #pragma unroll

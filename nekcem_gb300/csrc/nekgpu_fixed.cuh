@@ -21,9 +21,10 @@
 //
 // Every error is below 2^-57 of the line's largest value times the largest
 // entry of D, against about 2^-53 for each step of an FP64 sum.  A line that
-// holds an infinity, a NaN or a value above 2^1006 or lies below 2^-823 as a
-// whole, and a D that does not fit the table (FixedD::ok), is contracted in
-// FP64 instead, term by term.
+// holds an infinity, a NaN or a value above 2^1006 (with a D of large entries
+// less: FixedD::maxexp, so that no output's exponent leaves FP64's range) or
+// lies below 2^-823 as a whole, and a D that does not fit the table
+// (FixedD::ok), is contracted in FP64 instead, term by term.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,8 +42,6 @@ __device__ __forceinline__ unsigned long long shr64(unsigned long long v, unsign
   return r;
 }
 
-// biased exponents of the lines contracted in integers: [min, max)
-constexpr int kFixedMinExp = 200, kFixedMaxExp = 2030;
 
 template <int NX>
 struct FixedLine {
@@ -51,13 +50,14 @@ struct FixedLine {
   bool special;  // contract in FP64
 };
 
+// maxexp: FixedD::maxexp
 template <int NX>
-__device__ __forceinline__ void fixed_line(const double* u, FixedLine<NX>& f) {
+__device__ __forceinline__ void fixed_line(const double* u, int maxexp, FixedLine<NX>& f) {
   unsigned em = 0;
 #pragma unroll
   for (int k = 0; k < NX; ++k) em = max(em, (unsigned)__double2hiint(u[k]) & 0x7FFFFFFFu);
   f.E = max((int)(em >> 20), kFixedMinExp);  // (a line of zeros: any exponent)
-  f.special = (em > 0 && em < ((unsigned)kFixedMinExp << 20)) || f.E >= kFixedMaxExp;
+  f.special = (em > 0 && em < ((unsigned)kFixedMinExp << 20)) || f.E >= maxexp;
 #pragma unroll
   for (int k = 0; k < NX; ++k) {
     const unsigned hi = (unsigned)__double2hiint(u[k]), lo = (unsigned)__double2loint(u[k]);

@@ -603,6 +603,9 @@ void fixed_table(const double* D, int n, FixedD& t) {
     if (fits) {
       t.ok = 1;
       t.bias = 1022 + kd;
+      // fixed_join's exponent field stays below that of infinity: the largest
+      // output, 2^63 2^(E - bias), has 1023 + 63 + E - bias
+      t.maxexp = std::min(kFixedMaxExp, t.bias + 960);
       return;
     }
   }

@@ -215,10 +215,13 @@ __device__ inline void graphene_slot(const GrapheneDev& G, long g, const double 
 
 // D in fixed point for the integer contractions of the FP64 kernels
 // (nekgpu_fixed.cuh): entry i + nx*l holds D(i,l) 2^kd = hi 2^31 + lo, hi8 =
-// 8 hi; bias = 1022 + kd.  ok = 0: D does not fit, contract in FP64.
+// 8 hi; bias = 1022 + kd.  ok = 0: D does not fit, contract in FP64.  Lines
+// whose largest biased exponent lies in [kFixedMinExp, maxexp) are contracted
+// in integers.
 constexpr int kMaxFixed = 9;
+constexpr int kFixedMinExp = 200, kFixedMaxExp = 2030;
 struct FixedD {
-  int ok, bias;
+  int ok, bias, maxexp;
   int hi[kMaxFixed * kMaxFixed], lo[kMaxFixed * kMaxFixed], hi8[kMaxFixed * kMaxFixed];
 };
 

@@ -82,7 +82,7 @@ __device__ __forceinline__ void line_outputs(const double* pu, int step, int i0,
     double u[NX];
 #pragma unroll
     for (int l = 0; l < NX; ++l) u[l] = pu[step * l];
-    fixed_line<NX>(u, f);
+    fixed_line<NX>(u, fd.maxexp, f);
   }
   if (fd.ok && !f.special) {
     if (!SPLIT) {
