@@ -44,7 +44,8 @@ extern "C" {
 /* Compute forms. */
 #define NEKGPU_PLAIN 0   /* unfused all-FP64 kernels, one per reference routine */
 #define NEKGPU_FUSED64 1 /* fused curl+flux+lift+mass+RK stage kernel, FP64 (the
-                            contractions in 64-bit fixed point, as accurate) */
+                            contractions in 64-bit fixed point per GLL line, at
+                            a smaller error than an FP64 sum's) */
 #define NEKGPU_MIXED 2   /* fused stage kernel: FP32 contractions/curl/flux,
                             FP64 state, RK register, inverse mass and norms;
                             exact-hi compensated contractions on a normalised
@@ -338,6 +339,11 @@ int nekgpu_selftest_wait(nekgpu_ctx* ctx, int polls);
  * (test hook): out[i] = s[i] + t[i], exact whenever the sum fits in 53 bits,
  * else truncated below one FP64 ulp. */
 int nekgpu_selftest_pair_join(const float* s, const float* t, double* out, long n);
+/* The FP64 stage's fixed-point contraction of n lines of nx values (3..9) with
+ * the nx x nx matrix D (D(i,l) at [i + nx*l]) on host arrays, on device 0 (test
+ * hook): out[i + nx*line] = sum_l D(i,l) u[l + nx*line].  split: by the kernel
+ * variant of meshes with few elements. */
+int nekgpu_selftest_fixed_lines(int nx, const double* D, const double* u, double* out, long n, int split);
 /* chk_blowup (src/cem_common.F:1150-1165): NEKGPU_ERR_BLOWUP if any state
  * value is non-finite or above 1e20 in magnitude */
 int nekgpu_check_blowup(nekgpu_ctx* ctx);

@@ -106,6 +106,7 @@ SIGNATURES = [
     ("nekgpu_check_blowup", C.c_int, [C.c_void_p]),
     ("nekgpu_selftest_wait", C.c_int, [C.c_void_p, C.c_int]),
     ("nekgpu_selftest_pair_join", C.c_int, [C.c_void_p, C.c_void_p, dp, C.c_long]),
+    ("nekgpu_selftest_fixed_lines", C.c_int, [C.c_int, dp, dp, dp, C.c_long, C.c_int]),
     ("nekgpu_adjoint_gradient", C.c_int, [C.c_void_p, C.c_int, C.c_double, C.c_double, dp, dp, dp,
                                          C.c_int, dp, dp]),
     ("nekgpu_adjoint_init", C.c_int, [C.c_void_p, dp, C.c_int]),

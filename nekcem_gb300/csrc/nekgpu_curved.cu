@@ -78,10 +78,9 @@ __device__ __forceinline__ void curved_lines(const double* s_u, double* s_d, con
   if (a.fd.ok && !f.special) {
 #pragma unroll
     for (int i = 0; i < NX; ++i)
-      s_d[base + step * i] = fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
+      s_d[base + step * i] = fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo) {
         hi = a.fd.hi[i + NX * l];
         lo = a.fd.lo[i + NX * l];
-        hi8 = a.fd.hi8[i + NX * l];
       });
   } else {  // a line out of the integer form's range: in FP64
 #pragma unroll 1

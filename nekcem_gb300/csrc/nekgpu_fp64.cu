@@ -44,7 +44,7 @@ struct DCfg : ElemCfg<NX> {
   // state, residual, flux [face][line slot][N2], D rows (split form)
   static constexpr size_t off_R = 6 * (size_t)E::N3P * 8, off_F = 2 * off_R;
   static constexpr size_t off_D = (off_F + 24 * (size_t)E::N2 * 8 + 15) / 16 * 16;
-  static constexpr size_t smem(bool split) { return off_D + (split ? E::N2 * 16 : 0); }
+  static constexpr size_t smem(bool split) { return off_D + (split ? E::N2 * 8 : 0); }
 };
 
 // Field component of the k-th partner value of face f: all six with the
@@ -116,7 +116,7 @@ __device__ __forceinline__ void line_put(double* Rp, double x, bool neg, double 
 // constant bank).
 template <int NX, int PH, int OP, bool SPLIT>
 __device__ __forceinline__ void line_task(int type, int lam, int i0, int i1, const double* s_u,
-                                          double* s_R, const double* s_F, const int4* s_D,
+                                          double* s_R, const double* s_F, const int2* s_D,
                                           double rho_s, double rho_t, const Fp64Dev& a) {
   using C = DCfg<NX>;
   constexpr int N2 = C::N2;
@@ -142,7 +142,7 @@ __device__ __forceinline__ void line_task(int type, int lam, int i0, int i1, con
 // split form (type, group of og outputs, line).
 template <int NX, int PH, bool SPLIT>
 __device__ __forceinline__ void line_phase(const double* s_u, double* s_R, const double* s_F,
-                                           const int4* s_D, double rho_s, double rho_t, Slab sl,
+                                           const int2* s_D, double rho_s, double rho_t, Slab sl,
                                            int og, const Fp64Dev& a) {
   using C = DCfg<NX>;
   constexpr int N2 = C::N2, NT = C::NT;
@@ -304,9 +304,12 @@ __device__ __noinline__ void face_extras(const Fp64Dev& a, int e, int t, int f, 
   }
 }
 
+// Blocks per SM the launch is built for.  EXT 1 at N=4: four blocks of 96
+// threads (168 registers; 336 elements with PML 19.8 us per stage, 1000 32.1;
+// built for two the compiler takes 204 registers, three blocks: 25.5 and 50.4).
 template <int NX, int EXT>
 constexpr int fp64_min_blocks() {
-  return NX == 9 || EXT ? 2 : (NX == 8 ? 3 : 4);
+  return EXT == 1 && NX == 5 ? 4 : (NX == 9 || EXT ? 2 : (NX == 8 ? 3 : 4));
 }
 
 template <int NX, int EXT, bool SPLIT>
@@ -319,12 +322,12 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
   double* s_u = reinterpret_cast<double*>(smem);
   double* s_R = reinterpret_cast<double*>(smem + C::off_R);
   double* s_F = reinterpret_cast<double*>(smem + C::off_F);
-  int4* s_D = reinterpret_cast<int4*>(smem + C::off_D);
+  int2* s_D = reinterpret_cast<int2*>(smem + C::off_D);
   const int tid = threadIdx.x;
   const long P = a.npts;
   const bool first_stage = (a.a == 0.0);  // rk4a(1) = 0: k restarts
   if (SPLIT)
-    for (int t = tid; t < N2; t += NT) s_D[t] = make_int4(a.fd.hi[t], a.fd.lo[t], a.fd.hi8[t], 0);
+    for (int t = tid; t < N2; t += NT) s_D[t] = make_int2(a.fd.hi[t], a.fd.lo[t]);
   // a programmatic dependent of the previous stage: nothing it wrote is read
   // before it has completed; the next stage may launch from the last task on
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -567,10 +570,35 @@ int fp64_launch(Context* c, Fp64Dev& a, int rkstep, double time, double dt, bool
   return a.pml.slot || a.disp.slot ? dispatch<1>(c, a, pdl) : dispatch<0>(c, a, pdl);
 }
 
+// line_outputs over arrays (self-test of the fixed-point contractions)
+struct LinesDev {
+  FixedD fd;
+  double D[kMaxFixed * kMaxFixed];
+};
+template <int NX, bool SPLIT>
+__global__ void __launch_bounds__(256) k_fixed_lines(const __grid_constant__ LinesDev a, const double* u,
+                                                     double* out, long n) {
+  __shared__ int2 s_D[NX * NX];
+  for (int t = threadIdx.x; t < NX * NX; t += blockDim.x) s_D[t] = make_int2(a.fd.hi[t], a.fd.lo[t]);
+  __syncthreads();
+  const long line = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (line >= n) return;
+  double* o = out + line * NX;
+  line_outputs<NX, SPLIT>(u + line * NX, 1, 0, NX, a.fd, a.D, s_D, [&](int i, double x) { o[i] = x; });
+}
+template <int NX>
+int launch_lines(const LinesDev& a, const double* u, double* out, long n, bool split) {
+  const unsigned g = (unsigned)((n + 255) / 256);
+  if (split) k_fixed_lines<NX, true><<<g, 256>>>(a, u, out, n);
+  else k_fixed_lines<NX, false><<<g, 256>>>(a, u, out, n);
+  return check_cuda(cudaGetLastError());
+}
+
 }  // namespace
 
 // The fixed-point table of D (nekgpu_fixed.cuh): the largest scale 2^kd with
-// |D| 2^kd < 2^59 whose cross sums stay below 2^63 for any line.
+// |D| 2^kd <= 2^61 whose cross sums stay below 2^63 for any line (the first one
+// tried for the GLL matrices of N=2..8; the second for N=8's weighted transpose).
 void fixed_table(const double* D, int n, FixedD& t) {
   t = FixedD{};
   double dmax = 0.0;
@@ -582,32 +610,46 @@ void fixed_table(const double* D, int n, FixedD& t) {
   if (!fine || !(dmax > 0.0)) return;
   int ex = 0;
   std::frexp(dmax, &ex);  // dmax < 2^ex
-  for (int kd = 59 - ex; kd >= 57 - ex; --kd) {
+  for (int kd = 61 - ex; kd >= 55 - ex; --kd) {
     if (kd > 150 || kd < -60) return;
     bool fits = true;
     for (int i = 0; i < n && fits; ++i) {
-      double cross = 0.0;
+      double cross = 0.0;  // bounds sum |h L + l H|, and sum |h H| with it
       for (int l = 0; l < n; ++l) {
         const int k = i + n * l;
-        const double d = std::ldexp(D[k], kd);
-        const long long m = std::llrint(std::fabs(d));
-        if (m >= (1LL << 59)) fits = false;
-        const int s = d < 0 ? -1 : 1;
-        t.hi[k] = s * (int)(m >> 31);
-        t.lo[k] = s * (int)(m & 0x7FFFFFFF);
-        t.hi8[k] = 8 * t.hi[k];
-        cross += (double)(1 << 28) * (double)(m & 0x7FFFFFFF) + 2147483648.0 * (double)(m >> 31);
+        const long long m = std::llrint(std::fabs(std::ldexp(D[k], kd)));
+        const long long H = (m + (1LL << 30)) >> 31, L = m - (H << 31);
+        const int s = D[k] < 0 ? -1 : 1;
+        t.hi[k] = s * (int)H;
+        t.lo[k] = s * (int)L;
+        cross += (double)(1 << 30) * ((double)H + std::fabs((double)L));
       }
-      fits = fits && cross < 9.2e18;
+      fits = cross < 9.2e18;
     }
     if (fits) {
       t.ok = 1;
-      t.bias = 1022 + kd;
+      t.bias = 1021 + kd;
       // fixed_join's exponent field stays below that of infinity: the largest
       // output, 2^63 2^(E - bias), has 1023 + 63 + E - bias
       t.maxexp = std::min(kFixedMaxExp, t.bias + 960);
       return;
     }
+  }
+}
+
+int fixed_lines_selftest(int nx, const double* D, const double* u, double* out, long n, bool split) {
+  LinesDev a{};
+  for (int k = 0; k < nx * nx; ++k) a.D[k] = D[k];
+  fixed_table(a.D, nx, a.fd);
+  switch (nx) {
+    case 3: return launch_lines<3>(a, u, out, n, split);
+    case 4: return launch_lines<4>(a, u, out, n, split);
+    case 5: return launch_lines<5>(a, u, out, n, split);
+    case 6: return launch_lines<6>(a, u, out, n, split);
+    case 7: return launch_lines<7>(a, u, out, n, split);
+    case 8: return launch_lines<8>(a, u, out, n, split);
+    case 9: return launch_lines<9>(a, u, out, n, split);
+    default: return NEKGPU_ERR_UNSUPPORTED;
   }
 }
 

@@ -2765,6 +2765,25 @@ int nekgpu_selftest_pair_join(const float* s, const float* t, double* out, long 
   return st;
 }
 
+int nekgpu_selftest_fixed_lines(int nx, const double* D, const double* u, double* out, long n, int split) {
+  if (!D || !u || !out || nx < 3 || nx > kMaxFixed || n < 1 || n > (1L << 24)) return NEKGPU_ERR_ARG;
+  int st = nekgpu_device_check(0);
+  if (st) return st;
+  const size_t bytes = (size_t)n * nx * sizeof(double);
+  double *du = nullptr, *dout = nullptr;
+  if (cudaMalloc(&du, bytes) != cudaSuccess || cudaMalloc(&dout, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(du), cudaFree(dout);
+    return NEKGPU_ERR_NOMEM;
+  }
+  if (check_cuda(cudaMemcpy(du, u, bytes, cudaMemcpyHostToDevice))) st = NEKGPU_ERR_CUDA;
+  if (!st) st = fixed_lines_selftest(nx, D, du, dout, n, split != 0);
+  if (!st && check_cuda(cudaMemcpy(out, dout, bytes, cudaMemcpyDeviceToHost))) st = NEKGPU_ERR_CUDA;
+  cudaFree(du);
+  cudaFree(dout);
+  return st;
+}
+
 int nekgpu_selftest_wait(nekgpu_ctx* c, int polls) {
   if (!c || polls < 1 || polls > (1 << 22)) return NEKGPU_ERR_ARG;
   c->last_launches = 0;

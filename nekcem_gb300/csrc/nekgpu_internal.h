@@ -214,15 +214,15 @@ __device__ inline void graphene_slot(const GrapheneDev& G, long g, const double 
 #endif
 
 // D in fixed point for the integer contractions of the FP64 kernels
-// (nekgpu_fixed.cuh): entry i + nx*l holds D(i,l) 2^kd = hi 2^31 + lo, hi8 =
-// 8 hi; bias = 1022 + kd.  ok = 0: D does not fit, contract in FP64.  Lines
+// (nekgpu_fixed.cuh): entry i + nx*l holds D(i,l) 2^kd = hi 2^31 + lo, |lo| <=
+// 2^30; bias = 1021 + kd.  ok = 0: D does not fit, contract in FP64.  Lines
 // whose largest biased exponent lies in [kFixedMinExp, maxexp) are contracted
 // in integers.
 constexpr int kMaxFixed = 9;
 constexpr int kFixedMinExp = 200, kFixedMaxExp = 2030;
 struct FixedD {
   int ok, bias, maxexp;
-  int hi[kMaxFixed * kMaxFixed], lo[kMaxFixed * kMaxFixed], hi8[kMaxFixed * kMaxFixed];
+  int hi[kMaxFixed * kMaxFixed], lo[kMaxFixed * kMaxFixed];
 };
 
 // Fused FP64 stage (nekgpu_fp64.cu): arguments as in FusedDev, with the
@@ -559,6 +559,9 @@ int fp64_stage(Context* c, int rkstep, double time, double dt);
 int fp64_stage_buffers(Context* c, int rkstep, double time, double dt, const double* u_in,
                        double* u_out, const double* k_in, double* k_out);
 void fixed_table(const double* D, int n, FixedD& t);
+// n lines of nx values contracted with D (entry i + nx*l) as the stage kernels
+// do, rows of D from the constant bank or (split) from shared memory
+int fixed_lines_selftest(int nx, const double* D, const double* u, double* out, long n, bool split);
 
 int num_sms(Context* c);
 

@@ -75,7 +75,7 @@ __constant__ const LineType kLine[2][6] = {
 // constant bank (all NX of them).
 template <int NX, bool SPLIT, typename Put>
 __device__ __forceinline__ void line_outputs(const double* pu, int step, int i0, int i1,
-                                             const FixedD& fd, const double* D, const int4* s_D,
+                                             const FixedD& fd, const double* D, const int2* s_D,
                                              Put put) {
   FixedLine<NX> f;
   {
@@ -88,19 +88,17 @@ __device__ __forceinline__ void line_outputs(const double* pu, int step, int i0,
     if (!SPLIT) {
 #pragma unroll
       for (int i = 0; i < NX; ++i)
-        put(i, fixed_dot<NX>(f, fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
+        put(i, fixed_dot<NX>(f, fd.bias, [&](int l, int& hi, int& lo) {
               hi = fd.hi[i + NX * l];
               lo = fd.lo[i + NX * l];
-              hi8 = fd.hi8[i + NX * l];
             }));
     } else {
 #pragma unroll 1
       for (int i = i0; i < i1; ++i)
-        put(i, fixed_dot<NX>(f, fd.bias, [&](int l, int& hi, int& lo, int& hi8) {
-              const int4 d = s_D[i + NX * l];
+        put(i, fixed_dot<NX>(f, fd.bias, [&](int l, int& hi, int& lo) {
+              const int2 d = s_D[i + NX * l];
               hi = d.x;
               lo = d.y;
-              hi8 = d.z;
             }));
     }
   } else {  // a line out of the integer form's range: in FP64
