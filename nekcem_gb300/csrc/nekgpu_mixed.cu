@@ -168,7 +168,8 @@ __host__ __device__ constexpr int slab_lo(int s) {
   return s >= S ? NX : (s * NX / S) & ~1;
 }
 
-template <int NX>
+// TPL: threads per line of an unsplit element (2: each takes a part of its outputs)
+template <int NX, int TPL = 1>
 struct MCfg {
   static constexpr int N2 = NX * NX, N3 = N2 * NX;
   // Node layout of the FP32 pair arrays.  NX = 8: unpadded, node
@@ -181,7 +182,7 @@ struct MCfg {
   static constexpr int SZ = RS * NX;
   static constexpr int N3P = NX * SZ;
   static constexpr int NF = 6 * N2;
-  static constexpr int NTASK = 4 * N2;  // line tasks per direction
+  static constexpr int NTASK = 4 * N2 * TPL;  // line tasks per direction
   static constexpr int NT = round32(cmax(NTASK, (N3 + 1) / 2));
   static constexpr int NW = NT / 32;
   static constexpr int NPT = (N3 + NT - 1) / NT;
@@ -212,7 +213,7 @@ struct MCfg {
   // in turn, the staged FP64 state (until the split), the partner face values
   // parked for the flux (FP64) and the residual pairs (hi, lo); the other the
   // split pairs (uh, ul), dead after the t-lines, so the next element's state
-  // can land there while this one is finished.  54 KB in all at NX=8, four
+  // can land there while this one is finished.  61 KB in all at NX=8, three
   // blocks per SM.
   static constexpr size_t SA = cmax(cmax(6 * N3 * 8, 6 * N3P * 8), 6 * NF * 8);
   static constexpr size_t off_F = 2 * SA;  // float2 flux pairs [face][line slot][N2]
@@ -459,23 +460,25 @@ __device__ __forceinline__ void line_outputs(const float2* u, float2* R0, float2
 // them (inverse mass, RK update) instead of storing the pairs.  S > 1: the
 // block's k-slab only -- r- and s-lines inside the slab, S threads on each
 // with the outputs of one part (part-major: warp-uniform at NX = 8), t-lines
-// with the slab's outputs.
-template <int NX, int DIR, bool FIN, int S>
+// with the slab's outputs.  TPL > 1: the whole element, TPL threads on every line.
+template <int NX, int DIR, bool FIN, int S, int TPL>
 __device__ __forceinline__ void line_phase(const float2* s_u2, float2* s_R2, const float2* s_F,
                                            bool cubic, float rh, float rl, const MixedDev& a,
                                            int e, bool first_stage, int slab) {
-  using C = MCfg<NX>;
+  using C = MCfg<NX, TPL>;
+  static_assert(TPL == 1 || (TPL == 2 && S == 1 && !FIN), "two threads per line: unsplit, no FIN");
+  constexpr int Q = S > 1 ? S : TPL;  // parts of a line's outputs
   const int tid = opaque_tid();
   const int k0 = S == 1 ? 0 : slab_lo<NX, S>(slab), k1 = S == 1 ? NX : slab_lo<NX, S>(slab + 1);
   const int nl = S > 1 && DIR < 2 ? NX * (k1 - k0) : C::N2;  // lines per component
-  const int ntask = 4 * nl * (DIR < 2 ? S : 1);
+  const int ntask = 4 * nl * (DIR < 2 ? S : 1) * TPL;
   constexpr int ROUNDS = S > 1 ? (4 * C::N2 * (DIR < 2 ? 2 : 1) + C::NT - 1) / C::NT : C::TPT;
 #pragma unroll
   for (int q = 0; q < ROUNDS; ++q) {
     const int task = tid + q * C::NT;
     if (task < ntask) {
-      const int part = S > 1 ? (DIR < 2 ? task / (4 * nl) : slab) : 0;
-      const int lt = S > 1 && DIR < 2 ? task - part * 4 * nl : task;
+      const int part = TPL > 1 || (S > 1 && DIR < 2) ? task / (4 * nl) : (S > 1 ? slab : 0);
+      const int lt = TPL > 1 || (S > 1 && DIR < 2) ? task - part * 4 * nl : task;
       const int slot = lt / nl, lam = lt - slot * nl + (S > 1 && DIR < 2 ? NX * k0 : 0);
       const int la = lam % NX, lb = lam / NX;
       const int comp = kLineComp[DIR][slot], rt = kLineRes[DIR][slot];
@@ -504,21 +507,21 @@ __device__ __forceinline__ void line_phase(const float2* s_u2, float2* s_R2, con
       for (int l = 0; l < NX; ++l) u[l] = pu[line_node<NX, DIR>(la, lb, l)];
       float2* R0 = s_R2 + rt * C::N3P;
       auto outputs = [&](auto p) {
-        constexpr int I0 = slab_lo<NX, S>(decltype(p)::value), NP = slab_lo<NX, S>(decltype(p)::value + 1) - I0;
+        constexpr int I0 = slab_lo<NX, Q>(decltype(p)::value), NP = slab_lo<NX, Q>(decltype(p)::value + 1) - I0;
         line_outputs<NX, DIR, FIN, I0, NP>(u, R0, flux_m, flux_p, cubic, rh, rl, sg, init, la, lb, rt,
                                            a, e, first_stage);
       };
-      if constexpr (S == 1) {
+      if constexpr (Q == 1) {
         outputs(std::integral_constant<int, 0>{});
-      } else if constexpr (S == 2) {
+      } else if constexpr (Q == 2) {
         if (part == 0) outputs(std::integral_constant<int, 0>{});
         else outputs(std::integral_constant<int, 1>{});
-      } else if constexpr (S == 3) {
+      } else if constexpr (Q == 3) {
         if (part == 0) outputs(std::integral_constant<int, 0>{});
         else if (part == 1) outputs(std::integral_constant<int, 1>{});
         else outputs(std::integral_constant<int, 2>{});
       } else {
-        static_assert(S == 4, "one to four slabs");
+        static_assert(Q == 4, "one to four parts");
         if (part == 0) outputs(std::integral_constant<int, 0>{});
         else if (part == 1) outputs(std::integral_constant<int, 1>{});
         else if (part == 2) outputs(std::integral_constant<int, 2>{});
@@ -647,10 +650,10 @@ __device__ __noinline__ void face_extras(const MixedDev& a, int e, int t, int f,
 // registers), six at NX = 6 (160 threads, 32 KB, 64 registers), two at NX = 9
 // (384 threads, 94 KB), three otherwise and with the extension branches
 // (two, with 128 registers and no spills, take 95 instead of 60 us per stage
-// on 8^3 elements with PML at N=8).
-template <int NX, int EXT, int S>
+// on 8^3 elements with PML at N=8); one with two threads per line.
+template <int NX, int EXT, int S, int TPL>
 constexpr int mixed_min_blocks() {
-  return NX == 9 ? 2 : (EXT || S > 1 ? 3 : (NX == 6 ? 6 : 3));
+  return TPL > 1 ? 1 : NX == 9 ? 2 : (EXT || S > 1 ? 3 : (NX == 6 ? 6 : 3));
 }
 
 // EXT: 0 plain, 1 with the PML and dispersive-current terms of the nodes, 2
@@ -658,10 +661,10 @@ constexpr int mixed_min_blocks() {
 // with few elements: every block stages and splits the whole element (the
 // t-lines need it) and works out the nodes of its slab, so the blocks share
 // nothing; the arithmetic of a node is the same.
-template <int NX, int EXT, int S>
-__global__ void __launch_bounds__(MCfg<NX>::NT, mixed_min_blocks<NX, EXT, S>())
+template <int NX, int EXT, int S, int TPL>
+__global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, S, TPL>())
     k_mixed_stage(const MixedDev a) {
-  using C = MCfg<NX>;
+  using C = MCfg<NX, TPL>;
   constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF, N3P = C::N3P;
   constexpr int NPT = C::NPT, FPT = C::FPT;
   constexpr bool FIN = EXT == 0 && C::kFin;  // the extension terms need all six at a node
@@ -950,13 +953,13 @@ __global__ void __launch_bounds__(MCfg<NX>::NT, mixed_min_blocks<NX, EXT, S>())
     {
       const bool cubic = eg[0] == 1.0f && eg[1] == 0.0f && eg[2] == 1.0f && eg[3] == 0.0f;
       const float r1h = eg[0], r1l = eg[1], r2h = eg[2], r2l = eg[3];
-      line_phase<NX, 0, false, S>(s_u2, s_R2, s_F, cubic, 0.0f, 0.0f, a, e, first_stage, slab);
+      line_phase<NX, 0, false, S, TPL>(s_u2, s_R2, s_F, cubic, 0.0f, 0.0f, a, e, first_stage, slab);
       __syncthreads();
-      line_phase<NX, 1, false, S>(s_u2, s_R2, s_F, cubic, r1h, r1l, a, e, first_stage, slab);
+      line_phase<NX, 1, false, S, TPL>(s_u2, s_R2, s_F, cubic, r1h, r1l, a, e, first_stage, slab);
       __syncthreads();
       // without the extension terms each component can finish on its own
       // (MCfg::kFin): H3, E3 (no t-derivative) are complete since the s-lines
-      line_phase<NX, 2, FIN, S>(s_u2, s_R2, s_F, cubic, r2h, r2l, a, e, first_stage, slab);
+      line_phase<NX, 2, FIN, S, TPL>(s_u2, s_R2, s_F, cubic, r2h, r2l, a, e, first_stage, slab);
     }
     if constexpr (FIN) {
       tid = opaque_tid();
@@ -1037,10 +1040,10 @@ __global__ void k_scale_coef_pairs(float2* coef, const double* base, long n2, do
   coef[i] = make_float2(d2f_hi(v), d2f_lo(v));
 }
 
-template <int NX, int EXT, int S>
+template <int NX, int EXT, int S, int TPL = 1>
 int launch_mixed(Context* c, const MixedDev& a, bool pdl) {
-  using C = MCfg<NX>;
-  auto kern = k_mixed_stage<NX, EXT, S>;
+  using C = MCfg<NX, TPL>;
+  auto kern = k_mixed_stage<NX, EXT, S, TPL>;
   static int grid = 0;
   if (!grid) {
     if (check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1071,22 +1074,40 @@ int launch_mixed(Context* c, const MixedDev& a, bool pdl) {
   return check_cuda(cudaGetLastError());
 }
 
-// Slabs per element (k_mixed_stage): the most slabs the order has, else two,
-// while the tasks stay within what the SMs take side by side without slowing
-// each other -- one per SM at N=7 and 8, more for smaller elements.  us per
-// stage, unsplit / two / most slabs: 64 elements N=7 9.4 / 7.0 / 9.1 (four),
-// 27 elements N=7 9.4 / 6.8 / 6.5, N=8 13.1 / 11.7 / 9.6, 100 elements N=6
-// 11.7 / 12.2 / 11.4 (three), N=5 9.1 / 8.9 / 6.8, 180 elements N=5 9.9 / 9.8
-// / 10.1, 294 elements N=3 8.6 / 9.5.
+// Slabs per element (k_mixed_stage) and threads per line, for meshes with few
+// elements: slabs while their blocks (elements times slabs) stay within what
+// the SMs take side by side without slowing each other.  us per stage on both
+// sides of each line, without / with PML (EXT 1):
+//   N=8  four slabs up to 38 elements: 9.5 against 11.7 in two, 13.4 unsplit /
+//        13.4 against 19.8, 22.9; two up to 76: 12.1 against 13.5 / 20.1
+//        against 23.3; unsplit from 77 on: 13.5 against 15.1 / 23.3, 23.0
+//   N=7  four up to 38: 7.1, 6.9, 9.3 / 9.6, 11.0, 16.5; two up to 114, three
+//        blocks on two SMs: 8.5 against 9.4 / 12.6, 17.0, above that 11.1
+//        against 9.5 / 14.6 to 17.4 against 17.1; then, up to one element per
+//        SM, unsplit with two threads per line: 8.9 against 9.5 / 15.3, 17.2;
+//        above one per SM 15.4 against 12.2 / 22.5, 19.4
+//   N=6  three up to 101, two blocks per SM: 9.7 against 11.4 at 76, 11.4, 11.5
+//        at 100 / 12.2, 16.0 and 16.0, 16.1; in two above that 12.0 to 14.3
+//        against 11.3 to 11.7
+//   N=5  three up to 152, three blocks per SM: 7.3 against 8.3 / 11.8, 12.7;
+//        in two above that 9.7 to 10.3 against 8.7 to 9.7 / 13.7 to 16.2
+//        against 14.1 to 14.7
+//   N=4  two up to 152, two blocks per SM: 7.4 against 8.0, at 200 elements 9.2
+//        against 8.2; unsplit with PML: 9.3 against 9.2 at 64, 10.7, 9.4 at 150
+//   N=3  two up to 456, six blocks per SM: 6.1 against 6.7; with PML up to 228:
+//        7.9 against 8.6, at 400 elements 9.3 against 8.8
 template <int NX, int EXT>
 int launch_mixed_split(Context* c, const MixedDev& a, bool pdl) {
-  constexpr int SM = EXT == 2 ? 1 : (NX >= 8 ? 4 : (NX >= 6 ? 3 : (NX >= 4 ? 2 : 1)));
-  constexpr int kPerSm = NX >= 8 ? 1 : (NX == 7 ? 2 : (NX == 3 ? 6 : 3));
-  const int n = a.e_end - a.e_begin, room = kPerSm * num_sms(c);
-  if constexpr (SM > 2)
-    if (n * SM <= room) return launch_mixed<NX, EXT, SM>(c, a, pdl);
+  constexpr int SM =
+      EXT == 2 ? 1 : (NX >= 8 ? 4 : (NX >= 6 ? 3 : (NX == 4 || (NX == 5 && EXT == 0) ? 2 : 1)));
+  constexpr int kPerSm = NX >= 8 ? 1 : (NX == 7 || NX == 5 ? 2 : (NX == 6 || EXT ? 3 : 6));
+  const int n = a.e_end - a.e_begin, sms = num_sms(c);
   if constexpr (SM > 1)
-    if (n * 2 <= room) return launch_mixed<NX, EXT, 2>(c, a, pdl);
+    if (n * SM <= kPerSm * sms) return launch_mixed<NX, EXT, SM>(c, a, pdl);
+  if constexpr (SM == 4)
+    if (4 * n <= (NX == 8 ? 3 : 2) * sms) return launch_mixed<NX, EXT, 2>(c, a, pdl);
+  if constexpr (NX == 8 && EXT < 2)
+    if (n <= sms) return launch_mixed<NX, EXT, 1, 2>(c, a, pdl);
   return launch_mixed<NX, EXT, 1>(c, a, pdl);
 }
 
