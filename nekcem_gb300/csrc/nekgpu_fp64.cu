@@ -253,60 +253,31 @@ __device__ __forceinline__ void disp_node(const Fp64Dev& a, int l, int v, const 
   }
 }
 
-// Incident field (userinc) and graphene sheet (userfsrc) terms of face node t
-// of element e in its jumps JH, JE.
-template <int NX>
-__device__ __noinline__ void face_extras(const Fp64Dev& a, int e, int t, int f, int pe,
-                                         const double* h, const double* ev, const double* hp,
-                                         const double* ep, bool first_stage, double* JH, double* JE) {
-  constexpr int NF = DCfg<NX>::NF;
-  double hm[3], em[3], hq[3], eq[3];
-  for (int c = 0; c < 3; ++c) {
-    hm[c] = h[c];
-    em[c] = ev[c];
-    hq[c] = hp[c];
-    eq[c] = ep[c];
-  }
-  const int io = a.inc_elem ? a.inc_elem[e] : -1;
-  if (io >= 0) {
-    // the incident field on the own side of a listed face node, or on the
-    // partner's side when the partner's slot is listed
-    const double* iv = a.inc_val + (long)io * 12 * NF + t;
-    for (int c = 0; c < 3; ++c) {
-      hm[c] += iv[c * NF];
-      em[c] += iv[(3 + c) * NF];
-      hq[c] += iv[(6 + c) * NF];
-      eq[c] += iv[(9 + c) * NF];
-    }
-  }
-  for (int c = 0; c < 3; ++c) {
-    JH[c] = pe >= 0 ? hq[c] - hm[c] : 0.0;
-    JE[c] = pe >= 0 ? eq[c] - em[c] : -2.0 * em[c];
-  }
-  if (!a.gr.elem) return;
-  // the sheet's currents on both sides of the face node enter as
-  // n x [H] - J, i.e. [H] + n x J
-  const int gr = a.gr.elem[e];
-  const int go = gr >= 0 ? a.gr.own[(long)gr * NF + t] : -1;
-  const int gp = gr >= 0 ? a.gr.part[(long)gr * NF + t] : -1;
-  if (go < 0 && gp < 0) return;
+// Graphene sheet (userfsrc) at a face node of slot f: n x J with the currents J
+// of the own (go) and the partner's (gp) listed slot, which the sheet adds to
+// [H] (n x [H] - J), from the fields h, ev here and hp, ep there (the incident
+// field included).  A PEC face keeps its mirror flux.
+__device__ __noinline__ double3 sheet_jump(const Fp64Dev& a, int f, int pe, int go, int gp, double3 h,
+                                           double3 ev, double3 hp, double3 ep, bool first_stage) {
   double nv[3], nm[3], J[3] = {0.0, 0.0, 0.0};
+  const double hm[3] = {h.x, h.y, h.z}, em[3] = {ev.x, ev.y, ev.z};
+  const double hq[3] = {hp.x, hp.y, hp.z}, eq[3] = {ep.x, ep.y, ep.z};
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
     nv[c] = c == slot_axis(f) ? (double)slot_side(f) : 0.0;
     nm[c] = -nv[c];
   }
   if (go >= 0) graphene_slot(a.gr, go, nv, hm, em, true, first_stage, a.a, a.b, a.dt, J);
   if (gp >= 0 && pe >= 0) graphene_slot(a.gr, gp, nm, hq, eq, false, first_stage, a.a, a.b, a.dt, J);
-  if (pe >= 0) {  // a PEC face keeps its mirror flux
-    JH[0] += nv[1] * J[2] - nv[2] * J[1];
-    JH[1] += nv[2] * J[0] - nv[0] * J[2];
-    JH[2] += nv[0] * J[1] - nv[1] * J[0];
-  }
+  if (pe < 0) return make_double3(0.0, 0.0, 0.0);
+  return make_double3(nv[1] * J[2] - nv[2] * J[1], nv[2] * J[0] - nv[0] * J[2],
+                      nv[0] * J[1] - nv[1] * J[0]);
 }
 
-// Blocks per SM the launch is built for.  EXT 1 at N=4: four blocks of 96
-// threads (168 registers; 336 elements with PML 19.8 us per stage, 1000 32.1;
-// built for two the compiler takes 204 registers, three blocks: 25.5 and 50.4).
+// Blocks per SM the launch is built for.  EXT 1 at N=4: four blocks of 128
+// threads (128 registers; built for two the compiler takes 204: 336 elements
+// with PML 25.5 us per stage with 96 threads, 19.8 built for four, 18.4 with 128
+// threads; 1000 elements 50.4, 32.0, 29.0).
 template <int NX, int EXT>
 constexpr int fp64_min_blocks() {
   return EXT == 1 && NX == 5 ? 4 : (NX == 9 || EXT ? 2 : (NX == 8 ? 3 : 4));
@@ -335,7 +306,7 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
   for (int w = blockIdx.x; w < ntask; w += gridDim.x) {
     if (w + (int)gridDim.x >= ntask) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const int q0 = SPLIT ? w / nsplit : w;
-    const int e = EXT > 0 && a.pml.order ? a.pml.order[q0] : q0;  // (PML elements first)
+    const int e = EXT == 1 && a.pml.order ? a.pml.order[q0] : q0;  // (see PmlDev::order)
     Slab sl{0, NX};
     if (SPLIT) {
       const int q = w - q0 * nsplit;
@@ -354,7 +325,7 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
     // what the finish reads, and the next element's state, on their way to L2
     if (!SPLIT) {
       const int wn = w + (int)gridDim.x;
-      const int en = wn < ntask ? (EXT > 0 && a.pml.order ? a.pml.order[wn] : wn) : e;
+      const int en = wn < ntask ? (EXT == 1 && a.pml.order ? a.pml.order[wn] : wn) : e;
 #pragma unroll 1
       for (int t = tid; t < 14 * ((N3 + 15) / 16); t += NT) {
         const int q = t / ((N3 + 15) / 16), o = 16 * (t - q * ((N3 + 15) / 16));
@@ -382,6 +353,9 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // ---- upwind flux per face node, lifted, into s_F ---------------------------
+    // rows of the listed elements in the incident field's and the sheets' tables
+    const int io = EXT == 2 && a.inc_elem ? a.inc_elem[e] : -1;
+    const int gr = EXT == 2 && a.gr.elem ? a.gr.elem[e] : -1;
 #pragma unroll
     for (int q = 0; q < C::FPT; ++q) {
       const int t = tid + q * NT;
@@ -397,27 +371,40 @@ __global__ void __launch_bounds__(DCfg<NX>::NT, fp64_min_blocks<NX, EXT>())
       const int ta = ax == 0 ? 1 : 0, tb = ax == 2 ? 1 : 2;
       double JHa, JHb, JEa, JEb;
       if (EXT == 2) {
-        double h[3], ev[3], JH[3], JE[3];
+        double h[3], ev[3], hp[3], ep[3], JH[3], JE[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           h[c] = s_u[c * C::N3P + pv];
           ev[c] = s_u[(3 + c) * C::N3P + pv];
-          JH[c] = pe >= 0 ? nbv[q][c] - h[c] : 0.0;
-          JE[c] = pe >= 0 ? nbv[q][EXT == 2 ? 3 + c : 0] - ev[c] : -2.0 * ev[c];
+          hp[c] = pe >= 0 ? nbv[q][c] : 0.0;
+          ep[c] = pe >= 0 ? nbv[q][EXT == 2 ? 3 + c : 0] : 0.0;
         }
-        if (a.inc_elem || a.gr.elem) {
-          double hp[3], ep[3];
+        // userinc: the incident field on the own side of a listed face node, or
+        // on the partner's side when the partner's slot is listed
+        if (io >= 0) {
+          const double* iv = a.inc_val + (long)io * 12 * NF + j;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            hp[c] = pe >= 0 ? nbv[q][c] : 0.0;
-            ep[c] = pe >= 0 ? nbv[q][EXT == 2 ? 3 + c : 0] : 0.0;
+            h[c] += iv[c * NF];
+            ev[c] += iv[(3 + c) * NF];
+            hp[c] += iv[(6 + c) * NF];
+            ep[c] += iv[(9 + c) * NF];
           }
-          double jh[3], je[3];
-          face_extras<NX>(a, e, j, f, pe, h, ev, hp, ep, first_stage, jh, je);
+        }
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            JH[c] = jh[c];
-            JE[c] = je[c];
+        for (int c = 0; c < 3; ++c) {
+          JH[c] = pe >= 0 ? hp[c] - h[c] : 0.0;
+          JE[c] = pe >= 0 ? ep[c] - ev[c] : -2.0 * ev[c];
+        }
+        if (gr >= 0) {
+          const int go = a.gr.own[(long)gr * NF + j], gp = a.gr.part[(long)gr * NF + j];
+          if (go >= 0 || gp >= 0) {
+            const double3 d = sheet_jump(a, f, pe, go, gp, make_double3(h[0], h[1], h[2]),
+                                         make_double3(ev[0], ev[1], ev[2]), make_double3(hp[0], hp[1], hp[2]),
+                                         make_double3(ep[0], ep[1], ep[2]), first_stage);
+            JH[0] += d.x;
+            JH[1] += d.y;
+            JH[2] += d.z;
           }
         }
         JHa = ax == 0 ? JH[1] : JH[0];

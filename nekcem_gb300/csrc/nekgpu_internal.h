@@ -146,7 +146,7 @@ struct PlainDev {
 constexpr int kPmlData = 16;
 struct PmlDev {
   const int* slot;        // nelt: PML slot of the element, -1 outside
-  const int* order;       // nelt: the PML elements, then the others (see upload_pml_fused)
+  const int* order;       // nelt: the PML elements, then the others; read by EXT 1 (see upload_pml_fused)
   const double* data;     // kPmlData * n
   double* aux;            // 6 * n: pmlbn, pmldn
   double* k;              // 6 * n: their RK registers

@@ -44,7 +44,11 @@ struct ElemCfg {
   // lines in every direction are read with at most two threads of a half warp
   // on a bank
   static constexpr int RS = NX | 1, SZ = RS * NX, N3P = NX * SZ;
-  static constexpr int NT = NX == 9 ? 384 : (NX == 8 ? 256 : round32(cmax(3 * N2, (N3 + 1) / 2)));
+  // threads per block: half a node each, at NX = 5 a whole one (with 96 threads
+  // the 125 nodes and 150 lines took a second, nearly empty turn: 336 elements
+  // 11.7 against 10.4 us per stage, 1000 20.7 against 17.9, with incident field
+  // and PML 128 elements 37.4 against 27.2)
+  static constexpr int NT = NX == 9 ? 384 : (NX == 8 ? 256 : (NX == 5 ? 128 : round32(cmax(3 * N2, (N3 + 1) / 2))));
   static constexpr int FPT = (NF + NT - 1) / NT;
 };
 

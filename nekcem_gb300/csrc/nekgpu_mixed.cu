@@ -600,49 +600,39 @@ __device__ __forceinline__ void disp_node(const MixedDev& a, int l, int v, long 
   }
 }
 
-// Incident field (userinc) and graphene sheet (userfsrc) terms of face node t
-// of element e added to its jumps JH, JE (FP64 differences; listed elements
-// only): the incident field on the own side of a listed face node, or on the
-// partner's side when the partner's slot is listed; the sheet's currents on
-// both sides as n x [H] - J, i.e. [H] + n x J.
-template <int NF>
-__device__ __noinline__ void face_extras(const MixedDev& a, int e, int t, int f, int pe, double* hm,
-                                         double* em, double* hp, double* ep, bool first_stage,
-                                         float2* JH, float2* JE) {
-  const int io = a.inc_elem ? a.inc_elem[e] : -1;
-  if (io >= 0) {
-    const double* iv = a.inc_val + (long)io * 12 * NF + t;
-    for (int c = 0; c < 3; ++c) {
-      const double ho = iv[c * NF], eo = iv[(3 + c) * NF], hq = iv[(6 + c) * NF], eq = iv[(9 + c) * NF];
-      if (pe >= 0) {
-        add_jump(JH[c], hq - ho);
-        add_jump(JE[c], eq - eo);
-      } else {
-        add_jump(JE[c], -2.0 * eo);
-      }
-      hm[c] += ho;
-      em[c] += eo;
-      hp[c] += hq;
-      ep[c] += eq;
-    }
-  }
-  if (!a.gr.elem) return;
-  const int gr = a.gr.elem[e];
-  const int go = gr >= 0 ? a.gr.own[(long)gr * NF + t] : -1;
-  const int gp = gr >= 0 ? a.gr.part[(long)gr * NF + t] : -1;
-  if (go < 0 && gp < 0) return;
-  double nv[3], nm[3], J[3] = {0.0, 0.0, 0.0};
+// Graphene sheet (userfsrc) at face node t of slot f, from the FP64 fields of
+// both sides (the incident field included, row io of its table): n x J with
+// the currents J of the own (go) and the partner's (gp) listed slot, which the
+// sheet adds to [H] (n x [H] - J).  A PEC face keeps its mirror flux.
+template <int NX>
+__device__ __forceinline__ double3 sheet_jump(const MixedDev& a, const float2* s_u2, const double* s_nbv,
+                                           int t, int pv, int f, int pe, int io, int go, int gp,
+                                           bool first_stage) {
+  using C = MCfg<NX>;
+  constexpr int NF = C::NF;
+  double hm[3], em[3], hp[3], ep[3], nv[3], nm[3], J[3] = {0.0, 0.0, 0.0};
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
+    const float2 h = s_u2[c * C::N3P + pv], ev = s_u2[(c + 3) * C::N3P + pv];
+    hm[c] = f2d(h.x) + f2d(h.y);
+    em[c] = f2d(ev.x) + f2d(ev.y);
+    hp[c] = pe >= 0 ? s_nbv[c * NF + t] : 0.0;
+    ep[c] = pe >= 0 ? s_nbv[(c + 3) * NF + t] : 0.0;
+    if (io >= 0) {
+      const double* iv = a.inc_val + (long)io * 12 * NF + t;
+      hm[c] += iv[c * NF];
+      em[c] += iv[(3 + c) * NF];
+      hp[c] += iv[(6 + c) * NF];
+      ep[c] += iv[(9 + c) * NF];
+    }
     nv[c] = c == slot_axis(f) ? (double)slot_side(f) : 0.0;
     nm[c] = -nv[c];
   }
   if (go >= 0) graphene_slot(a.gr, go, nv, hm, em, true, first_stage, a.a, a.b, a.dt, J);
   if (gp >= 0 && pe >= 0) graphene_slot(a.gr, gp, nm, hp, ep, false, first_stage, a.a, a.b, a.dt, J);
-  if (pe >= 0) {  // a PEC face keeps its mirror flux
-    add_jump(JH[0], nv[1] * J[2] - nv[2] * J[1]);
-    add_jump(JH[1], nv[2] * J[0] - nv[0] * J[2]);
-    add_jump(JH[2], nv[0] * J[1] - nv[1] * J[0]);
-  }
+  if (pe < 0) return make_double3(0.0, 0.0, 0.0);
+  return make_double3(nv[1] * J[2] - nv[2] * J[1], nv[2] * J[0] - nv[0] * J[2],
+                      nv[0] * J[1] - nv[1] * J[0]);
 }
 
 // Blocks per SM the launch is built for: three at NX = 8 (62 KB of shared
@@ -724,7 +714,7 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, S
   unsigned parity = 0;
   int buf = 0;  // area of the element's staged state and residual pairs
   // tasks: element w/S (with PML, of that mesh's order), slab w%S
-  auto element = [&](int w) { return EXT > 0 && a.pml.order ? a.pml.order[w / S] : w / S; };
+  auto element = [&](int w) { return EXT == 1 && a.pml.order ? a.pml.order[w / S] : w / S; };
   const int w0 = a.e_begin * S + (int)blockIdx.x, w1 = a.e_end * S;
   if (C::kTma && tid == 0 && w0 < w1) issue_tma(EXT == 0 ? w0 / S : element(w0), 0);
   if (C::kAsync && w0 < w1) issue_async(EXT == 0 ? w0 / S : element(w0), 0, tid);
@@ -846,6 +836,9 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, S
     // reads back only what it wrote) to keep the flux's registers free.
     tid = opaque_tid();
     double* s_nbv = s_u64;
+    // rows of the listed elements in the incident field's and the sheets' tables
+    const int io = EXT == 2 && a.inc_elem ? a.inc_elem[e] : -1;
+    const int gr = EXT == 2 && a.gr.elem ? a.gr.elem[e] : -1;
 #pragma unroll
     for (int q = 0; q < FPT; ++q) {
       const int t = face_task(tid, q);
@@ -879,27 +872,27 @@ __global__ void __launch_bounds__(MCfg<NX, TPL>::NT, mixed_min_blocks<NX, EXT, S
             JE[c] = make_float2(-2.0f * ev.x, -2.0f * ev.y);
           }
         }
-        if (EXT == 2 && (a.inc_elem || a.gr.elem)) {
-          double hm[3], em[3], hp[3], ep[3];
+        // userinc: the incident field on the own side of a listed face node, or
+        // on the partner's side when the partner's slot is listed
+        if (EXT == 2 && io >= 0) {
+          const double* iv = a.inc_val + (long)io * 12 * NF + t;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const float2 h = s_u2[c * N3P + pv], ev = s_u2[(c + 3) * N3P + pv];
-            hm[c] = f2d(h.x) + f2d(h.y);
-            em[c] = f2d(ev.x) + f2d(ev.y);
-            hp[c] = pe >= 0 ? s_nbv[c * NF + t] : 0.0;
-            ep[c] = pe >= 0 ? s_nbv[(EXT == 2 ? c + 3 : 0) * NF + t] : 0.0;
+            if (pe >= 0) {
+              add_jump(JH[c], iv[(6 + c) * NF] - iv[c * NF]);
+              add_jump(JE[c], iv[(9 + c) * NF] - iv[(3 + c) * NF]);
+            } else {
+              add_jump(JE[c], -2.0 * iv[(3 + c) * NF]);
+            }
           }
-          float2 jh[3], je[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            jh[c] = JH[c];
-            je[c] = JE[c];
-          }
-          face_extras<NF>(a, e, t, f, pe, hm, em, hp, ep, first_stage, jh, je);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            JH[c] = jh[c];
-            JE[c] = je[c];
+        }
+        if (EXT == 2 && gr >= 0) {
+          const int go = a.gr.own[(long)gr * NF + t], gp = a.gr.part[(long)gr * NF + t];
+          if (go >= 0 || gp >= 0) {
+            const double3 d = sheet_jump<NX>(a, s_u2, s_nbv, t, pv, f, pe, io, go, gp, first_stage);
+            add_jump(JH[0], d.x);
+            add_jump(JH[1], d.y);
+            add_jump(JH[2], d.z);
           }
         }
         // coefficient pairs Y02, C02Y, Z02, C02Z (hi in the first float4 of
