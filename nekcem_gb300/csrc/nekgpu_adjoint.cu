@@ -77,9 +77,12 @@ __device__ __forceinline__ double pdbl(P2 a) {
   return pair_to_double(s, t);
 }
 
-template <int NX>
+// WIDE: a thread per node, line and face node (dispatch_adjoint)
+template <int NX, bool WIDE>
 struct ACfg : ElemCfg<NX> {
   using E = ElemCfg<NX>;
+  static constexpr int NT = WIDE ? round32(cmax(E::N3, E::NF)) : E::NT;
+  static constexpr int FPT = (E::NF + NT - 1) / NT;
   // weights w; ub, completed in place; products of two GLL weights: 56 KB at
   // N=7, four blocks per SM
   static constexpr size_t off_R = 6 * (size_t)E::N3P * 8, off_w = 2 * off_R;
@@ -88,13 +91,13 @@ struct ACfg : ElemCfg<NX> {
 
 // Phase PH of the transposed curl: every line adds its outputs, times the
 // line's factor metric * w * w, to ub.
-template <int NX, int PH>
+template <int NX, int PH, int NT>
 __device__ __forceinline__ void adjoint_lines(const double* s_w, double* s_R, const double* s_ww,
                                               const double* eg, const AdjointDev& a) {
   using C = ElemCfg<NX>;
   constexpr int N2 = C::N2;
 #pragma unroll 1
-  for (int task = threadIdx.x; task < 6 * N2; task += C::NT) {
+  for (int task = threadIdx.x; task < 6 * N2; task += NT) {
     const int type = task / N2, lam = task - type * N2;
     const LineType& lt = kLine[PH][type];
     const int dir = lt.dir, la = lam % NX, lb = lam / NX;
@@ -107,15 +110,15 @@ __device__ __forceinline__ void adjoint_lines(const double* s_w, double* s_R, co
   }
 }
 
-template <int NX>
+template <int NX, bool WIDE>
 constexpr int adjoint_min_blocks() {
-  return NX == 9 ? 2 : 4;
+  return WIDE ? 1 : (NX == 9 ? 2 : 4);
 }
 
-template <int NX>
-__global__ void __launch_bounds__(ACfg<NX>::NT, adjoint_min_blocks<NX>())
+template <int NX, bool WIDE>
+__global__ void __launch_bounds__(ACfg<NX, WIDE>::NT, adjoint_min_blocks<NX, WIDE>())
     k_adjoint_stage(const __grid_constant__ AdjointDev a) {
-  using C = ACfg<NX>;
+  using C = ACfg<NX, WIDE>;
   constexpr int N2 = C::N2, N3 = C::N3, NT = C::NT, NF = C::NF, N3P = C::N3P;
   extern __shared__ __align__(16) unsigned char smem[];
   double* s_w = reinterpret_cast<double*>(smem);
@@ -246,9 +249,9 @@ __global__ void __launch_bounds__(ACfg<NX>::NT, adjoint_min_blocks<NX>())
     face_deps(1);
     __syncthreads();
     face_deps(2);
-    adjoint_lines<NX, 0>(s_w, s_R, s_ww, eg, a);
+    adjoint_lines<NX, 0, NT>(s_w, s_R, s_ww, eg, a);
     __syncthreads();
-    adjoint_lines<NX, 1>(s_w, s_R, s_ww, eg, a);
+    adjoint_lines<NX, 1, NT>(s_w, s_R, s_ww, eg, a);
     __syncthreads();
     if (e + (int)gridDim.x >= a.nelt) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     // ---- updates of ub, w and deps, node by node --------------------------------
@@ -308,10 +311,10 @@ __global__ void __launch_bounds__(kSeedThreads)
   if (threadIdx.x == 0) partial[blockIdx.x] = s_sum[0];
 }
 
-template <int NX>
+template <int NX, bool WIDE>
 int launch_adjoint(Context* c, const AdjointDev& a) {
-  using C = ACfg<NX>;
-  auto kern = k_adjoint_stage<NX>;
+  using C = ACfg<NX, WIDE>;
+  auto kern = k_adjoint_stage<NX, WIDE>;
   static bool ready = false;
   static int grid = 0;
   if (!ready) {
@@ -342,17 +345,37 @@ int launch_adjoint(Context* c, const AdjointDev& a) {
   return check_cuda(cudaGetLastError());
 }
 
+
+// Wide blocks take one turn where the others take two or three, which a stage
+// of few elements waits for: up to one element per SM, at N=5 three, at N <= 4
+// always.  us per reverse stage with the recomputation in mixed stages, wide /
+// not (a thread per node and contraction before: last): N=7 8 elements 15.1 /
+// 18.8 (19.4), 64 15.9 / 21.5 (20.2), 152 22.0 / 28.9 (25.9), 300 39.8 / 41.1
+// (43.5), 336 46.8 / 43.3 (53.2); N=6 64 15.9 / 20.1 (17.1), 336 38.6 / 34.0
+// (41.2); N=5 64 11.5 / 16.1 (14.1), 336 23.2 / 26.4 (28.8), 608 34.0 / 34.2
+// (40.0), 700 40.6 / 36.0 (47.4); N=4 64 11.3 / 13.3 (14.0), 2000 66.5 / 72.0
+// (85.3).
+template <int NX>
+int dispatch_adjoint(Context* c, const AdjointDev& a) {
+  if constexpr (NX <= 5) {
+    return launch_adjoint<NX, true>(c, a);
+  } else {
+    return c->nelt <= (NX == 6 ? 3 : 1) * num_sms(c) ? launch_adjoint<NX, true>(c, a)
+                                                     : launch_adjoint<NX, false>(c, a);
+  }
+}
+
 }  // namespace
 
 int adjoint_stage(Context* c, const AdjointDev& a) {
   switch (c->nx) {
-    case 3: return launch_adjoint<3>(c, a);
-    case 4: return launch_adjoint<4>(c, a);
-    case 5: return launch_adjoint<5>(c, a);
-    case 6: return launch_adjoint<6>(c, a);
-    case 7: return launch_adjoint<7>(c, a);
-    case 8: return launch_adjoint<8>(c, a);
-    case 9: return launch_adjoint<9>(c, a);
+    case 3: return dispatch_adjoint<3>(c, a);
+    case 4: return dispatch_adjoint<4>(c, a);
+    case 5: return dispatch_adjoint<5>(c, a);
+    case 6: return dispatch_adjoint<6>(c, a);
+    case 7: return dispatch_adjoint<7>(c, a);
+    case 8: return dispatch_adjoint<8>(c, a);
+    case 9: return dispatch_adjoint<9>(c, a);
     default: return NEKGPU_ERR_UNSUPPORTED;
   }
 }
