@@ -1089,12 +1089,17 @@ int launch_mixed(Context* c, const MixedDev& a, bool pdl) {
 //        against 8.2; unsplit with PML: 9.3 against 9.2 at 64, 10.7, 9.4 at 150
 //   N=3  two up to 456, six blocks per SM: 6.1 against 6.7; with PML up to 228:
 //        7.9 against 8.6, at 400 elements 9.3 against 8.8
+// A part of a mesh (a chunk of the host-field step, other chunks beside it) is
+// not split at N=6 and N=8: us per host-field step, split / unsplit, 512
+// elements N=6 308 / 287, N=8 393 / 384, but N=7 275 / 290, N=5 218 / 229, N=4
+// 201 / 209, N=3 169 / 183.
 template <int NX, int EXT>
 int launch_mixed_split(Context* c, const MixedDev& a, bool pdl) {
   constexpr int SM =
       EXT == 2 ? 1 : (NX >= 8 ? 4 : (NX >= 6 ? 3 : (NX == 4 || (NX == 5 && EXT == 0) ? 2 : 1)));
   constexpr int kPerSm = NX >= 8 ? 1 : (NX == 7 || NX == 5 ? 2 : (NX == 6 || EXT ? 3 : 6));
   const int n = a.e_end - a.e_begin, sms = num_sms(c);
+  if ((NX == 7 || NX == 9) && n < c->nelt) return launch_mixed<NX, EXT, 1>(c, a, pdl);
   if constexpr (SM > 1)
     if (n * SM <= kPerSm * sms) return launch_mixed<NX, EXT, SM>(c, a, pdl);
   if constexpr (SM == 4)
