@@ -891,6 +891,7 @@ int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
   const long npml = (long)p.elems.size(), nn = npml * n3;
   std::vector<int> slot(c->nelt, -1);
   std::vector<double> d((size_t)kPmlData * nn);
+  c->host_pml_sigma.resize(3 * (size_t)nn);
   for (long l = 0; l < npml; ++l) {
     const long e = p.elems[l];
     slot[e] = (int)l;
@@ -905,7 +906,7 @@ int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
         d[(3 + ax) * nn + q] = nrm * (s0 - s1);
         d[(6 + ax) * nn + q] = nrm * (sig2 / p.eps[j] * p.mu[j]);
         d[(9 + ax) * nn + q] = nrm * sig2;
-        d[(13 + ax) * nn + q] = p.sigma[j + ax * npts];
+        c->host_pml_sigma[ax * nn + q] = p.sigma[j + ax * npts];
       }
       d[12 * nn + q] = cp.w3[v] * cp.egeom[9 * e] / cp.bm1[j];
     }
@@ -2043,16 +2044,15 @@ int nekgpu_get_array(nekgpu_ctx* c, const char* name, double* out) {
     return check_cuda(cudaMemcpy(out, src, 3 * P * sizeof(double), cudaMemcpyDeviceToHost));
   }
   const long nn = (long)c->npml * n3;
-  std::vector<double> h(sg ? (size_t)kPmlData * nn : 6 * (size_t)nn);
-  const double* src = sg ? c->d_pml_data : c->d_pml_aux;
-  if (check_cuda(cudaMemcpy(h.data(), src, h.size() * sizeof(double), cudaMemcpyDeviceToHost)))
+  std::vector<double> h(sg ? 0 : 6 * (size_t)nn);
+  if (!sg && check_cuda(cudaMemcpy(h.data(), c->d_pml_aux, h.size() * sizeof(double), cudaMemcpyDeviceToHost)))
     return NEKGPU_ERR_CUDA;
   for (long l = 0; l < c->npml; ++l)
     for (long v = 0; v < n3; ++v) {
       const long q = l * n3 + v, g = (long)c->pml_elems[l] * n3 + v;
       for (int cc = 0; cc < 3; ++cc) {
         if (sg)
-          out[cc * P + g] = h[(13 + cc) * nn + q];
+          out[cc * P + g] = c->host_pml_sigma[cc * nn + q];
         else
           out[cc * P + g] = h[((dn ? 3 : 0) + cc) * nn + q];
       }

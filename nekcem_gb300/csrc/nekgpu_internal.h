@@ -142,8 +142,8 @@ struct PlainDev {
 //   df/dt = res/bm1 - s1 f,   res += bm1 ((s0 - s1) f - s2 mu H | - sigma_2 E).
 // Per node of a PML element, [q][l*N3 + v]: q = 0..2 s1; with the residual
 // R = res/(w3 rx) and n = bm1/(w3 rx), 3..5 n (s0 - s1), 6..8 n s2 mu, 9..11
-// n sigma_2, 12 1/n; 13..15 sigma along x, y, z (read back by the host only).
-constexpr int kPmlData = 16;
+// n sigma_2, 12 1/n.
+constexpr int kPmlData = 13;
 struct PmlDev {
   const int* slot;        // nelt: PML slot of the element, -1 outside
   const int* order;       // nelt: the PML elements, then the others; read by EXT 1 (see upload_pml_fused)
@@ -469,6 +469,7 @@ struct Context {
   double *d_pml_sigma = nullptr, *d_eps = nullptr, *d_mu = nullptr, *d_pml_res = nullptr;
   int* d_pmlptr = nullptr;
   double *d_pml_aux = nullptr, *d_pml_k = nullptr, *d_pml_data = nullptr;
+  std::vector<double> host_pml_sigma;  // fused forms: sigma along x, y, z of the PML nodes, read back
   int* d_pml_slot = nullptr;
   // dispersive currents: per node model (0 none, 1 Drude, 2 Lorentz) and
   // parameters a, b, c on the host; the device side in DispDev (all forms)
