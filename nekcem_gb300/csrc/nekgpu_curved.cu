@@ -28,10 +28,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 
-#include "nekgpu_fixed.cuh"
 #include "nekgpu_internal.h"
+#include "nekgpu_lines.cuh"
 
 namespace nekgpu {
 
@@ -40,14 +39,11 @@ namespace {
 template <int NX>
 __device__ __forceinline__ void face_node(int f, int a, int b, int& i, int& j, int& k) {
   // slot order s=-1, r=+1, s=+1, r=-1, t=-1, t=+1 (pff)
-  const int ax = f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2);
-  const int fix = f == 0 || f == 3 || f == 4 ? 0 : NX - 1;
+  const int ax = slot_axis(f), fix = slot_side(f) < 0 ? 0 : NX - 1;
   i = ax == 0 ? fix : a;
   j = ax == 1 ? fix : (ax == 0 ? a : b);
   k = ax == 2 ? fix : b;
 }
-
-constexpr int round32(int a) { return (a + 31) / 32 * 32; }
 
 template <int NX>
 struct KCfg {
@@ -68,29 +64,8 @@ __device__ __forceinline__ void curved_lines(const double* s_u, double* s_d, con
   const int base = c * C::N3P + (DIR == 0 ? C::RS * la + C::SZ * lb
                                           : (DIR == 1 ? la + C::SZ * lb : la + C::RS * lb));
   constexpr int step = DIR == 0 ? 1 : (DIR == 1 ? C::RS : C::SZ);
-  FixedLine<NX> f;
-  {
-    double u[NX];
-#pragma unroll
-    for (int l = 0; l < NX; ++l) u[l] = s_u[base + step * l];
-    fixed_line<NX>(u, a.fd.maxexp, f);
-  }
-  if (a.fd.ok && !f.special) {
-#pragma unroll
-    for (int i = 0; i < NX; ++i)
-      s_d[base + step * i] = fixed_dot<NX>(f, a.fd.bias, [&](int l, int& hi, int& lo) {
-        hi = a.fd.hi[i + NX * l];
-        lo = a.fd.lo[i + NX * l];
-      });
-  } else {  // a line out of the integer form's range: in FP64
-#pragma unroll 1
-    for (int i = 0; i < NX; ++i) {
-      double x = a.D[i] * s_u[base];
-#pragma unroll 1
-      for (int l = 1; l < NX; ++l) x = fma(a.D[i + NX * l], s_u[base + step * l], x);
-      s_d[base + step * i] = x;
-    }
-  }
+  line_outputs<NX, false>(s_u + base, step, 0, NX, a.fd, a.D, nullptr,
+                          [&](int i, double x) { s_d[base + step * i] = x; });
 }
 
 template <int NX>
@@ -133,7 +108,7 @@ __global__ void __launch_bounds__(KCfg<NX>::NT, KCfg<NX>::kMinBlocks)
       int i, j, k;
       face_node<NX>(f, ab % NX, ab / NX, i, j, k);
       fv = i + C::RS * j + C::SZ * k;
-      fax = f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2);
+      fax = slot_axis(f);
       later = (fax > 0 && (i == 0 || i == NX - 1)) || (fax > 1 && (j == 0 || j == NX - 1));
       const long js = (long)e * NF + tid, L = a.nxzfl;
       const int pv = a.partner[js];

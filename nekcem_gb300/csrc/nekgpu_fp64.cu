@@ -47,16 +47,6 @@ struct DCfg : ElemCfg<NX> {
   static constexpr size_t smem(bool split) { return off_D + (split ? E::N2 * 8 : 0); }
 };
 
-// Field component of the k-th partner value of face f: all six with the
-// face terms (EXT 2), else H and E along the two axes tangential to f.
-template <int EXT>
-__device__ __forceinline__ int partner_comp(int f, int k) {
-  if (EXT == 2) return k;
-  const int ax = slot_axis(f);
-  const int tang = (k & 1) ? (ax == 2 ? 1 : 2) : (ax == 0 ? 1 : 0);
-  return (k < 2 ? 0 : 3) + tang;
-}
-
 // The part of an element a block works out: its nodes with k in [k0, k1).
 struct Slab {
   int k0, k1;

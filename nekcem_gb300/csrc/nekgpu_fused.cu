@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "nekgpu_elem.cuh"
 #include "nekgpu_internal.h"
 
 namespace nekgpu {
@@ -98,19 +99,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
     if (mbar_try_wait(bar, parity)) return true;
   atomicExch(status, 1);
   return false;
-}
-
-// face slot f (reference order) -> reference axis 0=r,1=s,2=t and side
-__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
-__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
-__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
-
-template <int NX>
-__device__ __forceinline__ int face_vol(int f, int a, int b) {
-  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
-  const int ax = slot_axis(f);
-  return ax == 0 ? fixed + NX * a + NX * NX * b
-                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
 }
 
 template <int NX>

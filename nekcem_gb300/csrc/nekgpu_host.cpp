@@ -1130,7 +1130,6 @@ int upload_fused(Context* c, const Compact& cp) {
   a.k = c->d_k;
   a.coef = c->d_coef;
   a.nbr = c->d_nbr;
-  a.egeom = c->d_egeom;
   a.egeomf = c->d_egeomf;
   a.fcoef = c->d_fcoef;
   a.C0 = cp.C0;

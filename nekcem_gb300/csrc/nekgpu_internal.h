@@ -252,10 +252,11 @@ struct Fp64Dev {
   double D[kMaxFixed * kMaxFixed];  // D(i,j) at [i + nx*j]
 };
 
+// Arguments of the plain FP32 stage (nekgpu_fused.cu); the other forms read the
+// source, extension and matrix members from here too.
 struct FusedDev {
   int nelt;
   long npts;
-  PmlDev pml;
   DispDev disp;
   GrapheneDev gr;
   const int* inc_elem;    // nelt: row of the element in inc_val, -1 without incident faces
@@ -264,18 +265,15 @@ struct FusedDev {
   const double* u_in;
   double* u_out;
   double* k;            // RK register read
-  double* k_out;        // RK register written (== k unless stage data is being kept)
+  double* k_out;        // RK register written
   const double* coef;   // 2*npts: dt*hbm1 then dt*ebm1
   const int* nbr;       // 6*nelt
-  const double* egeom;  // 9*nelt
   const float* egeomf;  // 9*nelt, FP32 copy for the mixed form
   const void* fcoef;    // 4 per face node (T), null when uniform
   const int* src_elem;  // nelt: offset (in elements) into src_w or -1; null if no source
   const void* src_w;    // T, nx^3 per source element
-  double src_ft;        // amp*ricker(rktime)
-  float src_ftf;
+  float src_ftf;        // amp*ricker(rktime)
   double a, b;          // rk4a(i), rk4b(i)
-  double dt;            // for the PML auxiliary fields (coef carries dt for u)
   double C0;
   float C0f;
   int* status;

@@ -5,36 +5,16 @@
 
 #include <cuda_runtime.h>
 
+#include "nekgpu_elem.cuh"
 #include "nekgpu_fixed.cuh"
 #include "nekgpu_internal.h"
 
 namespace nekgpu {
 namespace {
 
-__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
-__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
-__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
-constexpr int cmax(int a, int b) { return a > b ? a : b; }
-constexpr int round32(int a) { return (a + 31) / 32 * 32; }
-
-template <int NX>
-__device__ __forceinline__ int face_vol(int f, int a, int b) {
-  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
-  const int ax = slot_axis(f);
-  return ax == 0 ? fixed + NX * a + NX * NX * b
-                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
-}
-
 // x with its sign flipped where neg (no FP64 instruction)
 __device__ __forceinline__ double flip(double x, bool neg) {
   return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
-}
-
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
 }
 
 template <int NX>

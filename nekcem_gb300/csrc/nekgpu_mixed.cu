@@ -43,6 +43,7 @@
 
 #include <type_traits>
 
+#include "nekgpu_elem.cuh"
 #include "nekgpu_internal.h"
 #include "nekgpu_pair.cuh"
 
@@ -95,11 +96,6 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned
       "l"(src), "r"(bytes), "r"(smem_addr(bar))
       : "memory");
 }
-// 8-byte asynchronous global -> shared copies (element blocks whose size is
-// not a multiple of 16 bytes, where a bulk copy cannot start on every element)
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 // one line into L1 ahead of a load
@@ -129,18 +125,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
   return false;
 }
 
-__host__ __device__ constexpr int slot_axis(int f) { return f == 1 || f == 3 ? 0 : (f < 4 ? 1 : 2); }
-__host__ __device__ constexpr int slot_side(int f) { return (f == 0 || f == 3 || f == 4) ? -1 : 1; }
-__host__ __device__ constexpr int slot_opp(int f) { return f < 4 ? (f + 2) & 3 : 9 - f; }
-
-template <int NX>
-__device__ __forceinline__ int face_vol(int f, int a, int b) {
-  const int fixed = slot_side(f) < 0 ? 0 : NX - 1;
-  const int ax = slot_axis(f);
-  return ax == 0 ? fixed + NX * a + NX * NX * b
-                 : (ax == 1 ? a + NX * fixed + NX * NX * b : a + NX * b + NX * NX * fixed);
-}
-
 // D of order nx-1 in the FP32 pieces of the exact-hi contraction, as float
 // pairs indexed by nx so that every coefficient is a compile-time
 // constant-bank operand: [nx][0][i + nx*l] = (Dh, Df) of D(i,l),
@@ -157,9 +141,6 @@ __device__ __forceinline__ int opaque_tid() {
   asm volatile("" : "+r"(t));
   return t;
 }
-
-constexpr int cmax(int a, int b) { return a > b ? a : b; }
-constexpr int round32(int a) { return (a + 31) / 32 * 32; }
 
 // First k-layer of slab s of S (even, so that the outputs' float pairs of D
 // stay whole), and the slab of a part of a line's outputs alike
@@ -360,17 +341,6 @@ __device__ __forceinline__ void add_jump(float2& J, double d) {
   float s, t;
   two_sum(J.x, d2f_hi(d), s, t);
   J = make_float2(s, (J.y + d2f_lo(d)) + t);
-}
-
-// Field component of the k-th parked partner value of face f: all six with
-// the face terms (EXT 2), else H and E along the two axes tangential to f
-// (k = 0, 1: H; k = 2, 3: E; lower axis first).
-template <int EXT>
-__device__ __forceinline__ int partner_comp(int f, int k) {
-  if (EXT == 2) return k;
-  const int ax = slot_axis(f);
-  const int tang = (k & 1) ? (ax == 2 ? 1 : 2) : (ax == 0 ? 1 : 0);
-  return (k < 2 ? 0 : 3) + tang;
 }
 
 // The jump p - (uh + ul) of a partner value p (FP64) against the own split
