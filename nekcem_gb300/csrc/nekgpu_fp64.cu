@@ -7,8 +7,8 @@
 // (src/cem_common.F:18-75), one kernel per stage.
 //
 // What bounds it: GB300 issues two FP64 lanes per clock and SM.  With the
-// contractions in FP64 (96 of its ~165 operations per node at N=7) a stage of
-// the 16^3-element N=7 box took 690 us; it takes 223 us (56 G DOF-stage
+// contractions in FP64 (96 of its 206 FP64-pipe instructions per node at N=7) a
+// stage of the 16^3-element N=7 box took 690 us; it takes 221 us (57 G DOF-stage
 // updates/s, FP64 pipe 61 % busy) with
 //  * the contractions in 64-bit integer arithmetic (nekgpu_fixed.cuh) on
 //    another pipe, one thread per GLL line, D as constant-bank operands;
@@ -17,7 +17,7 @@
 //    the lift factor is part of the face coefficients, and w3 is folded into
 //    the inverse-mass coefficient;
 //  * only the four field components tangential to a face in its flux.
-// About 40 FP64 operations per node are left (finish 18, curl 8, flux 12): 20
+// 40.5 FP64-pipe instructions per node are left (finish 18, curl 8, flux 12): 20
 // of the 33 clocks per node and SM.
 //
 // Phases per element: state to shared memory (8-byte asynchronous copies into
@@ -507,11 +507,12 @@ int launch(Context* c, const Fp64Dev& a, bool pdl, int nsplit, int og) {
 }
 
 // Fewer elements than half the SMs: each is split over as many blocks as give
-// one block per SM (27 elements, N=8: 10.0 us per stage in five slabs, 11.3
-// in three or four, 13.0 in eight, 17.8 unsplit; 64 elements, N=7: 10.8 us in
-// two, 12.7 in four, 13.4 unsplit).  With more elements the slabs only repeat
-// the staging and the t-lines' conversions (100 elements, N=7: 13.4 us
-// unsplit, 14.6 in two).
+// one block per SM (us per stage: 27 elements, N=8: 10.2 in five slabs, 11.5 in
+// three or four, 17.9 unsplit; 64 elements, N=7: 11.2 in two, 12.7 in four,
+// 13.4 unsplit; with PML 15.0, 14.4, 20.5).  With more elements the slabs only
+// repeat the staging and the t-lines' conversions (100 elements, N=7: 13.3
+// unsplit, 14.7 in two; with PML 20.5, 21.2).  N=2 is not split in two (64
+// elements: 9.4, unsplit 8.3, in three 8.0); at N=3 and 4 the two are equal.
 template <int NX, int EXT>
 int dispatch_split(Context* c, const Fp64Dev& a, bool pdl) {
   // outputs per task of a split line: three at NX = 9 (10.0 against 10.6 us
@@ -519,7 +520,7 @@ int dispatch_split(Context* c, const Fp64Dev& a, bool pdl) {
   // 11.4 with two)
   constexpr int og = NX == 9 ? 3 : (NX + 1) / 2;
   const int ns = std::min(num_sms(c) / a.nelt, NX);
-  return ns >= 2 ? launch<NX, EXT, true>(c, a, pdl, ns, og) : launch<NX, EXT, false>(c, a, pdl, 1, NX);
+  return ns >= (NX == 3 ? 3 : 2) ? launch<NX, EXT, true>(c, a, pdl, ns, og) : launch<NX, EXT, false>(c, a, pdl, 1, NX);
 }
 
 template <int EXT>
