@@ -32,8 +32,8 @@
 // result joined into one FP64 value.
 //
 // What bounds it: latencies at four blocks per SM, the FP64 pipe (41 slots per
-// node) 42 % and issue (75 warp instructions per node, the face terms most of
-// them) 38 % busy; 49 us per stage at 512 elements, N=7.  With double-float
+// node) 42 % and issue (74 warp instructions per node, the face terms most of
+// them) 39 % busy; 49 us per stage at 512 elements, N=7.  With double-float
 // contractions per node and the face terms added per node by divergent warps
 // (~100 FP64 slots per node, 512 threads and one block per SM) the reverse
 // sweep of 100 steps of the 8^3-element N=7 box, the recomputation beside it,

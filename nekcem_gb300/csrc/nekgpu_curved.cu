@@ -13,10 +13,11 @@
 // What bounds it: the FP64 pipe (two lanes per clock and SM).  The 18
 // contractions per node run in 64-bit integer arithmetic (nekgpu_fixed.cuh),
 // one thread per GLL line; the node's weight w3 multiplies the curl once, as
-// the lift is added, and the areas are inside the face coefficients.  That leaves ~90 FP64 operations per node at
-// N=7 (curl 36, flux 32, finish 18) of the ~230 of a form with FP64
-// contractions: 57 us per stage for 990 elements at N=5 (135 before; FP64 pipe
-// 73 % busy), 117 for 1000 at N=7.
+// the lift is added, and the areas are inside the face coefficients.  That
+// leaves 117 FP64-pipe instructions per node at N=5 with two media (curl 36,
+// flux about 60 on the many face nodes of this order, finish 18) of the ~230 of
+// a form with FP64 contractions: 58.6 us per stage for 990 elements (135 before;
+// FP64 pipe 77 % busy), at N=7 116 us for 1000 elements.
 //
 // One block per element at a time, thread per node: state in shared memory;
 // face nodes' fluxes summed per node, axis by axis so that no two threads
