@@ -353,6 +353,14 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
   }
   cp.egeom.assign(9 * (size_t)nelt, 0.0);
   cp.lift.assign(6 * (size_t)nelt, 0.0);
+  // the weights of a face's nodes, and one face's quotients
+  std::vector<double> ww(n2), w3f(6 * n2), qa(n2), ql(n2);
+  for (int f = 0; f < 6; ++f)
+    for (int b = 0; b < n; ++b)
+      for (int a = 0; a < n; ++a) {
+        ww[a + (long)n * b] = cp.w[a] * cp.w[b];
+        w3f[a + (long)n * b + n2 * f] = m->w3mn[face_vol(f, a, b, n)];
+      }
   const double* mt[9] = {m->rxmn, m->rymn, m->rzmn, m->sxmn, m->symn, m->szmn, m->txmn, m->tymn, m->tzmn};
   for (int e = 0; e < nelt; ++e) {
     const long o = n3 * e;
@@ -376,7 +384,10 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
     cp.egeom[9 * e + 2] = diag[2];
     for (int f = 0; f < 6; ++f) {
       const int ax = kSlotAxis[f], sd = kSlotSide[f];
-      double s = 0, sl = 0, l0 = 0;
+      const double* area = m->aream + n2 * (f + 6L * e);
+      for (long k = 0; k < n2; ++k) qa[k] = area[k] / ww[k];
+      for (long k = 0; k < n2; ++k) ql[k] = area[k] / w3f[k + n2 * f];
+      double s = 0, sl = 0;
       for (int b = 0; b < n; ++b)
         for (int a = 0; a < n; ++a) {
           const long j = a + (long)n * b + n2 * (f + 6L * e);
@@ -386,18 +397,15 @@ int build_compact(const nekgpu_mesh* m, Compact& cp) {
             const double want = (d == ax) ? (double)sd : 0.0;
             if (std::fabs(nv[d] - want) > tol) return NEKGPU_ERR_MESH;
           }
-          s += m->aream[j] / (cp.w[a] * cp.w[b]);
-          const double l = m->aream[j] / m->w3mn[face_vol(f, a, b, n)];
-          if (a == 0 && b == 0) l0 = l;
-          sl += l - l0;
         }
+      for (long k = 0; k < n2; ++k) {
+        s += qa[k];
+        sl += ql[k] - ql[0];
+      }
       s /= n2;
-      cp.lift[6 * e + f] = l0 + sl / n2;
-      for (int b = 0; b < n; ++b)
-        for (int a = 0; a < n; ++a) {
-          const long j = a + (long)n * b + n2 * (f + 6L * e);
-          if (std::fabs(m->aream[j] / (cp.w[a] * cp.w[b]) - s) > tol * s) return NEKGPU_ERR_MESH;
-        }
+      cp.lift[6 * e + f] = ql[0] + sl / n2;
+      for (long k = 0; k < n2; ++k)
+        if (std::fabs(qa[k] - s) > tol * s) return NEKGPU_ERR_MESH;
       cp.egeom[9 * e + 3 + f] = s;
     }
   }
@@ -883,7 +891,8 @@ int upload_plain(Context* c, const PlainHost& p) {
 }
 
 // PML data of the fused forms (layout: PmlDev), compact over the PML elements
-int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
+// (sigma moves from cp to the context)
+int upload_pml_fused(Context* c, DevAlloc& A, Compact& cp, PmlDev& out) {
   out = PmlDev{};
   if (!cp.pml.on()) return NEKGPU_OK;
   const PmlHost& p = cp.pml;
@@ -891,24 +900,25 @@ int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
   const long npml = (long)p.elems.size(), nn = npml * n3;
   std::vector<int> slot(c->nelt, -1);
   std::vector<double> d((size_t)kPmlData * nn);
-  c->host_pml_sigma.resize(3 * (size_t)nn);
   for (long l = 0; l < npml; ++l) {
     const long e = p.elems[l];
     slot[e] = (int)l;
     for (long v = 0; v < n3; ++v) {
       const long j = e * n3 + v, q = l * n3 + v;
-      const double nrm = cp.bm1[j] / (cp.w3[v] * cp.egeom[9 * e]);
+      const double fac = cp.w3[v] * cp.egeom[9 * e], nrm = cp.bm1[j] / fac;
+      double sig[3], s[3];
       for (int ax = 0; ax < 3; ++ax) {
-        const double sig2 = p.sigma[j + ((ax + 2) % 3) * npts];
-        const double s0 = p.sigma[j + ax * npts] / p.eps[j];
-        const double s1 = p.sigma[j + ((ax + 1) % 3) * npts] / p.eps[j];
-        d[ax * nn + q] = s1;
-        d[(3 + ax) * nn + q] = nrm * (s0 - s1);
-        d[(6 + ax) * nn + q] = nrm * (sig2 / p.eps[j] * p.mu[j]);
-        d[(9 + ax) * nn + q] = nrm * sig2;
-        c->host_pml_sigma[ax * nn + q] = p.sigma[j + ax * npts];
+        sig[ax] = p.sigma[j + ax * npts];
+        s[ax] = sig[ax] / p.eps[j];
       }
-      d[12 * nn + q] = cp.w3[v] * cp.egeom[9 * e] / cp.bm1[j];
+      for (int ax = 0; ax < 3; ++ax) {
+        const int a1 = (ax + 1) % 3, a2 = (ax + 2) % 3;
+        d[ax * nn + q] = s[a1];
+        d[(3 + ax) * nn + q] = nrm * (s[ax] - s[a1]);
+        d[(6 + ax) * nn + q] = nrm * (s[a2] * p.mu[j]);
+        d[(9 + ax) * nn + q] = nrm * sig[a2];
+      }
+      d[12 * nn + q] = fac / cp.bm1[j];
     }
   }
   // Elements in the order the stage kernels take them: the PML elements, whose
@@ -931,6 +941,7 @@ int upload_pml_fused(Context* c, DevAlloc& A, const Compact& cp, PmlDev& out) {
     return NEKGPU_ERR_CUDA;
   c->npml = (int)npml;
   c->pml_elems = p.elems;
+  c->host_pml_sigma = std::move(cp.pml.sigma);
   out.slot = c->d_pml_slot;
   out.order = d_order;
   out.data = c->d_pml_data;
@@ -965,7 +976,8 @@ void split_D(const std::vector<double>& D, int n, std::vector<float>& tab) {
   }
 }
 
-int upload_fused(Context* c, const Compact& cp) {
+// (the face coefficients move from cp to the context)
+int upload_fused(Context* c, Compact& cp) {
   DevAlloc A(c);
   int st;
   const long n3 = (long)c->nx * c->nx * c->nx;
@@ -979,31 +991,31 @@ int upload_fused(Context* c, const Compact& cp) {
   for (int e = 0; e < c->nelt; ++e) c->host_rx[e] = cp.egeom[9 * (size_t)e];
   // unscaled inverse-mass coefficients: hbm1|ebm1, or for the mixed and fused
   // FP64 forms the normalised hbm1*w3*rx | ebm1*w3*rx (their residual is
-  // res/(w3*rx))
+  // res/(w3*rx)).  w3, rx and the lift factors over rx go through d_coef, which
+  // the first stage fills.
+  if ((st = A.get(&c->d_cbase, 2 * c->npts))) return st;
   {
-    std::vector<double> base(2 * c->npts);
-    for (long g = 0; g < c->npts; ++g) {
-      double f = 1.0;
-      if (c->form != NEKGPU_MIXED_NAIVE) f = cp.w3[g % n3] * cp.egeom[9 * (g / n3)];
-      base[g] = cp.hbm1[g] * f;
-      base[c->npts + g] = cp.ebm1[g] * f;
-    }
-    if ((st = A.put(&c->d_cbase, base))) return st;
+    std::vector<double> tab(cp.w3);
+    tab.insert(tab.end(), c->host_rx.begin(), c->host_rx.end());
+    for (size_t k = 0; k < cp.lift.size(); ++k) tab.push_back(cp.lift[k] / c->host_rx[k / 6]);
+    if (check_cuda(cudaMemcpy(c->d_coef, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice)))
+      return NEKGPU_ERR_CUDA;
+  }
+  if (c->form != NEKGPU_MIXED_NAIVE) {
+    if ((st = util_mass_base(c, c->d_cbase, c->d_coef, c->d_coef + n3))) return st;
+  } else if (check_cuda(cudaMemcpy(c->d_cbase, c->d_hbm1, c->npts * sizeof(double), cudaMemcpyDeviceToDevice)) ||
+             check_cuda(cudaMemcpy(c->d_cbase + c->npts, c->d_ebm1, c->npts * sizeof(double),
+                                   cudaMemcpyDeviceToDevice))) {
+    return NEKGPU_ERR_CUDA;
   }
   c->uniform = cp.uniform;
   c->d_fcoef = nullptr;
   if (!cp.uniform) {
     if (c->form == NEKGPU_FUSED64) {  // times the lift factor of the slot
-      std::vector<double> f(cp.fcoef);
-      const size_t n2 = (size_t)c->nx * c->nx;
-      for (size_t j = 0; j < f.size() / 4; ++j) {
-        const double lf = cp.lift[j / n2] / cp.egeom[9 * (j / (6 * n2))];
-        for (int q = 0; q < 4; ++q) f[4 * j + q] *= lf;
-      }
       double* d;
-      if ((st = A.put(&d, f))) return st;
+      if ((st = A.put(&d, cp.fcoef)) || (st = util_scale_faces(c, d, c->d_coef + n3 + c->nelt))) return st;
       c->d_fcoef = d;
-      c->host_fcoef64 = cp.fcoef;
+      c->host_fcoef64 = std::move(cp.fcoef);
     } else {
       std::vector<float> f(cp.fcoef.begin(), cp.fcoef.end());
       if (c->form == NEKGPU_MIXED) {
@@ -1080,7 +1092,7 @@ int upload_fused(Context* c, const Compact& cp) {
     f.C0 = cp.C0;
     for (int i = 0; i < c->nx * c->nx; ++i) f.D[i] = cp.D[i];
     for (int i = 0; i < c->nx; ++i) f.w[i] = cp.w[i];
-    if (!cp.uniform) c->host_fcoef64 = cp.fcoef;
+    if (!cp.uniform) c->host_fcoef64 = std::move(cp.fcoef);
     return upload_pml_fused(c, A, cp, m.pml);
   }
   if ((st = A.put(&c->d_egeom, cp.egeom))) return st;
@@ -1201,38 +1213,34 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   // the mixed form's residual is res/w3, and its metrics and face data are
   // stored as (hi, lo) float pairs in the same 8 bytes
   const bool norm = c->form == NEKGPU_MIXED;
-  std::vector<double> base(2 * npts);
-  for (long e = 0; e < m->nelt; ++e)
-    for (long v = 0; v < n3; ++v) {
-      const double w = norm ? m->w3mn[v] : 1.0;
-      base[e * n3 + v] = hb[e * n3 + v] * w;
-      base[npts + e * n3 + v] = eb[e * n3 + v] * w;
-    }
-  if ((st = A.put(&c->d_cbase, base))) return st;
+  CurvedDev& a = c->cargs;
+  a = CurvedDev{};
+  double* d;
+  if ((st = A.put(&d, std::vector<double>(m->w3mn, m->w3mn + n3)))) return st;
+  a.w3 = d;
+  if ((st = A.get(&c->d_cbase, 2 * npts))) return st;
+  if (norm) {
+    if ((st = util_mass_base(c, c->d_cbase, a.w3, nullptr))) return st;
+  } else if (check_cuda(cudaMemcpy(c->d_cbase, c->d_hbm1, npts * sizeof(double), cudaMemcpyDeviceToDevice)) ||
+             check_cuda(cudaMemcpy(c->d_cbase + npts, c->d_ebm1, npts * sizeof(double),
+                                   cudaMemcpyDeviceToDevice))) {
+    return NEKGPU_ERR_CUDA;
+  }
   c->coef_dt = std::nan("");
   const double* mt[9] = {m->rxmn, m->rymn, m->rzmn, m->sxmn, m->symn, m->szmn, m->txmn, m->tymn, m->tzmn};
   const double* nr[3] = {m->unxm, m->unym, m->unzm};
   // one row of `count` values to the device
-  std::vector<float> row(norm ? 2 * (size_t)std::max(npts, nxzfl) : 0);
   auto put_row = [&](double* dst, const double* src, long count) -> int {
-    if (norm) {
-      for (long i = 0; i < count; ++i) {
-        row[2 * i] = (float)src[i];
-        row[2 * i + 1] = (float)(src[i] - (double)row[2 * i]);
-      }
-    }
-    return check_cuda(cudaMemcpy(dst, norm ? (const void*)row.data() : src, count * sizeof(double),
-                                 cudaMemcpyHostToDevice));
+    return check_cuda(cudaMemcpy(dst, src, count * sizeof(double), cudaMemcpyHostToDevice));
   };
-  std::vector<double> area(nxzfl), half(nxzfl);
+  std::vector<double> w3f(6 * n2), area(nxzfl), half(nxzfl);  // w3f: of a face's nodes
+  for (int f = 0; f < 6; ++f)
+    for (int b = 0; b < n; ++b)
+      for (int a = 0; a < n; ++a)
+        w3f[a + (long)n * b + n2 * f] = norm ? m->w3mn[face_vol(f, a, b, n)] : 1.0;
   for (long e = 0; e < m->nelt; ++e)
-    for (int f = 0; f < 6; ++f)
-      for (int b = 0; b < n; ++b)
-        for (int a = 0; a < n; ++a) {
-          const long j = a + (long)n * b + n2 * (f + 6 * e);
-          area[j] = norm ? m->aream[j] / m->w3mn[face_vol(f, a, b, n)] : m->aream[j];
-          half[j] = 0.5 * area[j];
-        }
+    for (long k = 0; k < 6 * n2; ++k) area[k + 6 * n2 * e] = m->aream[k + 6 * n2 * e] / w3f[k];
+  for (long j = 0; j < nxzfl; ++j) half[j] = 0.5 * area[j];
   auto impedance = [&](int q, long j) {
     const double Y0 = m->Y_0[j], Z0 = m->Z_0[j];
     return q == 0 ? -0.5 / Y0 * m->Y_1[j] : q == 1 ? 0.5 / Y0 * m->C0
@@ -1242,19 +1250,16 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
   for (long j = 0; j < nxzfl && uniform; ++j)
     uniform = impedance(0, j) == -0.5 && impedance(1, j) == 0.5 && impedance(2, j) == 0.5 &&
               impedance(3, j) == 0.5;
-  CurvedDev& a = c->cargs;
-  a = CurvedDev{};
-  double* d;
   int* di;
   if ((st = A.get(&d, 9 * (size_t)npts))) return st;
   for (int q = 0; q < 9; ++q)
     if ((st = put_row(d + q * npts, mt[q], npts))) return st;
+  if (norm && (st = util_split_pairs(d, 9 * npts))) return st;
   a.metrics = d;
-  if ((st = A.put(&d, std::vector<double>(m->w3mn, m->w3mn + n3)))) return st;
-  a.w3 = d;
   if ((st = A.get(&d, 4 * (size_t)nxzfl))) return st;
   for (int q = 0; q < 4; ++q)
     if ((st = put_row(d + q * nxzfl, q < 3 ? nr[q] : half.data(), nxzfl))) return st;
+  if (norm && (st = util_split_pairs(d, 4 * nxzfl))) return st;
   a.face = d;
   if (!uniform) {
     if ((st = A.get(&d, 4 * (size_t)nxzfl))) return st;
@@ -1262,6 +1267,7 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
       for (long j = 0; j < nxzfl; ++j) half[j] = area[j] * impedance(q, j);
       if ((st = put_row(d + q * nxzfl, half.data(), nxzfl))) return st;
     }
+    if (norm && (st = util_split_pairs(d, 4 * nxzfl))) return st;
     a.fcoef = d;
   }
   if ((st = A.put(&di, partner))) return st;
@@ -1283,6 +1289,8 @@ int upload_curved(Context* c, const nekgpu_mesh* m) {
 }
 
 int finish_init(Context* c, int st) {
+  // the set-up on the default stream, which the context's does not wait for
+  if (!st && check_cuda(cudaStreamSynchronize(nullptr))) st = NEKGPU_ERR_CUDA;
   if (st) {
     free_all(c);
     return st;
@@ -2051,7 +2059,7 @@ int nekgpu_get_array(nekgpu_ctx* c, const char* name, double* out) {
       const long q = l * n3 + v, g = (long)c->pml_elems[l] * n3 + v;
       for (int cc = 0; cc < 3; ++cc) {
         if (sg)
-          out[cc * P + g] = c->host_pml_sigma[cc * nn + q];
+          out[cc * P + g] = c->host_pml_sigma[cc * P + g];
         else
           out[cc * P + g] = h[((dn ? 3 : 0) + cc) * nn + q];
       }
@@ -2522,8 +2530,9 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
     c->d_src_w = nullptr;
     // elements whose weights are all below 1e-30 of the peak carry no source
     const long n3 = (long)c->nx * c->nx * c->nx;
+    const bool norm = c->curved ? c->form == NEKGPU_MIXED : c->form != NEKGPU_MIXED_NAIVE;
     std::vector<int> off(c->nelt, -1);
-    std::vector<double> wd;
+    std::vector<double> wd, rx;
     int cnt = 0;
     for (int e = 0; e < c->nelt; ++e) {
       double m = 0;
@@ -2531,30 +2540,12 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
       if (m > 1e-30 * gmax) {
         off[e] = cnt++;
         wd.insert(wd.end(), g.begin() + e * n3, g.begin() + (e + 1) * n3);
+        rx.push_back(norm && !c->curved ? c->host_rx[e] : 1.0);
       }
     }
     int* d_off;
     if ((st = A.put(&d_off, off))) return st;
-    if (c->curved ? c->form == NEKGPU_MIXED : c->form != NEKGPU_MIXED_NAIVE) {
-      // normalised like the residual: weight / (w3 * rx), on curved meshes / w3
-      for (int e = 0; e < c->nelt; ++e)
-        if (off[e] >= 0)
-          for (long v = 0; v < n3; ++v)
-            wd[off[e] * n3 + v] /= c->host_w3[v] * (c->curved ? 1.0 : c->host_rx[e]);
-    }
-    if (c->form == NEKGPU_MIXED && !c->curved) {
-      // as (hi, lo) float pairs (~2^-48 of the weight)
-      std::vector<float> wf(2 * wd.size());
-      for (size_t i = 0; i < wd.size(); ++i) {
-        wf[2 * i] = (float)wd[i];
-        wf[2 * i + 1] = (float)(wd[i] - (double)wf[2 * i]);
-      }
-      float* d;
-      if ((st = A.put(&d, wf))) return st;
-      c->d_src_w = d;
-      c->margs.src_elem = d_off;
-      c->margs.src_w = reinterpret_cast<const float2*>(d);
-    } else if (c->form == NEKGPU_MIXED_NAIVE) {
+    if (c->form == NEKGPU_MIXED_NAIVE) {
       std::vector<float> wf(wd.begin(), wd.end());
       float* d;
       if ((st = A.put(&d, wf))) return st;
@@ -2563,6 +2554,27 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
       double* d;
       if ((st = A.put(&d, wd))) return st;
       c->d_src_w = d;
+      const long nw = (long)wd.size();
+      if (norm && nw) {  // like the residual: weight / (w3 * rx), on curved meshes / w3
+        rx.insert(rx.begin(), c->host_w3.begin(), c->host_w3.end());
+        double* t = nullptr;
+        if (cudaMalloc(&t, rx.size() * sizeof(double)) != cudaSuccess) {
+          cudaGetLastError();
+          return NEKGPU_ERR_NOMEM;
+        }
+        st = check_cuda(cudaMemcpy(t, rx.data(), rx.size() * sizeof(double), cudaMemcpyHostToDevice))
+                 ? NEKGPU_ERR_CUDA
+                 : util_source_norm(c, d, t, t + n3, nw);
+        if (!st && check_cuda(cudaStreamSynchronize(nullptr))) st = NEKGPU_ERR_CUDA;
+        cudaFree(t);
+        if (st) return st;
+      }
+      if (c->form == NEKGPU_MIXED && !c->curved) {  // as (hi, lo) float pairs (~2^-48 of the weight)
+        if (nw && ((st = util_split_pairs(d, nw)) || check_cuda(cudaStreamSynchronize(nullptr))))
+          return NEKGPU_ERR_CUDA;
+        c->margs.src_elem = d_off;
+        c->margs.src_w = reinterpret_cast<const float2*>(d);
+      }
     }
     c->d_src_elem = d_off;
     c->fargs.src_elem = d_off;

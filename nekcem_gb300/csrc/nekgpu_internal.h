@@ -467,7 +467,7 @@ struct Context {
   double *d_pml_sigma = nullptr, *d_eps = nullptr, *d_mu = nullptr, *d_pml_res = nullptr;
   int* d_pmlptr = nullptr;
   double *d_pml_aux = nullptr, *d_pml_k = nullptr, *d_pml_data = nullptr;
-  std::vector<double> host_pml_sigma;  // fused forms: sigma along x, y, z of the PML nodes, read back
+  std::vector<double> host_pml_sigma;  // fused forms: sigma (3*npts), read back
   int* d_pml_slot = nullptr;
   // dispersive currents: per node model (0 none, 1 Drude, 2 Lorentz) and
   // parameters a, b, c on the host; the device side in DispDev (all forms)
@@ -619,6 +619,14 @@ int norms_noalloc(Context* c, const double* exact_dev, double l2[6], double linf
 // reductions / utilities (nekgpu_util.cu)
 int util_norms(Context* c, const double* d_exact, double l2[6], double linf[6]);
 int util_energy(Context* c, double* energy);
+// set-up of a context's arrays on the default stream: base = hbm1 | ebm1 times
+// w3 * rx (rx null: times w3), the four coefficients of every face node times
+// their face's lf, source weights over w3 * rx (rx per listed element), and FP64
+// values into (hi, lo) float pairs in place
+int util_mass_base(Context* c, double* base, const double* w3, const double* rx);
+int util_scale_faces(Context* c, double* fcoef, const double* lf);
+int util_source_norm(Context* c, double* w, const double* w3, const double* rx, long n);
+int util_split_pairs(double* x, long n);
 int util_blowup(Context* c, int* bad);
 
 }  // namespace nekgpu

@@ -78,6 +78,37 @@ __global__ void k_blowup(const double* __restrict__ u, long n, int* flag) {
   }
 }
 
+// ---- set-up -----------------------------------------------------------------
+__global__ void k_mass_base(double* base, const double* hbm1, const double* ebm1, const double* w3,
+                            const double* rx, long npts, int n3) {
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (g >= npts) return;
+  const long e = g / n3;
+  const double f = rx ? w3[g - e * n3] * rx[e] : w3[g - e * n3];
+  base[g] = hbm1[g] * f;
+  base[npts + g] = ebm1[g] * f;
+}
+
+__global__ void k_scale_faces(double* fcoef, const double* lf, long n, int per_face) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i < n) fcoef[i] *= lf[i / per_face];
+}
+
+__global__ void k_source_norm(double* w, const double* w3, const double* rx, long n, int n3) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i < n) w[i] /= w3[i % n3] * rx[i / n3];
+}
+
+__global__ void k_split_pairs(double* x, long n) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double v = x[i];
+  const float hi = (float)v;
+  reinterpret_cast<float2*>(x)[i] = make_float2(hi, (float)(v - (double)hi));
+}
+
+unsigned blocks_for(long n) { return (unsigned)((n + kRedThreads - 1) / kRedThreads); }
+
 }  // namespace
 
 static const double* state_ptr(Context* c) { return c->d_u[c->cur]; }
@@ -132,6 +163,27 @@ int util_blowup(Context* c, int* bad) {
   if (check_cuda(cudaStreamSynchronize(c->stream))) return NEKGPU_ERR_CUDA;
   *bad = h;
   return NEKGPU_OK;
+}
+
+int util_mass_base(Context* c, double* base, const double* w3, const double* rx) {
+  k_mass_base<<<blocks_for(c->npts), kRedThreads>>>(base, c->d_hbm1, c->d_ebm1, w3, rx, c->npts,
+                                                    c->nx * c->nx * c->nx);
+  return check_cuda(cudaGetLastError());
+}
+
+int util_scale_faces(Context* c, double* fcoef, const double* lf) {
+  k_scale_faces<<<blocks_for(4 * c->nxzfl), kRedThreads>>>(fcoef, lf, 4 * c->nxzfl, 4 * c->nx * c->nx);
+  return check_cuda(cudaGetLastError());
+}
+
+int util_source_norm(Context* c, double* w, const double* w3, const double* rx, long n) {
+  k_source_norm<<<blocks_for(n), kRedThreads>>>(w, w3, rx, n, c->nx * c->nx * c->nx);
+  return check_cuda(cudaGetLastError());
+}
+
+int util_split_pairs(double* x, long n) {
+  k_split_pairs<<<blocks_for(n), kRedThreads>>>(x, n);
+  return check_cuda(cudaGetLastError());
 }
 
 }  // namespace nekgpu
