@@ -2528,6 +2528,11 @@ int nekgpu_set_source(nekgpu_ctx* c, int enabled, const double xc[3], double sig
     release_dev(c, c->d_src_w);
     c->d_src_elem = nullptr;
     c->d_src_w = nullptr;
+    c->src.enabled = false;  // until the new ones are there
+    c->fargs.src_elem = nullptr;
+    c->fargs.src_w = nullptr;
+    c->margs.src_elem = nullptr;
+    c->margs.src_w = nullptr;
     // elements whose weights are all below 1e-30 of the peak carry no source
     const long n3 = (long)c->nx * c->nx * c->nx;
     const bool norm = c->curved ? c->form == NEKGPU_MIXED : c->form != NEKGPU_MIXED_NAIVE;
